@@ -101,7 +101,8 @@ def _declare(lib):
         "b200_rope": [P, P, P, L, I, I, I, I, I, P],
         "b200_embedding_fwd": [P, P, P, L, I, I, P],
         "b200_embedding_bwd": [P, P, P, L, I, I, P],
-        "b200_embedding_bwd_sorted": [P, P, P, P, L, I, I, I, P],
+        "b200_embedding_bwd_sorted": [P, P, P, P, P, L, I, I, I, P],
+        "b200_embedding_bwd_sorted_bf16": [P, P, P, P, P, L, I, I, P],
         "b200_xent": [P, P, P, P, L, L, I, I, F, I, I, P, P],
         "b200_argmax": [P, L, L, I, I, P, P],
         "b200_sample_topk": [P, L, L, I, I, P, F, I, P, P],
@@ -176,7 +177,7 @@ def check_status(device=None):
 
 # Kernels launched per launcher call (a launcher may issue several).  Used to count this package's
 # own launches inside a timed region.
-_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "xent": 3, "flash_bwd": 3, "latent_decode": 2, "grouped_decode": 2}
+_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "embedding_bwd_sorted": 2, "xent": 3, "flash_bwd": 3, "latent_decode": 2, "grouped_decode": 2}
 _LAUNCHES = 0
 
 
@@ -594,9 +595,14 @@ def embedding_fwd(tokens, weight, out_dtype=None):
     return out
 
 
+def _embedding_parts(lib, rows: int, d: int, device):
+    lib.b200_embedding_bwd_parts.restype, lib.b200_embedding_bwd_parts.argtypes = c_ll, [c_ll, c_int]
+    return torch.empty(lib.b200_embedding_bwd_parts(rows, d), dtype=torch.float32, device=device)
+
+
 def embedding_bwd(dx, tokens, grad_weight, accumulate=False, deterministic=True):
     """Scatter-add of dx rows into the fp32 gradient table.  The default sorts the token ids (stable device sort)
-    and adds every run of equal ids in order inside one warp: no atomics, bitwise reproducible.
+    and adds every run of equal ids in a fixed order: no atomics, bitwise reproducible.
     ``deterministic=False`` uses 16-byte vector atomics instead (one launch, no sort)."""
     lib = load()
     _req(dx.dtype == torch.bfloat16 and dx.is_contiguous(), "dx must be contiguous bf16")
@@ -610,11 +616,9 @@ def embedding_bwd(dx, tokens, grad_weight, accumulate=False, deterministic=True)
              "a bf16 gradient table is written by the deterministic kernel only, without accumulation")
         grad_weight.zero_()
         sorted_tokens, order = torch.sort(tokens.reshape(-1), stable=True)
-        fn = lib.b200_embedding_bwd_sorted_bf16
-        fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p]
-        fn.restype = c_int
-        _check(fn(_ptr(sorted_tokens), _ptr(order), _ptr(dx), _ptr(grad_weight), rows, d, v, _stream()),
-               "embedding_bwd_sorted")
+        parts = _embedding_parts(lib, rows, d, dx.device)
+        _check(lib.b200_embedding_bwd_sorted_bf16(_ptr(sorted_tokens), _ptr(order), _ptr(dx), _ptr(grad_weight), _ptr(parts), rows, d, v,
+                                                  _stream()), "embedding_bwd_sorted")
         return grad_weight
     _req(grad_weight.dtype == torch.float32 and grad_weight.is_contiguous(), "grad table must be fp32")
     if not accumulate:
@@ -622,7 +626,8 @@ def embedding_bwd(dx, tokens, grad_weight, accumulate=False, deterministic=True)
     if deterministic:
         flat = tokens.reshape(-1)
         sorted_tokens, order = torch.sort(flat, stable=True)
-        _check(lib.b200_embedding_bwd_sorted(_ptr(sorted_tokens), _ptr(order), _ptr(dx), _ptr(grad_weight), rows, d, v,
+        parts = _embedding_parts(lib, rows, d, dx.device)
+        _check(lib.b200_embedding_bwd_sorted(_ptr(sorted_tokens), _ptr(order), _ptr(dx), _ptr(grad_weight), _ptr(parts), rows, d, v,
                                              1 if accumulate else 0, _stream()), "embedding_bwd_sorted")
         return grad_weight
     _check(lib.b200_embedding_bwd(_ptr(tokens), _ptr(dx), _ptr(grad_weight), rows, d, v, _stream()), "embedding_bwd")

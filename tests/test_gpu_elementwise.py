@@ -260,3 +260,14 @@ def test_embedding_backward_segments(runs, d):
     assert bool(((more.double() - 2 * want).abs() <= 2 * bound + 2.0 ** -23 * want.abs()).all())
     low = native.embedding_bwd(dx, tok, torch.empty(v, d, device="cuda", dtype=torch.bfloat16))
     assert torch.equal(low, got.bfloat16())
+
+
+def test_scale_by_one_and_others():
+    from llm_systems_from_scratch_b200.ops import native
+    for dt in (torch.float32, torch.bfloat16):
+        x = torch.randn(1003, device="cuda").to(dt)
+        x[3], x[4] = float("inf"), -0.0
+        for c in (1.0, 0.37, 0.0):
+            want = (x.float() * c).to(dt)
+            got = native.scale_(x.clone(), torch.tensor(c, device="cuda"))
+            assert torch.equal(torch.nan_to_num(got, 7.0), torch.nan_to_num(want, 7.0))

@@ -102,6 +102,7 @@ struct GemmParams {
   GemmFinish finish;
   int relu;                   // gated instances of the single-CTA kernel: relu(gate) * up instead of silu(gate) * up
   int splits;
+  int full_tiles;             // CTA-pair kernel: the tiles before this one are contracted whole, the others in `splits` slices
   float* ws;                  // splits * tiles partial tiles of BM x BN floats
   uint32_t* tile_counters;    // four per tile (one per 32-row quarter), zero between launches (the last warp resets its own)
 };

@@ -11,6 +11,9 @@
 //   tmem_full[a]   one per CTA; commit multicast
 //   tmem_empty[a]  lives in the leader; the 2 x 128 epilogue threads of the pair arrive on it
 // TMA loads are ordinary (non-multicast) loads.  Every wait is bounded (see ptx.cuh).
+//
+// Last wave (weight gradients): with T tiles on P pairs, the T % P tiles of the last wave are contracted in `splits` slices of K each, on all
+// pairs; the partial tiles go to a workspace and pair_tail_sum_kernel adds them in slice order (no atomics: reproducible).
 #include "gemm_common.cuh"
 
 namespace b200 {
@@ -154,6 +157,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   const int num_tiles = p.num_m_tiles * p.num_n_tiles;   // tiles of 256 x 256
   const int num_kb = (p.K + BK - 1) / BK;
+  // work unit: a whole tile, or behind the first full_tiles of them a slice of K of a tile (`part`: which partial tile it leaves, else -1)
+  const int full_tiles = p.splits > 1 ? p.full_tiles : num_tiles;
+  const int num_units = full_tiles + (num_tiles - full_tiles) * p.splits;
+  auto unit_tile = [&](int unit, int& kb_lo, int& kb_hi, int& part) {
+    part = unit - full_tiles;
+    kb_lo = 0;
+    kb_hi = num_kb;
+    if (part < 0) return unit;
+    const int t = part / p.splits, sl = part - t * p.splits;
+    kb_lo = sl * num_kb / p.splits;
+    kb_hi = (sl + 1) * num_kb / p.splits;
+    return full_tiles + t;
+  };
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
   if (warp == 0) {
@@ -174,13 +190,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
         asm volatile("fence.proxy.async.global;" ::: "memory");   // generic-proxy writes -> TMA reads
       }
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int m_blk, n_blk;
-        tile_coords(tile, p, m_blk, n_blk);
+      for (int unit = pair; unit < num_units && ok; unit += num_pairs) {
+        int m_blk, n_blk, kb_lo, kb_hi, part;
+        tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, m_blk, n_blk);
         const int m0 = m_blk * 256 + (int)rank * BM;
         // SwiGLU mode: the leader loads 128 gate rows, its peer the matching 128 up rows (F rows further down)
         const int n0 = p.swiglu_f > 0 ? n_blk * P_HALF + (int)rank * p.swiglu_f : n_blk * P_BN + (int)rank * P_HALF;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) {
             report(p, abort_word, ERR_WAIT_EMPTY);
             ok = false;
@@ -217,7 +233,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       uint32_t phase = 0, acc_phase[2] = {0, 0};
       int local = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
+      for (int unit = pair; unit < num_units && ok; unit += num_pairs, ++local) {
+        int kb_lo, kb_hi, part;
+        unit_tile(unit, kb_lo, kb_hi, part);
         const int acc = local & 1;
         if (!mbar_wait(&tmem_empty[acc], acc_phase[acc] ^ 1, abort_word)) {
           report(p, abort_word, ERR_WAIT_TMEM_EMPTY);
@@ -227,7 +245,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         acc_phase[acc] ^= 1;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * P_BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_word)) {
             report(p, abort_word, ERR_WAIT_FULL);
             ok = false;
@@ -242,7 +260,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                                          : make_smem_desc(a_base + k * (UMMA_K * 2), 16, 1024);
             const uint64_t b_desc = B_MN ? make_smem_desc(b_base + k * (UMMA_K * 128), 8192, 1024)
                                          : make_smem_desc(b_base + k * (UMMA_K * 2), 16, 1024);
-            umma_pair_f16_ss(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_pair_f16_ss(d_tmem, a_desc, b_desc, idesc, (kb > kb_lo || k > 0) ? 1u : 0u);
           }
           umma_commit_pair(&empty_bar[stage]);   // frees this stage in both CTAs
           if (++stage == P_STAGES) {
@@ -310,9 +328,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     int local = 0;
     uint32_t out_slab = 0;
     bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
-      int m_blk, n_blk;
-      tile_coords(tile, p, m_blk, n_blk);
+    for (int unit = pair; unit < num_units && ok; unit += num_pairs, ++local) {
+      int m_blk, n_blk, kb_lo, kb_hi, part;
+      tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, m_blk, n_blk);
       const int acc = local & 1;
       if (!mbar_wait(&tmem_full[acc], acc_phase[acc], abort_word)) {
         if (lane == 0) report(p, abort_word, ERR_WAIT_TMEM_FULL);
@@ -329,6 +347,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       // also makes the st.shared.v4 of a quarter warp conflict-free.  A warp alternates between its two slabs and
       // waits, before refilling one, until the store that last used it has read it.
       const int row0 = m_blk * 256 + (int)rank * BM + quarter * 32;
+      const int y0 = part < 0 ? row0 : part * 256 + (int)rank * BM + quarter * 32;      // row of the output or of the workspace
       auto emit = [&](const CUtensorMap* tm, int x, const uint32_t (&o)[32], bool add) {
         uint8_t* slab = smem_out + ((warp - 2) * 2 + (out_slab & 1)) * P_SLAB;
         ++out_slab;
@@ -342,12 +361,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         __syncwarp();
         if (lane == 0) {
           if (row0 < p.M) {
-            if (add) tma_reduce_add_2d(tm, slab, x, row0);
-            else tma_store_2d(tm, slab, x, row0);
+            if (add) tma_reduce_add_2d(tm, slab, x, y0);
+            else tma_store_2d(tm, slab, x, y0);
           }
           tma_store_commit();
         }
       };
+      if (part >= 0) {
+#pragma unroll 1
+        for (int c = 0; c < P_BN / 32; ++c) {
+          if (n0 + c * 32 >= p.N) break;
+          uint32_t o[32];
+          tmem_ld_32x32(taddr + c * 32, o);
+          tmem_ld_wait();
+          emit(&tmH, c * 32, o, false);
+        }
+        tc_fence_before();
+        mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+        continue;
+      }
       if (p.swiglu_f > 0 && p.tma_store) {
         // accumulator columns [0,128) are gate_j, [128,256) the matching up_j; three outputs per 64 columns
         const int col = n_blk * P_HALF;
@@ -573,6 +605,51 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
 }
 
+// The partial tiles of the last wave, added in slice order: block (tile, 8 rows), two rows and one float4 per thread.
+template <typename OUT>
+__global__ void __launch_bounds__(256)
+pair_tail_sum_kernel(const float4* __restrict__ ws, OUT* __restrict__ C, const GemmParams p) {
+  const int t = blockIdx.x >> 5, r0 = (blockIdx.x & 31) * 8 + (threadIdx.x >> 6), c = (threadIdx.x & 63) * 4;
+  int m_blk, n_blk;
+  tile_coords(p.full_tiles + t, p, m_blk, n_blk);
+  const int col = n_blk * P_BN + c;
+  if (col >= p.N) return;
+  const float4* src = ws + ((size_t)t * p.splits * 256 + r0) * 64 + (c >> 2);
+  float4 sum[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+  for (int s0 = 0; s0 < p.splits; s0 += 4) {
+    float4 v[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (s0 + u < p.splits) {
+        v[u][0] = __ldcs(src + (size_t)(s0 + u) * 256 * 64);
+        v[u][1] = __ldcs(src + (size_t)(s0 + u) * 256 * 64 + 4 * 64);
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (s0 + u < p.splits) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          sum[k].x += v[u][k].x; sum[k].y += v[u][k].y; sum[k].z += v[u][k].z; sum[k].w += v[u][k].w;
+        }
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int row = m_blk * 256 + r0 + 4 * k;
+    if (row >= p.M) break;
+    OUT* dst = C + (long long)row * p.ldc + col;
+    if constexpr (sizeof(OUT) == 2) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(sum[k].x, sum[k].y), pack_bf16x2(sum[k].z, sum[k].w));
+    } else {
+      if (p.epi == EPI_F32_ACC) {
+        const float4 o = *reinterpret_cast<const float4*>(dst);
+        sum[k].x += o.x; sum[k].y += o.y; sum[k].z += o.z; sum[k].w += o.w;
+      }
+      *reinterpret_cast<float4*>(dst) = sum[k];
+    }
+  }
+}
+
 template <bool A_MN, bool B_MN>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmH,
                        GemmParams p, int sms, cudaStream_t stream) {
@@ -587,8 +664,14 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   p.group_m = 8;
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   int pairs = sms / 2;
-  if (tiles < pairs) pairs = tiles;
+  const int units = p.splits > 1 ? p.full_tiles + (tiles - p.full_tiles) * p.splits : tiles;
+  if (units < pairs) pairs = units;
   kern<<<pairs * 2, P_THREADS, P_SMEM, stream>>>(tmA, tmB, tmC, tmH, p);
+  if (p.splits > 1) {
+    const unsigned grid = (unsigned)(tiles - p.full_tiles) * 32;
+    if (p.epi == EPI_BF16) pair_tail_sum_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((const float4*)p.ws, (__nv_bfloat16*)p.C, p);
+    else pair_tail_sum_kernel<float><<<grid, 256, 0, stream>>>((const float4*)p.ws, (float*)p.C, p);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -624,7 +707,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
                           const GatherTask* gather, const uint32_t* wait_counter, uint32_t wait_value,
                           uint32_t* status, cudaStream_t stream, const float* rope_cs = nullptr, int rope_seq = 0,
                           int rope_d = 0, int rope_dh = 0, int rope_ctx = 0, int swiglu_f = 0, void* H = nullptr,
-                          long long ldh = 0, const ReduceTask* reduce = nullptr, const GemmFinish* finish = nullptr) {
+                          long long ldh = 0, const ReduceTask* reduce = nullptr, const GemmFinish* finish = nullptr, int splits = 1, float* ws = nullptr) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return -10;
@@ -649,7 +732,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   else { p.gather.dst = nullptr; p.gather.done = nullptr; p.gather.shard_vec = 0; p.gather.world = 0; p.gather.rank = 0; }
   if (reduce != nullptr) p.reduce = *reduce;
   else p.reduce.n = 0;
-  p.splits = 1; p.ws = nullptr; p.tile_counters = nullptr; p.b_early = 0; p.head_gate = 0;
+  p.splits = 1; p.full_tiles = 0; p.ws = nullptr; p.tile_counters = nullptr; p.b_early = 0; p.head_gate = 0;
   p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;
   p.wait_counter = wait_counter; p.wait_value = wait_value; p.wait_limit_ns = g_counter_wait_limit_ns;
@@ -690,6 +773,12 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (splits > 1 && p.tma_store) {
+    const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN), rest = tiles % (sms / 2);
+    if (rest > 0 && make_tmap_out_2d(&tmH, true, ws, (uint64_t)rest * splits * 256, P_BN, P_BN, 32, 32) == 0) {
+      p.splits = splits; p.full_tiles = tiles - rest; p.ws = ws;
+    }
+  }
   if (a_mn && b_mn) return launch_pair<true, true>(tmA, tmB, tmC, tmH, p, sms, stream);
   if (a_mn) return launch_pair<true, false>(tmA, tmB, tmC, tmH, p, sms, stream);
   if (b_mn) return launch_pair<false, true>(tmA, tmB, tmC, tmH, p, sms, stream);
@@ -700,6 +789,42 @@ extern "C" int b200_gemm_bf16_pair(const void* A, const void* B, void* C, const 
                                    long long lda, long long ldb, long long ldc, long long ldr, int a_mn, int b_mn,
                                    int epi, uint32_t* status, cudaStream_t stream) {
   return gemm_pair_impl(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, nullptr, nullptr, 0, status, stream);
+}
+
+// Slices of K for the tiles of the last wave of a launch (1 = leave them whole) and the floats of workspace they need.  The estimate counts
+// k-blocks of 64 (0.27 us on a pair): a wave of slices, a pipeline fill of 8 per unit, and for the second launch 14 and 0.2 per partial tile.
+// Measured, us per weight gradient over 16384 rows, before (on one SM per 128 x 128 tile where that was better) -> now: 512 x 512 46 -> 18,
+// 768 x 2048 59 -> 44, 2304 x 768 58 -> 51, 2048 x 5504 319 -> 289, 6144 x 2048 342 -> 314.
+// cost_out (may be null): the launch's estimate in k-blocks.
+extern "C" long long b200_gemm_pair_tail_plan(int M, int N, int K, int* splits_out, double* cost_out) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  const int pairs = sms / 2, num_kb = (K + BK - 1) / BK;
+  const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN), rest = tiles % pairs;
+  double best = rest > 0 ? num_kb + 8 : 0;
+  *splits_out = 1;
+  if (rest > 0 && N % 4 == 0)
+    for (int s = 2; s <= 24 && s <= num_kb / 4; ++s) {
+      const int units = rest * s;
+      const double cost = ((units + pairs - 1) / pairs) * ((double)num_kb / s + 8) + 14 + 0.2 * units;
+      if (cost < 0.95 * best) { best = cost; *splits_out = s; }
+    }
+  if (cost_out != nullptr) *cost_out = best + (tiles / pairs) * (double)num_kb;
+  return *splits_out > 1 ? (long long)rest * *splits_out * 256 * P_BN : 0;
+}
+
+// b200_gemm_bf16_pair (epi 0, 1 or 3) whose last wave is contracted in `splits` slices, as planned above; `ws` (16-byte aligned) belongs to
+// this launch until it ends.
+extern "C" int b200_gemm_bf16_pair_tail(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                                        long long ldc, int a_mn, int b_mn, int epi, int splits, float* ws, long long ws_floats,
+                                        uint32_t* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (epi != EPI_BF16 && epi != EPI_F32 && epi != EPI_F32_ACC) return -11;
+  int planned = 1;
+  const long long need = b200_gemm_pair_tail_plan(M, N, K, &planned, nullptr);
+  if (splits != planned || (splits > 1 && (ws == nullptr || (reinterpret_cast<uintptr_t>(ws) & 15) || ws_floats < need))) return -12;
+  return gemm_pair_impl(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, epi, nullptr, nullptr, 0, status, stream, nullptr, 0, 0, 0,
+                        0, 0, nullptr, 0, nullptr, nullptr, splits, ws);
 }
 
 // K-major operands, epi 0, 1 or 3, accumulators finished first (see GemmFinish).

@@ -13,6 +13,7 @@ triton_swiglu.py:27-91, triton_cross_entropy.py:22-145, triton_adamw.py:134-191)
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from pathlib import Path
@@ -84,6 +85,7 @@ def _declare(lib):
         "b200_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, L, I, I, I, P, P],
         "b200_gemm_bf16_pair_gather": [P, P, P, P, I, I, I, L, L, L, L, I, I, I, P, P, ctypes.c_ulonglong, I, I, P, P,
                                        P, ctypes.c_uint, P, P],
+        "b200_gemm_bf16_pair_tail": [P, P, P, I, I, I, L, L, L, I, I, I, I, P, L, P, P],
         "b200_gemm_bf16_finish": [P, P, P, I, I, I, L, L, L, I, P, P, P],
         "b200_gemm_bf16_pair_finish": [P, P, P, I, I, I, L, L, L, I, P, P, P],
         "b200_gemm_bf16_splitk_finish": [P, P, P, I, I, I, L, L, L, I, P, P, L, P, I, P, P],
@@ -177,7 +179,7 @@ def check_status(device=None):
 
 # Kernels launched per launcher call (a launcher may issue several).  Used to count this package's
 # own launches inside a timed region.
-_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "embedding_bwd_sorted": 2, "xent": 3, "flash_bwd": 3, "latent_decode": 2, "grouped_decode": 2}
+_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "embedding_bwd_sorted": 2, "b200_gemm_bf16_pair_tail": 2, "xent": 3, "flash_bwd": 3, "latent_decode": 2, "grouped_decode": 2}
 _LAUNCHES = 0
 
 
@@ -238,6 +240,20 @@ def _pair_pays(m: int, n: int, sms: int = 148) -> bool:
     cost_pair = waves(-(-m // 256) * -(-n // 256), sms // 2)
     cost_single = waves(-(-m // 128) * -(-n // 128), sms) * 0.625
     return cost_pair <= cost_single
+
+
+@functools.lru_cache(maxsize=4096)
+def pair_tail_plan(m: int, n: int, k: int) -> tuple[int, int, bool]:
+    """For a weight gradient (layout 'tn') of this size: (K slices of the last wave's tiles on CTA pairs, floats of workspace they need,
+    whether the CTA pairs are the better kernel).  Costs are in 64-deep steps of a pair's 256 x 256 tile; a 128 x 128 tile on one SM takes 0.625
+    of that (see ``_pair_pays``)."""
+    lib = load()
+    fn = lib.b200_gemm_pair_tail_plan
+    fn.restype, fn.argtypes = c_ll, [c_int, c_int, c_int, c_void_p, c_void_p]
+    splits, cost = c_int(1), ctypes.c_double(0.0)
+    floats = int(fn(m, n, k, ctypes.byref(splits), ctypes.byref(cost)))
+    waves = -(-(-(-m // 128) * -(-n // 128)) // 148)
+    return splits.value, floats, cost.value <= waves * 0.625 * -(-k // 64) + 8
 
 
 def set_gemm_tma_store(on: bool) -> bool:
@@ -334,6 +350,12 @@ def gemm(a, b, layout: str, out=None, out_dtype=None, residual=None, accumulate=
         _rowmajor(residual, "residual")
         _req(residual.dtype == torch.bfloat16 and tuple(residual.shape) == (m, n), "residual must be bf16 (M,N)")
         ldr = residual.stride(0)
+    tail = (1, 0)
+    if (layout == "tn" and USE_PAIR and bn_hint == 0 and max_ctas == 0 and pair is not False and gather is None and reduce is None
+            and residual is None and not FORCE_PAIR and out.data_ptr() % 16 == 0 and out.stride(0) * out.element_size() % 16 == 0):
+        splits, floats, pays = pair_tail_plan(m, n, k)
+        if pays or pair:
+            pair, tail = True, (splits, floats)
     if pair is None:
         pair = USE_PAIR and bn_hint == 0 and max_ctas == 0 and (
             FORCE_PAIR or (m >= PAIR_MIN_M and n >= 256 and _pair_pays(m, n)))
@@ -359,6 +381,12 @@ def gemm(a, b, layout: str, out=None, out_dtype=None, residual=None, accumulate=
     if pair and finish is not None:
         _check(lib.b200_gemm_bf16_pair_finish(_ptr(a), _ptr(b), _ptr(out), m, n, k, lda, ldb, out.stride(0), epi & ~EPI_PAD_WRITABLE,
                                               ctypes.byref(finish), _ptr(status_word(a.device)), _stream()), "b200_gemm_bf16_pair")
+        return out
+    if pair and tail[0] > 1:
+        ws = torch.empty(tail[1], dtype=torch.float32, device=a.device)
+        _check(lib.b200_gemm_bf16_pair_tail(_ptr(a), _ptr(b), _ptr(out), m, n, k, lda, ldb, out.stride(0), a_mn, b_mn,
+                                            epi & ~EPI_PAD_WRITABLE, tail[0], _ptr(ws), ws.numel(), _ptr(status_word(a.device)),
+                                            _stream()), "b200_gemm_bf16_pair_tail")
         return out
     if pair:
         rc = lib.b200_gemm_bf16_pair(_ptr(a), _ptr(b), _ptr(out), _ptr(residual), m, n, k, lda, ldb, out.stride(0),

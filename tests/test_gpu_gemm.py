@@ -324,3 +324,29 @@ def test_gemm_early_weight_tiles_give_the_same_result(shape, max_ctas, pdl):
     finally:
         native.set_pdl(prev)
     _check(want, _ref(a, b, "nt") + res.float(), k)
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 512, 16384), (256, 256, 4000), (264, 272, 4104), (768, 2304, 8200), (2048, 5504, 8192), (2560, 2048, 8192),
+                                   (10000, 512, 4096), (8, 16, 9000)])
+def test_last_wave_in_slices(m, n, k):
+    """Weight gradients whose last wave of tiles is contracted in slices of K: fp32, accumulated and bf16 results, the same ones every time."""
+    from llm_systems_from_scratch_b200.ops import native
+    splits, floats, pays = native.pair_tail_plan(m, n, k)
+    assert splits > 1 and floats > 0
+    a, b = _make("tn", m, n, k, "cuda")
+    want = a.double().t() @ b.double()
+    # fp32 additions, truncated by the tensor core at worst: 16 products at a time, then the slices
+    bound = (k / 16 + 32) * 2.0 ** -23 * (a.double().abs().t() @ b.double().abs())
+    out = native.gemm(a, b, "tn", out_dtype=torch.float32, pair=True)
+    native.check_status()
+    assert bool(((out.double() - want).abs() <= bound).all())
+    assert torch.equal(out, native.gemm(a, b, "tn", out_dtype=torch.float32, pair=True))
+    whole = native.gemm(a, b, "tn", out_dtype=torch.float32, pair=False)
+    assert (out.double() - want).norm() <= 1.05 * (whole.double() - want).norm()
+    more = native.gemm(a, b, "tn", out=out.clone(), accumulate=True, pair=True)
+    assert bool(((more.double() - 2 * want).abs() <= 2 * bound + 2.0 ** -22 * want.abs()).all())
+    if n % 8 == 0:
+        assert torch.equal(native.gemm(a, b, "tn", pair=True), out.bfloat16())
+    wide = torch.full((m, n + 12), 7.0, device="cuda")
+    native.gemm(a, b, "tn", out=wide[:, :n], pair=True)
+    assert torch.equal(wide[:, :n], out) and bool((wide[:, n:] == 7.0).all())

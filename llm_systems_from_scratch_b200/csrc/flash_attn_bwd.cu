@@ -12,6 +12,9 @@
 //   flash_dq_kernel      CTA = 128 queries; walks 128-key steps j <= diagonal:
 //                          S = Q K_j^T, dP = dO V_j^T ; dS -> tensor memory ; dQ += dS K_j
 //
+// Heads of 32 columns (HW) run in the instances for 64: a box of 64 columns also holds those behind the head, which stay out of S and dP
+// (their contractions end at HW) and whose part of dQ, dK and dV is not stored.
+//
 // Roles per CTA: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warps 2-5 one tile row per thread.
 #include "ptx.cuh"
 
@@ -166,7 +169,7 @@ struct DkDvSmem {
   static constexpr int TOTAL = OFF_BAR + NUM_BARS * 8 + 16 + 1024;
 };
 
-template <int DH>
+template <int DH, int HW>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 over qkv
                   const __grid_constant__ CUtensorMap tm_q,    // box 64 x 64 over qkv
@@ -230,7 +233,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
   const uint32_t tm_dv = tmem_base + 256;   // DH columns
   const uint32_t tm_dk = tmem_base + 384;   // DH columns
 
-  const int col_q = h * DH, col_k = p.d + h * DH, col_v = 2 * p.d + h * DH;
+  const int col_q = h * HW, col_k = p.d + h * HW, col_v = 2 * p.d + h * HW;
 
   if (warp == 0) {
     if (elect_one()) {   // elect.sync keeps the issuing code warp-uniform (descriptors in uniform registers)
@@ -251,7 +254,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
 #pragma unroll
         for (int pn = 0; pn < L::PANELS; ++pn) {
           tma_load_2d(smem + L::OFF_Q + st * L::Q_TILE + pn * 8192, &tm_q, &qd_full[st], col_q + pn * 64, qrow);
-          tma_load_2d(smem + L::OFF_DO + st * L::Q_TILE + pn * 8192, &tm_do, &qd_full[st], h * DH + pn * 64, qrow);
+          tma_load_2d(smem + L::OFF_DO + st * L::Q_TILE + pn * 8192, &tm_do, &qd_full[st], h * HW + pn * 64, qrow);
         }
       }
     }
@@ -267,14 +270,14 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
         const uint32_t q_addr = smem_u32(smem + L::OFF_Q + rs * L::Q_TILE);
         const uint32_t do_addr = smem_u32(smem + L::OFF_DO + rs * L::Q_TILE);
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
+        for (int k = 0; k < HW / 16; ++k) {
           const uint32_t offa = (k / 4) * 16384 + (k % 4) * 32;   // 128-row panels
           const uint32_t offb = (k / 4) * 8192 + (k % 4) * 32;    // 64-row panels
           umma_f16_ss(tm_st + st * 64, make_smem_desc(k_addr + offa, 16, 1024), make_smem_desc(q_addr + offb, 16, 1024),
                       idesc_12, k > 0 ? 1u : 0u);
         }
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
+        for (int k = 0; k < HW / 16; ++k) {
           const uint32_t offa = (k / 4) * 16384 + (k % 4) * 32;
           const uint32_t offb = (k / 4) * 8192 + (k % 4) * 32;
           umma_f16_ss(tm_dpt + st * 64, make_smem_desc(v_addr + offa, 16, 1024),
@@ -412,12 +415,12 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
       __nv_bfloat16* dk_row = p.dqkv + (size_t)(row_base + key_idx) * 3 * p.d + col_k;
       __nv_bfloat16* dv_row = p.dqkv + (size_t)(row_base + key_idx) * 3 * p.d + col_v;
 #pragma unroll 1
-      for (int c = cg; c < DH / 32; c += BWD_CG) {   // each warpgroup stores its own 32-column slices
+      for (int c = cg; c < HW / 32; c += BWD_CG) {   // each warpgroup stores its own 32-column slices
         uint32_t a[32], g[32];
         tmem_ld_32x32(tm_dk + lane_addr + c * 32, a);
         tmem_ld_32x32(tm_dv + lane_addr + c * 32, g);
         tmem_ld_wait();
-        if (valid && p.rope_cs != nullptr) unrotate32<DH>(p, key_idx, c * 32, a);
+        if (valid && p.rope_cs != nullptr) unrotate32<HW>(p, key_idx, c * 32, a);
         if (valid) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -479,7 +482,7 @@ struct DqSmem {
   static constexpr int TOTAL = OFF_BAR + NUM_BARS * 8 + 16 + 1024;
 };
 
-template <int DH>
+template <int DH, int HW>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 over qkv
                 const __grid_constant__ CUtensorMap tm_do,    // box 64 x 128 over dO
@@ -545,7 +548,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
   const uint32_t tm_ds = tmem_base + 256;    // 2 x 64 columns of packed bf16 pairs
   const uint32_t tm_dq = tmem_base + 384;    // DH columns
 
-  const int col_q = h * DH, col_k = p.d + h * DH, col_v = 2 * p.d + h * DH;
+  const int col_q = h * HW, col_k = p.d + h * HW, col_v = 2 * p.d + h * HW;
 
   if (warp == 0) {
     if (elect_one()) {   // elect.sync keeps the issuing code warp-uniform (descriptors in uniform registers)
@@ -555,7 +558,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
 #pragma unroll
       for (int pn = 0; pn < L::PANELS; ++pn) {
         tma_load_2d(smem + L::OFF_Q + pn * 16384, &tm_qkv, qd_full, col_q + pn * 64, row_base + q0);
-        tma_load_2d(smem + L::OFF_DO + pn * 16384, &tm_do, qd_full, h * DH + pn * 64, row_base + q0);
+        tma_load_2d(smem + L::OFF_DO + pn * 16384, &tm_do, qd_full, h * HW + pn * 64, row_base + q0);
       }
       for (int t = 0; t < n_steps; ++t) {
         const int ks = t % DQ_KSTAGES, vs = t % DQ_VSTAGES;
@@ -595,12 +598,12 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
         const uint64_t k_desc = make_smem_desc(smem_u32(smem + L::OFF_K + (t % DQ_KSTAGES) * L::TILE), 16, 1024);
         const uint64_t v_desc = make_smem_desc(smem_u32(smem + L::OFF_V + (t % DQ_VSTAGES) * L::TILE), 16, 1024);
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
+        for (int k = 0; k < HW / 16; ++k) {
           const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4;
           umma_f16_ss(tm_s, q_desc + off, k_desc + off, idesc_12, k > 0 ? 1u : 0u);
         }
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
+        for (int k = 0; k < HW / 16; ++k) {
           const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4;
           umma_f16_ss(tm_dp, do_desc + off, v_desc + off, idesc_12, k > 0 ? 1u : 0u);
         }
@@ -708,11 +711,11 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
       tc_fence_after();
       __nv_bfloat16* dq_row = p.dqkv + (size_t)(row_base + q_idx) * 3 * p.d + col_q;
 #pragma unroll 1
-      for (int c = cg; c < DH / 32; c += BWD_CG) {
+      for (int c = cg; c < HW / 32; c += BWD_CG) {
         uint32_t a[32];
         tmem_ld_32x32(tm_dq + lane_addr + c * 32, a);
         tmem_ld_wait();
-        if (valid && p.rope_cs != nullptr) unrotate32<DH>(p, q_idx, c * 32, a);
+        if (valid && p.rope_cs != nullptr) unrotate32<HW>(p, q_idx, c * 32, a);
         if (valid) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
@@ -744,7 +747,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
   BWD_CTA_LOG_END(1, t_cta_start, n_steps);
 }
 
-template <int DH>
+template <int DH, int HW = DH>
 static int launch_flash_bwd(const void* qkv, const void* dout, const FlashBwdParams& p, cudaStream_t stream) {
   const uint64_t rows = (uint64_t)p.batch * p.seq;
   CUtensorMap tm_qkv128, tm_qkv64, tm_do128, tm_do64;
@@ -752,8 +755,8 @@ static int launch_flash_bwd(const void* qkv, const void* dout, const FlashBwdPar
   if (make_tmap_bf16_2d(&tm_qkv64, qkv, rows, 3ull * p.d, 3ull * p.d, 64, 64)) return -20;
   if (make_tmap_bf16_2d(&tm_do128, dout, rows, (uint64_t)p.d, (uint64_t)p.d, 64, 128)) return -20;
   if (make_tmap_bf16_2d(&tm_do64, dout, rows, (uint64_t)p.d, (uint64_t)p.d, 64, 64)) return -20;
-  auto k1 = flash_dkdv_kernel<DH>;
-  auto k2 = flash_dq_kernel<DH>;
+  auto k1 = flash_dkdv_kernel<DH, HW>;
+  auto k2 = flash_dq_kernel<DH, HW>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DkDvSmem<DH>::TOTAL) != cudaSuccess) return -3;
@@ -786,11 +789,11 @@ extern "C" void b200_flash_bwd_set_trace(long long* buf, int cta) {
 }
 
 // qkv (rows, 3d), o / dout (rows, d) bf16; lse (batch, heads, seq) from the forward; delta: scratch of the
-// same shape (fp32); dqkv (rows, 3d) bf16 receives dQ | dK | dV.  dh must be 64 or 128.
+// same shape (fp32); dqkv (rows, 3d) bf16 receives dQ | dK | dV.  dh must be 32, 64 or 128.
 static int flash_bwd_impl(const void* qkv, const void* o, const void* dout, const float* lse, float* delta, void* dqkv,
                           int batch, int seq, int heads, int dh, float scale, const float* rope_cs, int rope_ctx,
                           uint32_t* status, cudaStream_t stream) {
-  if (dh != 64 && dh != 128) return -10;
+  if (dh != 32 && dh != 64 && dh != 128) return -10;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout) |
        reinterpret_cast<uintptr_t>(dqkv)) & 15)
     return -10;
@@ -804,6 +807,9 @@ static int flash_bwd_impl(const void* qkv, const void* o, const void* dout, cons
     if (dh == 128)
       flash_delta_kernel<128><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                     delta, items, seq, heads);
+    else if (dh == 32)
+      flash_delta_kernel<32><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+                                                                   delta, items, seq, heads);
     else
       flash_delta_kernel<64><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                    delta, items, seq, heads);
@@ -815,6 +821,7 @@ static int flash_bwd_impl(const void* qkv, const void* o, const void* dout, cons
   p.status = status;
   p.rope_cs = rope_cs; p.rope_ctx = rope_ctx;
   p.trace = g_bwd_trace; p.trace_cta = g_bwd_trace_cta;
+  if (dh == 32) return launch_flash_bwd<64, 32>(qkv, dout, p, stream);
   return dh == 64 ? launch_flash_bwd<64>(qkv, dout, p, stream) : launch_flash_bwd<128>(qkv, dout, p, stream);
 }
 

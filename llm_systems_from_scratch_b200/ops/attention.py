@@ -1,7 +1,7 @@
 """Causal attention on packed QKV: tcgen05 FlashAttention forward/backward wrappers.
 
 qkv is (batch*seq, 3*H*dh) row-major (Q | K | V, heads inside each third); o is (batch*seq, H*dh).
-Head sizes 64 and 128 run on the tensor-core kernels; other multiples of 8 up to 128 are zero-padded
+Head sizes 32, 64 and 128 run on the tensor-core kernels; other multiples of 8 up to 128 are zero-padded
 to the next supported size around the call (the scale keeps the true head size).
 
 Replaces the reference's attention call (llm-core/llm_core/model.py:381-385: ``scaled_dot_product_attention`` with
@@ -32,10 +32,10 @@ def _unpad_heads(t: torch.Tensor, parts: int, n_heads: int, dh: int, dh_pad: int
 
 
 def _supported(dh: int) -> int:
-    if dh in (64, 128):
+    if dh in (32, 64, 128):
         return dh
     _req(dh % 8 == 0 and dh <= 128, "head size must be a multiple of 8 and at most 128")
-    return 64 if dh < 64 else 128
+    return 32 if dh < 32 else 64 if dh < 64 else 128
 
 
 def attention_fwd(qkv, batch: int, seq: int, n_heads: int):

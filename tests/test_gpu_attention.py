@@ -76,3 +76,33 @@ def test_rope_fused_into_qkv_gemm_and_attention_backward(b, s, h, dh):
     native.check_status()
     assert (a.float() - plain.float()).abs().max().item() < 3e-2 * max(1.0, plain.float().abs().max().item())
     assert torch.equal(a[:, 2 * d:], plain[:, 2 * d:])
+
+
+@pytest.mark.parametrize("b,s,h,dh", [(1, 1, 2, 32), (2, 127, 3, 32), (1, 129, 5, 32), (2, 256, 16, 32), (1, 300, 1, 32), (1, 130, 2, 16)])
+def test_narrow_heads(b, s, h, dh):
+    """Heads narrower than the boxes they are loaded in, beside a head that holds infinities (in a sequence of its own) and with rotation."""
+    from llm_systems_from_scratch_b200.models.transformer import RotaryEmbedding
+    from llm_systems_from_scratch_b200.ops import attention, native, torch_impl
+    qkv = _rand_qkv(b, s, h, dh, seed=3)
+    do = torch.randn(b * s, h * dh, device="cuda").bfloat16()
+    ro, rl = torch_impl.attention_fwd(qkv.float(), b, s, h)
+    ref = torch_impl.attention_bwd(do.float(), qkv.float(), ro, rl, b, s, h)
+    clean = torch.ones(h, dtype=torch.bool)
+    if h > 1:
+        clean[-1] = False
+        qkv.view(b * s, 3, h, dh)[:, :, -1] = float("inf")
+    o, lse = attention.attention_fwd(qkv, b, s, h)
+    dqkv = attention.attention_bwd(do, qkv, o, lse, b, s, h)
+    native.check_status()
+    assert (o.view(b * s, h, dh)[:, clean].float() - ro.view(b * s, h, dh)[:, clean]).abs().max().item() < 2e-2
+    assert (lse[:, clean] - rl[:, clean]).abs().max().item() < 2e-2
+    got, want = (t.view(b * s, 3, h, dh)[:, :, clean].float() for t in (dqkv, ref))
+    assert (got - want).abs().max().item() < 5e-2 * max(1.0, want.abs().max().item() / 4)
+    cu = torch.arange(b + 1, dtype=torch.int32, device="cuda") * s
+    ov = attention.varlen_attention_fwd(qkv, cu, s, h)
+    assert torch.equal(ov.view(b * s, h, dh)[:, clean], o.view(b * s, h, dh)[:, clean])
+    cache = RotaryEmbedding._build_cache(s + 5, dh, 10000.0).cuda().contiguous()
+    turned = attention.attention_bwd(do, qkv, o, lse, b, s, h, rope_cache=cache)
+    plain = native.rope_(dqkv.contiguous(), cache, None, h, True, s)
+    a, c = (t.view(b * s, 3, h, dh)[:, :, clean].float() for t in (turned, plain))
+    assert (a - c).abs().max().item() < 3e-2 * max(1.0, c.abs().max().item())

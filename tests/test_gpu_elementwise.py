@@ -124,6 +124,23 @@ def test_argmax():
     assert torch.equal(got, x[:, :50257].float().argmax(-1))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("cols", [1, 3, 8, 9, 1023, 8191, 32768, 32775])
+@pytest.mark.parametrize("start", [0, 1, 7])
+def test_argmax_of_rows_that_start_anywhere(dtype, cols, start):
+    from llm_systems_from_scratch_b200.ops import native
+    x = torch.randn(7, start + cols + 5, generator=torch.Generator().manual_seed(cols)).to(dtype).cuda()[:, start:]
+    x[:, cols:] = 99.0
+    x[1, :cols] = -torch.inf
+    x[2, :cols] = torch.finfo(dtype).min
+    x[3, cols - 1] = x[3, cols // 2] = 50.0
+    x[4, 0] = torch.inf
+    x[5, :cols - 1] = torch.nan          # the oracle below would answer with the NaN: the kernel takes no NaN
+    want = x[:, :cols].float().nan_to_num(nan=-torch.inf, posinf=torch.inf, neginf=-torch.inf).argmax(-1).tolist()
+    want[5] = cols - 1
+    assert native.argmax_rows(x, valid_cols=cols).tolist() == want
+
+
 @pytest.mark.parametrize("n,gdt", [(1 << 20, torch.float32), (12345, torch.bfloat16), (4, torch.float32)])
 def test_adamw_matches_reference_order(n, gdt):
     from llm_systems_from_scratch_b200.ops import native, torch_impl

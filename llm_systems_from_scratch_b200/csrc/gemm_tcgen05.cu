@@ -79,7 +79,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         tile_coords(GROUP == GROUP_COLS ? tile % per_problem : tile, p, m_blk, n_blk);
         const int brow = (GROUP == GROUP_COLS ? (tile / per_problem) * p.group_rows : 0) + n_blk * (SWIGLU ? BN / 2 : BN);
         for (int i = 0; i < STAGES && kb_lo + i < kb_hi; ++i) {
-          mbar_expect_tx(&full_bar[i], S::A_BYTES + S::B_BYTES);
+          mbar_expect_tx(&full_bar[i], p.row_step * (BK * 2) + S::B_BYTES);
           tma_load_2d(smem_b + i * S::B_BYTES, &tmB, &full_bar[i], (kb_lo + i) * BK, brow);
           if (SWIGLU) tma_load_2d(smem_b + i * S::B_BYTES + S::B_BYTES / 2, &tmB, &full_bar[i], (kb_lo + i) * BK, brow + p.N);
         }
@@ -123,7 +123,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (GROUP == GROUP_ROWS) group = p.tile_group[m_blk];
         if (GROUP == GROUP_COLS) group = tile / tiles_one;
         if (GROUP == GROUP_ROWS && group < 0) continue;
-        const int m0 = m_blk * BM, n0 = (GROUP != GROUP_NONE ? group * p.group_rows : 0) + n_blk * BN_OUT;
+        const int m0 = m_blk * p.row_step, n0 = (GROUP != GROUP_NONE ? group * p.group_rows : 0) + n_blk * BN_OUT;
         if (unit != (int)blockIdx.x) early = 0;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           const bool posted = kb - kb_lo < early;
@@ -132,7 +132,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             ok = false;
             break;
           }
-          if (!posted) mbar_expect_tx(&full_bar[stage], S::A_BYTES + S::B_BYTES);
+          if (!posted) mbar_expect_tx(&full_bar[stage], p.row_step * (BK * 2) + S::B_BYTES);
           uint8_t* a_dst = smem_a + stage * S::A_BYTES;
           uint8_t* b_dst = smem_b + stage * S::B_BYTES;
           const int k0 = kb * BK;
@@ -233,7 +233,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       acc_phase[acc] ^= 1;
       tc_fence_after();
       const int row_in_tile = quarter * 32 + lane;
-      const int row = m_blk * BM + row_in_tile;
+      if (quarter * 32 >= p.row_step) {       // none of this warp's rows was loaded
+        tc_fence_before();
+        mbar_arrive(&tmem_empty[acc]);
+        continue;
+      }
+      const int row = row_in_tile < p.row_step ? m_blk * p.row_step + row_in_tile : p.M;
       const int n0 = n_blk * BN_OUT;
       const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc * BN;
       if (SWIGLU) {
@@ -417,6 +422,15 @@ static int num_sms() {
   return g_num_sms;
 }
 
+// Rows of a row tile.  With one or two row tiles (decode, short prompts) only the rows that exist are copied, in equal tiles of a
+// multiple of 8: TMA takes longer over rows outside the matrix than over rows inside (one row, N x K = 6144 x 2048: 17.0 -> 9.3 us,
+// where 128 rows take 9.9; 2048 x 2048 12.4 -> 8.5, 11008 x 2048 18.4 -> 12.6).  The rest of the tile in shared memory keeps what was
+// there; it meets rows of the accumulator that nobody reads.
+static int row_step_of(int M) {
+  const int mt = (M + BM - 1) / BM;
+  return mt > 2 ? BM : ((M + mt - 1) / mt + 7) / 8 * 8;
+}
+
 template <int BN, bool A_MN, bool B_MN, int GROUP = GROUP_NONE, bool SWIGLU = false>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, int max_ctas, cudaStream_t stream) {
   constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? 6 : 8);
@@ -427,7 +441,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return -3;
     configured = true;
   }
-  p.num_m_tiles = (p.M + BM - 1) / BM;
+  p.num_m_tiles = (p.M + p.row_step - 1) / p.row_step;
   constexpr int BN_OUT = SWIGLU ? BN / 2 : BN;
   p.num_n_tiles = (p.N + BN_OUT - 1) / BN_OUT;
   p.group_m = 16;
@@ -490,12 +504,13 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* R, 
     const long long w128 = (mt * ((N + 127) / 128) + sms - 1) / sms * 128 * 11;
     bn = (w128 < w256) ? 128 : 256;
   }
+  const int row_step = a_mn ? BM : row_step_of(M);
   CUtensorMap tmA, tmB;
   int rc;
   if (a_mn)
     rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, 64);
   else
-    rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BM);
+    rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, row_step);
   if (rc) return -20 + rc;
   if (b_mn)
     rc = make_tmap_bf16_2d(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, 64);
@@ -515,6 +530,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* R, 
   p.swiglu_f = 0; p.H = nullptr; p.ldh = 0;
   p.splits = splits > 1 ? splits : 1; p.ws = ws; p.tile_counters = tile_counters;
   p.b_early = b_early;
+  p.row_step = row_step;
   p.tile_group = nullptr; p.group_rows = 0; p.batch = 1; p.a_step = p.c_step = 0; p.relu = 0; p.head_gate = 0;
   p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;
@@ -660,7 +676,8 @@ extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, con
   CUtensorMap tmA, tmB;
   const uint64_t a_cols = rows ? (uint64_t)K : (uint64_t)(batch - 1) * a_step + K;
   const uint64_t b_rows = rows ? (uint64_t)n_groups * group_rows : (uint64_t)batch * group_rows;
-  int rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)M, a_cols, (uint64_t)lda, 64, BM);
+  const int row_step = rows ? BM : row_step_of(M);
+  int rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)M, a_cols, (uint64_t)lda, 64, row_step);
   if (rc) return -20 + rc;
   rc = make_tmap_bf16_2d(&tmB, B, b_rows, (uint64_t)K, (uint64_t)ldb, 64, swiglu ? bn / 2 : bn);
   if (rc) return -30 + rc;
@@ -676,6 +693,7 @@ extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, con
   p.swiglu_f = 0; p.H = nullptr; p.ldh = 0;
   p.splits = 1; p.ws = nullptr; p.tile_counters = nullptr;
   p.b_early = b_early;
+  p.row_step = row_step;
   p.tile_group = tile_group; p.group_rows = group_rows; p.batch = rows ? 1 : batch; p.a_step = a_step; p.c_step = c_step; p.relu = swiglu == 2;
   p.head_gate = head_gate; p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;

@@ -350,3 +350,27 @@ def test_last_wave_in_slices(m, n, k):
     wide = torch.full((m, n + 12), 7.0, device="cuda")
     native.gemm(a, b, "tn", out=wide[:, :n], pair=True)
     assert torch.equal(wide[:, :n], out) and bool((wide[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("epilogue", ["bf16", "residual", "fp32", "accumulate"])
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 31, 33, 120, 127, 128, 129, 144, 200, 241, 256, 257])
+@pytest.mark.parametrize("n,k", [(40, 72), (1000, 512), (512, 4160)])
+def test_row_tiles_of_the_rows_that_exist(m, n, k, epilogue):
+    from llm_systems_from_scratch_b200.ops import native
+    g = torch.Generator("cuda").manual_seed(m)
+    a, b = (torch.randn(r, k, generator=g, device="cuda").bfloat16() for r in (m, n))
+    base = torch.randn(m + 3, n, generator=g, device="cuda")
+    want = a.double() @ b.double().T
+    if epilogue == "residual":
+        res = base[:m].bfloat16()
+        got, want = native.gemm(a, b, "nt", residual=res), want + res.double()
+    elif epilogue == "bf16":
+        got = native.gemm(a, b, "nt", b_stable=True)
+    else:
+        out = base.clone()
+        got = native.gemm(a, b, "nt", out=out[:m], accumulate=epilogue == "accumulate")
+        want = want + base[:m].double() if epilogue == "accumulate" else want
+        assert torch.equal(out[m:], base[m:])
+    # fp32 sums of k products of size 1 (4e-6 of the norm at this k), then one rounding to bf16 (2^-9)
+    assert (got.double() - want).norm() <= (2e-5 if got.dtype == torch.float32 else 2.0 ** -8) * want.norm()
+    native.check_status()

@@ -86,6 +86,7 @@ def _declare(lib):
         "b200_gemm_bf16_pair_gather": [P, P, P, P, I, I, I, L, L, L, L, I, I, I, P, P, ctypes.c_ulonglong, I, I, P, P,
                                        P, ctypes.c_uint, P, P],
         "b200_gemm_bf16_pair_tail": [P, P, P, I, I, I, L, L, L, I, I, I, I, P, L, P, P],
+        "b200_gemm_few_rows": [P, P, P, P, I, I, I, L, L, L, L, I, I, P, P, P],
         "b200_gemm_bf16_finish": [P, P, P, I, I, I, L, L, L, I, P, P, P],
         "b200_gemm_bf16_pair_finish": [P, P, P, I, I, I, L, L, L, I, P, P, P],
         "b200_gemm_bf16_splitk_finish": [P, P, P, I, I, I, L, L, L, I, P, P, L, P, I, P, P],
@@ -395,6 +396,11 @@ def gemm(a, b, layout: str, out=None, out_dtype=None, residual=None, accumulate=
         return out
     if b_stable and layout == "nt":
         epi |= EPI_B_STABLE
+    if layout == "nt" and bn_hint == 0 and max_ctas == 0 and few_rows(m, n) and (finish is None or finish.act != ACT_GELU):
+        _check(lib.b200_gemm_few_rows(_ptr(a), _ptr(b), _ptr(out), _ptr(residual), m, n, k, lda, ldb, out.stride(0), ldr, epi, 0,
+                                      None if finish is None else ctypes.byref(finish), _ptr(status_word(a.device)), _stream()),
+               "b200_gemm_few_rows")
+        return out
     if USE_SPLITK and layout == "nt" and m <= SPLITK_MAX_M and k >= SPLITK_MIN_K and bn_hint == 0 and max_ctas == 0:
         scratch = _splitk_scratch(a.device)
         if scratch is not None:
@@ -445,6 +451,16 @@ def _splitk_scratch(device):
         counters = torch.zeros(int(lib.b200_gemm_splitk_counters()), dtype=torch.int32, device=device)
         got = _SPLITK_SCRATCH[key] = (ws, counters)
     return got
+
+
+# The kernel for few rows of A (csrc/gemm_few_rows.cu), by size alone: its tiles are 128 output columns, and they have to leave it room to
+# cut K in slices (74 tiles in two slices are one CTA on each of 148 SMs).
+FEW_ROWS_MAX_M, FEW_ROWS_MAX_TILES = 64, 74
+ACT_GELU = 1
+
+
+def few_rows(m: int, n: int) -> bool:
+    return m <= FEW_ROWS_MAX_M and -(-n // 128) <= FEW_ROWS_MAX_TILES
 
 
 def splitk_plan(m: int, n: int, k: int) -> tuple[int, int]:

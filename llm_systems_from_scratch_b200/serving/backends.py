@@ -11,6 +11,7 @@ import torch
 
 from .. import ops
 from ..ops import mixer_ops as mo
+from ..ops import native
 from ..ops import serving_ops
 from .kv_cache import LayerCache, PagedKVCache, StateSpec
 
@@ -59,8 +60,11 @@ class TransformerBackend:
         o = attend(qkv, li)
         x = ops.gemm(o, w.wo, "nt", residual=x, b_stable=True)
         h, _ = ops.rmsnorm_fwd(x, w.n2, cfg.eps)
-        gu = ops.gemm(h, w.wgu, "nt", b_stable=True)
-        return ops.gemm(ops.silu_mul_fwd(gu), w.wdown, "nt", residual=x, b_stable=True)
+        if x.is_cuda and native.few_rows(x.shape[0], cfg.d_ff):
+            h = mo.glu(h, w.wgu, cfg.d_ff, "silu")
+        else:
+            h = ops.silu_mul_fwd(ops.gemm(h, w.wgu, "nt", b_stable=True))
+        return ops.gemm(h, w.wdown, "nt", residual=x, b_stable=True)
 
     def forward(self, batch):
         heads = self.cfg.n_heads

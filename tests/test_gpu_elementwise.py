@@ -288,3 +288,12 @@ def test_scale_by_one_and_others():
             want = (x.float() * c).to(dt)
             got = native.scale_(x.clone(), torch.tensor(c, device="cuda"))
             assert torch.equal(torch.nan_to_num(got, 7.0), torch.nan_to_num(want, 7.0))
+
+
+def test_launches_go_to_the_current_stream():
+    from llm_systems_from_scratch_b200.ops import native
+    assert native._stream() == torch.cuda.current_stream().cuda_stream
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert native._stream() == side.cuda_stream == torch.cuda.current_stream().cuda_stream
+    assert native._stream() != side.cuda_stream

@@ -402,6 +402,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const __grid_constan
     tmem_alloc(tmem_holder, 128);
     tmem_relinquish();
   }
+  __syncthreads();          // the CTA holds its tensor memory
   pdl_sync();
   const int rep = p.heads / p.kv_heads, sets = (rep + DP_HEADS - 1) / DP_HEADS, set = blockIdx.x % sets;
   const int hk = blockIdx.x / sets % p.kv_heads, chunk = blockIdx.x / (sets * p.kv_heads), D = p.dim;
@@ -719,6 +720,7 @@ __global__ void __launch_bounds__(DK_THREADS, 1) delta_chunk_kernel(const __grid
     *reinterpret_cast<uint4*>(smem + L::OFF_ONE + dl_swz(r, c8)) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   fence_proxy_async_smem();
+  __syncthreads();          // the CTA holds its tensor memory
   pdl_sync();
   const int seq = blockIdx.x / p.heads, h = blockIdx.x - seq * p.heads, hk = h / (p.heads / p.kv_heads), D = p.dim, E = p.vdim;
   const int row0 = p.cu[seq], rows = p.cu[seq + 1] - row0, slot = p.state_slots[seq];

@@ -167,6 +167,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int rows, int d) {
+  pdl_sync();
   __shared__ float red[32];
   float wreg[RMS_BWD_MAXC][8];
   float dwacc[RMS_BWD_MAXC][8];
@@ -271,6 +272,7 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
                         const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                         const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_partial, int rows) {
+  pdl_sync();
   constexpr int D = NC * 256;
   __shared__ float dw_s[D];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -349,6 +351,7 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
 constexpr int RMS_DW_GROUPS = 32;
 __global__ void __launch_bounds__(32 * RMS_DW_GROUPS)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nparts, int d, int accumulate) {
+  pdl_sync();
   __shared__ float sm[RMS_DW_GROUPS][33];
   const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + x;
@@ -395,6 +398,7 @@ __global__ void silu_mul_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_b
 
 __global__ void silu_mul_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gu,
                                     __nv_bfloat16* __restrict__ dgu, long long rows, int F) {
+  pdl_sync();
   const long long groups = rows * (F / 8);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < groups;
        i += (long long)gridDim.x * blockDim.x) {
@@ -515,6 +519,7 @@ __global__ void __launch_bounds__(256)
 embedding_bwd_sorted_kernel(const long long* __restrict__ sorted_tokens, const long long* __restrict__ order,
                             const __nv_bfloat16* __restrict__ dx, OUT* __restrict__ grad_table, float* __restrict__ parts,
                             long long rows, int d, int vocab, int accumulate) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const long long seg = blockIdx.x * 8ll + (threadIdx.x >> 5);
   const long long j0 = seg * EMB_SEG;
@@ -568,6 +573,7 @@ template <typename OUT>
 __global__ void __launch_bounds__(256)
 embedding_bwd_join_kernel(const long long* __restrict__ sorted_tokens, const float* __restrict__ parts, OUT* __restrict__ grad_table,
                           long long rows, int d, int vocab, int accumulate) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const long long seg = blockIdx.x * 8ll + (threadIdx.x >> 5);
   const long long j0 = seg * EMB_SEG, j1 = j0 + EMB_SEG;
@@ -613,6 +619,7 @@ constexpr int XENT_THREADS = 512;
 
 __global__ void count_valid_kernel(const long long* __restrict__ targets, long long rows, int ignore_index,
                                    float* __restrict__ n_valid) {
+  pdl_sync();
   __shared__ float red[32];
   float c = 0.f;
   for (long long i = threadIdx.x; i < rows; i += blockDim.x) c += (targets[i] != ignore_index) ? 1.f : 0.f;
@@ -624,6 +631,7 @@ __global__ void __launch_bounds__(XENT_THREADS)
 xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ row_loss,
             const float* __restrict__ n_valid, long long ld, int vocab, int ignore_index, float grad_scale,
             int write_grad) {
+  pdl_sync();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
@@ -675,6 +683,7 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
 
 // loss (=|+=) sum(row_loss) in a fixed order (single block).
 __global__ void sum_rows_kernel(const float* __restrict__ v, long long n, float* __restrict__ out, int accumulate) {
+  pdl_sync();
   __shared__ float red[32];
   float s = 0.f;
   for (long long i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
@@ -750,6 +759,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const GradT* __restrict__ g,
                              float* __restrict__ v, __nv_bfloat16* __restrict__ mirror, long long n,
                              const float* __restrict__ gscale, float lr, float b1, float b2, float eps, float wd,
                              float alpha_t) {
+  pdl_sync();
   const float gs = gscale ? *gscale : 1.f;
   const long long nvec = n / 4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
@@ -799,6 +809,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const GradT* __restrict__ g,
 // order (fixed summation order => bitwise reproducible gradient norm).
 template <typename T>
 __global__ void sumsq_partials_kernel(const T* __restrict__ x, long long n, float* __restrict__ partials) {
+  pdl_sync();
   __shared__ float red[32];
   float s = 0.f;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -811,6 +822,7 @@ __global__ void sumsq_partials_kernel(const T* __restrict__ x, long long n, floa
 }
 
 __global__ void sumsq_finish_kernel(const float* __restrict__ partials, int n, float* __restrict__ out) {
+  pdl_sync();
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += partials[i];   // fixed assignment of partials to threads
@@ -835,6 +847,7 @@ __global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __rest
 // coef = min(1, max_norm / (sqrt(sumsq) + 1e-6)); also stores the norm.
 __global__ void clip_coef_kernel(const float* __restrict__ sumsq, float max_norm, float* __restrict__ coef,
                                  float* __restrict__ norm_out) {
+  pdl_sync();
   const float nrm = sqrtf(*sumsq);
   if (norm_out) *norm_out = nrm;
   *coef = fminf(1.f, max_norm / (nrm + 1e-6f));
@@ -842,6 +855,7 @@ __global__ void clip_coef_kernel(const float* __restrict__ sumsq, float max_norm
 
 template <typename T>
 __global__ void scale_kernel(T* __restrict__ x, long long n, const float* __restrict__ coef) {
+  pdl_sync();
   // 16-byte accesses over the aligned body, scalar head and tail.  A factor of one (the gradient of a loss that is not scaled, a
   // norm below the clipping limit) leaves every value as it is: nothing is read or written (124 us at a head of 50257 x 2048).
   const float c = *coef;
@@ -967,7 +981,7 @@ extern "C" int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
     const int parts = 148;        // <= b200_rmsnorm_bwd_parts(rows) partial rows of the scratch are used
 #define RMS_BWD_ROWS(NC)                                                                                     \
   case NC:                                                                                                   \
-    rmsnorm_bwd_rows_kernel<NC><<<parts, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,    \
+    launch_dep(rmsnorm_bwd_rows_kernel<NC>, parts, 256, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,    \
                                                        (const __nv_bfloat16*)w, rstd,                        \
                                                        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx,       \
                                                        dw_partial, rows);                                    \
@@ -977,12 +991,12 @@ extern "C" int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
       RMS_BWD_ROWS(5); RMS_BWD_ROWS(6); RMS_BWD_ROWS(7); RMS_BWD_ROWS(8);
     }
 #undef RMS_BWD_ROWS
-    rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st>>>(dw_partial, dw, parts, d, accumulate_dw);
+    launch_dep(rmsnorm_dw_reduce_kernel, (d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st, dw_partial, dw, parts, d, accumulate_dw);
     CHECK_LAUNCH();
   }
   const int parts = b200_rmsnorm_bwd_parts(rows);
 #define RMS_BWD_LAUNCH(C)                                                                                   \
-  rmsnorm_bwd_kernel<C><<<parts, RMS_BWD_THREADS, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, \
+  launch_dep(rmsnorm_bwd_kernel<C>, parts, RMS_BWD_THREADS, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, \
                                                            (const __nv_bfloat16*)w, rstd,                     \
                                                            (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx,    \
                                                            dw_partial, rows, d)
@@ -990,7 +1004,7 @@ extern "C" int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
   else if (d <= 4096) RMS_BWD_LAUNCH(2);
   else RMS_BWD_LAUNCH(4);
 #undef RMS_BWD_LAUNCH
-  rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st>>>(dw_partial, dw, parts, d, accumulate_dw);
+  launch_dep(rmsnorm_dw_reduce_kernel, (d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st, dw_partial, dw, parts, d, accumulate_dw);
   CHECK_LAUNCH();
 }
 
@@ -1005,7 +1019,7 @@ extern "C" int b200_silu_mul_fwd(const void* gu, void* h, long long rows, int F,
 extern "C" int b200_silu_mul_bwd(const void* dh, const void* gu, void* dgu, long long rows, int F, cudaStream_t st) {
   if (F % 8 || !ALIGNED16(gu) || !ALIGNED16(dh) || !ALIGNED16(dgu)) return -10;
   if (rows == 0) return 0;
-  silu_mul_bwd_kernel<<<grid_for(rows * (F / 8), 256), 256, 0, st>>>((const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu,
+  launch_dep(silu_mul_bwd_kernel, grid_for(rows * (F / 8), 256), 256, 0, st, (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu,
                                                                      (__nv_bfloat16*)dgu, rows, F);
   CHECK_LAUNCH();
 }
@@ -1051,9 +1065,9 @@ static int embedding_bwd_sorted(const long long* sorted_tokens, const long long*
   if (rows == 0) return 0;
   const long long segs = (rows + EMB_SEG - 1) / EMB_SEG;
   const dim3 grid((unsigned)((segs + 7) / 8), (unsigned)((d + 255) / 256));
-  embedding_bwd_sorted_kernel<OUT><<<grid, 256, 0, st>>>(sorted_tokens, order, (const __nv_bfloat16*)dx, grad_table, parts, rows, d, vocab,
+  launch_dep(embedding_bwd_sorted_kernel<OUT>, grid, 256, 0, st, sorted_tokens, order, (const __nv_bfloat16*)dx, grad_table, parts, rows, d, vocab,
                                                          accumulate);
-  embedding_bwd_join_kernel<OUT><<<grid, 256, 0, st>>>(sorted_tokens, parts, grad_table, rows, d, vocab, accumulate);
+  launch_dep(embedding_bwd_join_kernel<OUT>, grid, 256, 0, st, sorted_tokens, parts, grad_table, rows, d, vocab, accumulate);
   CHECK_LAUNCH();
 }
 
@@ -1080,12 +1094,12 @@ extern "C" int b200_xent(void* logits, const long long* targets, float* loss, fl
   if (rows == 0) return 0;
   const float* n_valid = n_valid_in;
   if (n_valid == nullptr) {
-    count_valid_kernel<<<1, 1024, 0, st>>>(targets, rows, ignore_index, scratch + rows);
+    launch_dep(count_valid_kernel, 1, 1024, 0, st, targets, rows, ignore_index, scratch + rows);
     n_valid = scratch + rows;
   }
-  xent_kernel<<<(unsigned)rows, XENT_THREADS, 0, st>>>((__nv_bfloat16*)logits, targets, scratch, n_valid, ld, vocab,
+  launch_dep(xent_kernel, (unsigned)rows, XENT_THREADS, 0, st, (__nv_bfloat16*)logits, targets, scratch, n_valid, ld, vocab,
                                                        ignore_index, grad_scale, write_grad);
-  sum_rows_kernel<<<1, 1024, 0, st>>>(scratch, rows, loss, accumulate_loss);
+  launch_dep(sum_rows_kernel, 1, 1024, 0, st, scratch, rows, loss, accumulate_loss);
   CHECK_LAUNCH();
 }
 
@@ -1105,10 +1119,10 @@ extern "C" int b200_adamw(float* p, const void* g, int grad_is_bf16, float* m, f
   if (n == 0) return 0;
   const int grid = grid_for(n / 4 + 4, 256, 148 * 8);
   if (grad_is_bf16)
-    adamw_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, (const __nv_bfloat16*)g, m, v, (__nv_bfloat16*)mirror, n, gscale,
+    launch_dep(adamw_kernel<__nv_bfloat16>, grid, 256, 0, st, p, (const __nv_bfloat16*)g, m, v, (__nv_bfloat16*)mirror, n, gscale,
                                                       lr, b1, b2, eps, wd, alpha_t);
   else
-    adamw_kernel<float><<<grid, 256, 0, st>>>(p, (const float*)g, m, v, (__nv_bfloat16*)mirror, n, gscale, lr, b1, b2, eps,
+    launch_dep(adamw_kernel<float>, grid, 256, 0, st, p, (const float*)g, m, v, (__nv_bfloat16*)mirror, n, gscale, lr, b1, b2, eps,
                                               wd, alpha_t);
   CHECK_LAUNCH();
 }
@@ -1121,9 +1135,9 @@ extern "C" int b200_sumsq_det(const void* x, int is_bf16, long long n, float* ou
   if (n == 0) return 0;
   if (scratch == nullptr) return -10;
   const int grid = grid_for(n, 512, 148 * 4);
-  if (is_bf16) sumsq_partials_kernel<__nv_bfloat16><<<grid, 512, 0, st>>>((const __nv_bfloat16*)x, n, scratch);
-  else sumsq_partials_kernel<float><<<grid, 512, 0, st>>>((const float*)x, n, scratch);
-  sumsq_finish_kernel<<<1, 256, 0, st>>>(scratch, grid, out);
+  if (is_bf16) launch_dep(sumsq_partials_kernel<__nv_bfloat16>, grid, 512, 0, st, (const __nv_bfloat16*)x, n, scratch);
+  else launch_dep(sumsq_partials_kernel<float>, grid, 512, 0, st, (const float*)x, n, scratch);
+  launch_dep(sumsq_finish_kernel, 1, 256, 0, st, scratch, grid, out);
   CHECK_LAUNCH();
 }
 
@@ -1136,15 +1150,15 @@ extern "C" int b200_sumsq(const void* x, int is_bf16, long long n, float* out, c
 }
 
 extern "C" int b200_clip_coef(const float* sumsq, float max_norm, float* coef, float* norm_out, cudaStream_t st) {
-  clip_coef_kernel<<<1, 1, 0, st>>>(sumsq, max_norm, coef, norm_out);
+  launch_dep(clip_coef_kernel, 1, 1, 0, st, sumsq, max_norm, coef, norm_out);
   CHECK_LAUNCH();
 }
 
 extern "C" int b200_scale(void* x, int is_bf16, long long n, const float* coef, cudaStream_t st) {
   if (n == 0) return 0;
   const int grid = grid_for(n, 256, 148 * 8);
-  if (is_bf16) scale_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((__nv_bfloat16*)x, n, coef);
-  else scale_kernel<float><<<grid, 256, 0, st>>>((float*)x, n, coef);
+  if (is_bf16) launch_dep(scale_kernel<__nv_bfloat16>, grid, 256, 0, st, (__nv_bfloat16*)x, n, coef);
+  else launch_dep(scale_kernel<float>, grid, 256, 0, st, (float*)x, n, coef);
   CHECK_LAUNCH();
 }
 
@@ -1201,15 +1215,15 @@ extern "C" int b200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   if (scratch == nullptr) return B200_ERR_NOALLOC_SETUP;
   if (rows == 0) {
     // no rows: the weight gradient of this call is zero (dw is cleared, or left as it is when accumulating)
-    rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st>>>(scratch, dw, 0, d, accumulate_dw);
+    launch_dep(rmsnorm_dw_reduce_kernel, (d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st, scratch, dw, 0, d, accumulate_dw);
     CHECK_LAUNCH();
   }
   const int parts = rows < B200_NOALLOC_MAX_PARTS ? rows : B200_NOALLOC_MAX_PARTS;
   // Every partial row [0, parts) x [0, d) is written by the first kernel before the second reads it,
   // so nothing in the shared array has to be cleared between calls.
-  rmsnorm_bwd_kernel<RMS_BWD_MAXC_LIMIT><<<parts, RMS_BWD_THREADS, 0, st>>>(
+  launch_dep(rmsnorm_bwd_kernel<RMS_BWD_MAXC_LIMIT>, parts, RMS_BWD_THREADS, 0, st, 
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
       (__nv_bfloat16*)dx, scratch, rows, d);
-  rmsnorm_dw_reduce_kernel<<<(d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st>>>(scratch, dw, parts, d, accumulate_dw);
+  launch_dep(rmsnorm_dw_reduce_kernel, (d + 31) / 32, 32 * RMS_DW_GROUPS, 0, st, scratch, dw, parts, d, accumulate_dw);
   CHECK_LAUNCH();
 }

@@ -86,6 +86,7 @@ __device__ __forceinline__ void unrotate32(const FlashBwdParams& p, int pos, int
 template <int DH>
 __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                    float* __restrict__ delta, long long items, int seq, int heads) {
+  pdl_sync();
   constexpr int LPI = DH / 8;                       // lanes per item
   const int lane = threadIdx.x & 31;
   const int li = lane % LPI;
@@ -227,6 +228,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
   const uint32_t tm_st = tmem_base;         // S^T: 2 x 64 columns
   const uint32_t tm_dpt = tmem_base + 128;  // dP^T: 2 x 64 columns
@@ -542,6 +544,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
   const uint32_t tm_s = tmem_base;           // 128 columns
   const uint32_t tm_dp = tmem_base + 128;    // 128 columns
@@ -769,8 +772,8 @@ static int launch_flash_bwd(const void* qkv, const void* dout, const FlashBwdPar
   if (p.trace_cta == BWD_CTA_LOG) { }
   else if (p.trace_cta >= 0) p1.trace = nullptr;
   else { p2.trace = nullptr; p1.trace_cta = -p.trace_cta - 1; }
-  k1<<<p.batch * p.heads * n_kblk, BWD_THREADS, DkDvSmem<DH>::TOTAL, stream>>>(tm_qkv128, tm_qkv64, tm_do64, p1);
-  k2<<<p.batch * p.heads * n_kblk, BWD_THREADS, DqSmem<DH>::TOTAL, stream>>>(tm_qkv128, tm_do128, p2);
+  launch_dep(k1, p.batch * p.heads * n_kblk, BWD_THREADS, DkDvSmem<DH>::TOTAL, stream, tm_qkv128, tm_qkv64, tm_do64, p1);
+  launch_dep(k2, p.batch * p.heads * n_kblk, BWD_THREADS, DqSmem<DH>::TOTAL, stream, tm_qkv128, tm_do128, p2);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -805,13 +808,13 @@ static int flash_bwd_impl(const void* qkv, const void* o, const void* dout, cons
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < 1) blocks = 1;
     if (dh == 128)
-      flash_delta_kernel<128><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+      launch_dep(flash_delta_kernel<128>, (unsigned)blocks, 256, 0, stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                     delta, items, seq, heads);
     else if (dh == 32)
-      flash_delta_kernel<32><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+      launch_dep(flash_delta_kernel<32>, (unsigned)blocks, 256, 0, stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                    delta, items, seq, heads);
     else
-      flash_delta_kernel<64><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+      launch_dep(flash_delta_kernel<64>, (unsigned)blocks, 256, 0, stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                                                    delta, items, seq, heads);
   }
   FlashBwdParams p;

@@ -163,6 +163,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   const int bh = blockIdx.x % (p.batch * p.heads);
   const int pair = n_pair - 1 - blockIdx.x / (p.batch * p.heads);
   const int b = bh / p.heads, h = bh % p.heads;
+  if (p.cu_seqlens != nullptr || WINDOW) pdl_wait();
   int row_base, seq_len;
   if (p.cu_seqlens != nullptr) {
     row_base = p.cu_seqlens[b];
@@ -214,6 +215,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
   // columns: S_A [0,128)  S_B [128,256)  O_A [256,256+DH)  O_B [384,384+DH); P_X overlays the first 64 columns of S_X
 
@@ -558,7 +560,7 @@ static int launch_flash_fwd(const CUtensorMap& tm, const CUtensorMap& tm_kv, con
     configured = true;
   }
   const int grid = p.batch * p.heads * ((p.n_qblk + 1) / 2);   // one CTA per pair of query tiles
-  kern<<<grid, FA_THREADS, L::TOTAL, stream>>>(tm, tm_kv, tm_kr != nullptr ? *tm_kr : tm_kv, p);
+  launch_dep(kern, grid, FA_THREADS, L::TOTAL, stream, tm, tm_kv, tm_kr != nullptr ? *tm_kr : tm_kv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -92,10 +92,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
   // Everything above touches only shared and tensor memory, so as a programmatic dependent it overlaps the tail of
   // the kernel before this one; from here on global memory is read and written.
-  pdl_sync();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
 
   const int tiles_one = p.num_m_tiles * p.num_n_tiles;

@@ -153,6 +153,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   __syncthreads();
   cluster_sync_all();      // the peer's barriers are initialised before anything can arrive on them
   tc_fence_after();
+  // From here on global memory is read and written.  The next kernel is not let in early: its CTAs beside the tiles cost more than its
+  // launch (a training step of 180 launches 3971 us with, 3836 without; a prompt of 8192 tokens through grouped products 24336, 23857).
+  pdl_wait();
   const uint32_t tmem_base = *tmem_holder;
 
   const int num_tiles = p.num_m_tiles * p.num_n_tiles;   // tiles of 256 x 256
@@ -609,6 +612,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 template <typename OUT>
 __global__ void __launch_bounds__(256)
 pair_tail_sum_kernel(const float4* __restrict__ ws, OUT* __restrict__ C, const GemmParams p) {
+  pdl_sync();
   const int t = blockIdx.x >> 5, r0 = (blockIdx.x & 31) * 8 + (threadIdx.x >> 6), c = (threadIdx.x & 63) * 4;
   int m_blk, n_blk;
   tile_coords(p.full_tiles + t, p, m_blk, n_blk);
@@ -666,11 +670,11 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   int pairs = sms / 2;
   const int units = p.splits > 1 ? p.full_tiles + (tiles - p.full_tiles) * p.splits : tiles;
   if (units < pairs) pairs = units;
-  kern<<<pairs * 2, P_THREADS, P_SMEM, stream>>>(tmA, tmB, tmC, tmH, p);
+  launch_dep(kern, pairs * 2, P_THREADS, P_SMEM, stream, tmA, tmB, tmC, tmH, p);
   if (p.splits > 1) {
     const unsigned grid = (unsigned)(tiles - p.full_tiles) * 32;
-    if (p.epi == EPI_BF16) pair_tail_sum_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((const float4*)p.ws, (__nv_bfloat16*)p.C, p);
-    else pair_tail_sum_kernel<float><<<grid, 256, 0, stream>>>((const float4*)p.ws, (float*)p.C, p);
+    if (p.epi == EPI_BF16) launch_dep(pair_tail_sum_kernel<__nv_bfloat16>, grid, 256, 0, stream, (const float4*)p.ws, (__nv_bfloat16*)p.C, p);
+    else launch_dep(pair_tail_sum_kernel<float>, grid, 256, 0, stream, (const float4*)p.ws, (float*)p.C, p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

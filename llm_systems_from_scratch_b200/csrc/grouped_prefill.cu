@@ -183,6 +183,7 @@ grouped_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     tmem_alloc(tmem_holder, 512);
     tmem_relinquish();
   }
+  __syncthreads();          // the CTA holds its tensor memory
   pdl_sync();
   // Latest query tiles first (they may have more keys); the (portion, head) index varies fastest.
   const int bh = blockIdx.x % (p.portions * s.heads);

@@ -140,6 +140,7 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const Late
     tmem_alloc(tmem_holder, L::TMEM_COLS);
     tmem_relinquish();
   }
+  __syncthreads();          // the CTA holds its tensor memory
   pdl_sync();
   const int row = blockIdx.x, split = blockIdx.y;
   const int pos = p.positions[row];

@@ -345,6 +345,7 @@ __global__ void __launch_bounds__(ML_THREADS, 1) mlstm_chunk_kernel(const __grid
     tmem_relinquish();
   }
   for (int i = tid; i < (L::OFF_F >> 4); i += ML_THREADS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();          // the CTA holds its tensor memory
   pdl_sync();
   const int seq = blockIdx.x / p.heads, h = blockIdx.x - seq * p.heads;
   const int D = p.dim, E = p.vdim;

@@ -311,9 +311,11 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
 // then block in pdl_sync() until that kernel has completed and its writes are visible.  pdl_sync() must come before
 // the first access to global memory of any kind (a write may alias something the previous kernel still reads).  It
 // then lets the kernel after this one start the same way.  In a kernel launched the ordinary way both instructions
-// do nothing.
+// do nothing.  A kernel that allocates tensor memory calls it behind a barrier that follows the allocation: what the next
+// kernel's CTAs take while they wait is then never missing to this one.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 

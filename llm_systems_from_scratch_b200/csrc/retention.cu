@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(RC_THREADS, 1) retention_chunk_kernel(const __
     tmem_relinquish();
   }
   for (int i = tid; i < (L::OFF_RMS >> 4); i += RC_THREADS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();          // the CTA holds its tensor memory
   pdl_sync();
   const int seq = blockIdx.x / p.heads, h = blockIdx.x - seq * p.heads;
   const int D = p.dim, E = p.vdim;

@@ -615,7 +615,7 @@ embedding_bwd_join_kernel(const long long* __restrict__ sorted_tokens, const flo
 // One block per row of logits (rows, ld) bf16 with `vocab` valid columns.  Pass 1: online max / sum.
 // Pass 2: overwrite the row with (softmax - onehot) * grad_scale / n_valid.  Row losses go to
 // `row_loss` (fp32); `n_valid` is a device float computed by count_valid_kernel (no host sync).
-constexpr int XENT_THREADS = 512;
+constexpr int XENT_THREADS = 256;
 
 __global__ void count_valid_kernel(const long long* __restrict__ targets, long long rows, int ignore_index,
                                    float* __restrict__ n_valid) {
@@ -627,6 +627,28 @@ __global__ void count_valid_kernel(const long long* __restrict__ targets, long l
   if (threadIdx.x == 0) *n_valid = fmaxf(c, 1.f);
 }
 
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// exp(x - m) of two values.  The difference comes first: a product with m overflows where m is the type's lowest value.
+__device__ __forceinline__ float2 exp_below2(float2 x, float minus_m) {
+  constexpr float L2E = 1.4426950408889634f;
+  const float2 t = __fmul2_rn(__fadd2_rn(x, make_float2(minus_m, minus_m)), make_float2(L2E, L2E));
+  return make_float2(ex2(t.x), ex2(t.y));
+}
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 m = __hmax2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&m);
+}
+
+// Two exponentials per logit are the most of it (16 a clock and SM), and then what a thread has in flight: XENT_DEPTH 16-byte loads,
+// whose maximum is taken on pairs of bf16 before their 32 terms are added; blocks of 256 threads, so that the rows of an SM are in
+// different passes.  4096 rows, us, with one load in flight and 512 threads -> now: 10000 columns 54.6 -> 44.4, 32000 127 -> 97.7,
+// 50257 188 -> 166 (5.0 TB/s; 128 us at the rate of a copy).
+constexpr int XENT_DEPTH = 4;
+
 __global__ void __launch_bounds__(XENT_THREADS)
 xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ row_loss,
             const float* __restrict__ n_valid, long long ld, int vocab, int ignore_index, float grad_scale,
@@ -635,26 +657,37 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
   __shared__ float red[32];
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * ld;
+  uint4* lv = reinterpret_cast<uint4*>(lr);
   const long long tgt = targets[row];
   const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= vocab;
   const int nvec = vocab / 8;
+  const uint4 lowest = make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);      // -inf
   float m = -INFINITY, s = 0.f;
-  for (int g = threadIdx.x; g < nvec; g += XENT_THREADS) {
-    float f[8];
-    load8(lr + g * 8, f);
-    float lm = f[0];
+  for (int g = threadIdx.x; g < nvec; g += XENT_DEPTH * XENT_THREADS) {
+    uint4 v[XENT_DEPTH];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) lm = fmaxf(lm, f[i]);
-    const float nm = fmaxf(m, lm);
-    float add = 0.f;
+    for (int u = 0; u < XENT_DEPTH; ++u) v[u] = g + u * XENT_THREADS < nvec ? lv[g + u * XENT_THREADS] : lowest;
+    uint32_t top = 0xff80ff80u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) add += __expf(f[i] - nm);
-    s = s * __expf(m - nm) + add;
+    for (int u = 0; u < XENT_DEPTH; ++u)
+      top = max_bf16x2(top, max_bf16x2(max_bf16x2(v[u].x, v[u].y), max_bf16x2(v[u].z, v[u].w)));
+    const float2 t2 = unpack_bf16x2(top);
+    const float nm = fmaxf(m, fmaxf(t2.x, t2.y));
+    if (nm == -INFINITY) continue;
+    float2 add[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+    for (int u = 0; u < XENT_DEPTH; ++u) {
+      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add[i & 1] = __fadd2_rn(add[i & 1], exp_below2(unpack_bf16x2(w[i]), -nm));
+    }
+    s = s * __expf(m - nm) + ((add[0].x + add[0].y) + (add[1].x + add[1].y));
     m = nm;
   }
   for (int c = nvec * 8 + threadIdx.x; c < vocab; c += XENT_THREADS) {
     const float f = __bfloat162float(lr[c]);
     const float nm = fmaxf(m, f);
+    if (nm == -INFINITY) continue;
     s = s * __expf(m - nm) + __expf(f - nm);
     m = nm;
   }
@@ -667,15 +700,31 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
   if (!write_grad) return;
   __syncthreads();  // the target logit has been read before anyone overwrites it
   const float k = ignored ? 0.f : grad_scale / nv;
-  for (int g = threadIdx.x; g < nvec; g += XENT_THREADS) {
-    float f[8];
-    load8(lr + g * 8, f);
+  const int tgt_vec = ignored ? -1 : (int)(tgt / 8);
+  for (int g = threadIdx.x; g < nvec; g += XENT_DEPTH * XENT_THREADS) {
+    uint4 v[XENT_DEPTH];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int c = g * 8 + i;
-      f[i] = (__expf(f[i] - lse) - ((c == tgt) ? 1.f : 0.f)) * k;
+    for (int u = 0; u < XENT_DEPTH; ++u)
+      if (g + u * XENT_THREADS < nvec) v[u] = lv[g + u * XENT_THREADS];
+#pragma unroll
+    for (int u = 0; u < XENT_DEPTH; ++u) {
+      const int at = g + u * XENT_THREADS;
+      if (at >= nvec) break;
+      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+      float e[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = exp_below2(unpack_bf16x2(w[i]), -lse);
+        e[2 * i] = f.x * k;
+        e[2 * i + 1] = f.y * k;
+      }
+      if (at == tgt_vec) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (at * 8 + i == tgt) e[i] -= k;
+      }
+      store8(lr + at * 8, e);
     }
-    store8(lr + g * 8, f);
   }
   for (int c = nvec * 8 + threadIdx.x; c < vocab; c += XENT_THREADS)   // columns past `vocab` are never touched
     lr[c] = __float2bfloat16((__expf(__bfloat162float(lr[c]) - lse) - ((c == tgt) ? 1.f : 0.f)) * k);

@@ -117,6 +117,32 @@ def test_xent(rows, v, ld):
     assert buf[3].abs().max().item() == 0
 
 
+@pytest.mark.parametrize("rows,v", [(5, 1), (5, 7), (5, 8), (9, 4095), (9, 16384), (3, 16392), (3, 50257)])
+def test_xent_of_rows_of_any_length(rows, v):
+    """Ends of the passes of 16384 columns and of 8; logits of the lowest value, of minus infinity, and one that leads by far."""
+    from llm_systems_from_scratch_b200.ops import native
+    ld = -(-v // 8) * 8 + 8
+    buf = (4 * torch.randn(rows, ld, generator=torch.Generator().manual_seed(v))).bfloat16().cuda()
+    keep = buf[:, v:].clone()
+    buf[0, :v] = torch.finfo(torch.bfloat16).min
+    if v > 8:
+        buf[1, :v - 3] = -torch.inf
+        buf[2, v // 2] = 3e4
+    tgt = torch.arange(rows, device="cuda") % v
+    tgt[1] = v - 1
+    tgt[0] = -100               # beside 3e38 the logarithm of a sum is lost in 32 bits: the row has to stay finite
+    logits = buf[:, :v].double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(logits, tgt)
+    want.backward()
+    assert abs(native.xent_fwd(buf, tgt, valid_cols=v).item() - want.item()) <= 1e-5 * max(1.0, abs(want.item()))
+    got = native.xent_fwd_bwd(buf, tgt, 1.0, valid_cols=v)
+    assert abs(got.item() - want.item()) <= 1e-5 * max(1.0, abs(want.item()))
+    # one rounding to bf16 is at most 2^-9 of a value; the argument of the exponential carries fp32 rounding of |logit| <= 30
+    diff = (buf[:, :v].double() - logits.grad).norm(dim=1)
+    assert bool((diff <= 2.0 ** -8 * logits.grad.norm(dim=1) + 1e-7).all()), diff
+    assert torch.equal(buf[:, v:], keep)
+
+
 def test_argmax():
     from llm_systems_from_scratch_b200.ops import native
     x = torch.randn(37, 50264, device="cuda").bfloat16()

@@ -383,11 +383,34 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
         continue;
       }
-      if (p.swiglu_f > 0 && p.tma_store) {
+      if (p.swiglu_f > 0 && p.C == nullptr) {
+        // the product alone: nothing is rounded before it
+        const int col = n_blk * P_HALF;
+#pragma unroll 1
+        for (int c = 0; c < P_HALF / 64; ++c) {
+          if (col + c * 64 >= p.swiglu_f) break;
+          uint32_t o[32];
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t g[32], u[32];
+            tmem_ld_32x32(taddr + c * 64 + half * 32, g);
+            tmem_ld_32x32(taddr + P_HALF + c * 64 + half * 32, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float g0 = __uint_as_float(g[2 * j]), g1 = __uint_as_float(g[2 * j + 1]);
+              o[half * 16 + j] = pack_bf16x2(__fdividef(g0, 1.f + __expf(-g0)) * __uint_as_float(u[2 * j]),
+                                             __fdividef(g1, 1.f + __expf(-g1)) * __uint_as_float(u[2 * j + 1]));
+            }
+          }
+          emit(&tmH, col + c * 64, o, false);
+        }
+      } else if (p.swiglu_f > 0 && p.tma_store) {
         // accumulator columns [0,128) are gate_j, [128,256) the matching up_j; three outputs per 64 columns
         const int col = n_blk * P_HALF;
 #pragma unroll 1
         for (int c = 0; c < P_HALF / 64; ++c) {
+          if (col + c * 64 >= p.swiglu_f) break;       // gate columns past F are up rows
           uint32_t og[32], ou[32];
           {
             uint32_t r0[32], r1[32];
@@ -426,6 +449,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const int col = n_blk * P_HALF;
 #pragma unroll 1
         for (int c = 0; c < P_HALF / 32; ++c) {
+          if (col + c * 32 >= p.swiglu_f) break;
           uint32_t g[32], u[32];
           tmem_ld_32x32(taddr + c * 32, g);
           tmem_ld_32x32(taddr + P_HALF + c * 32, u);
@@ -664,7 +688,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
     configured = true;
   }
   p.num_m_tiles = (p.M + 255) / 256;
-  p.num_n_tiles = p.swiglu_f > 0 ? p.swiglu_f / P_HALF : (p.N + P_BN - 1) / P_BN;
+  p.num_n_tiles = p.swiglu_f > 0 ? (p.swiglu_f + P_HALF - 1) / P_HALF : (p.N + P_BN - 1) / P_BN;
   p.group_m = 8;
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   int pairs = sms / 2;
@@ -757,9 +781,9 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   const long long per16 = 16 / esz;
   const bool row_end_ok = (N % per16 == 0) || (pad_writable && (N + per16 - 1) / per16 * per16 <= ldc);
   if (g_pair_tma_store && swiglu_f > 0) {
-    // gate | up (M x 2F) and h (M x F): F is a multiple of 128, so no 64-column box straddles the gate / up border
-    if ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0 && (ldc & 7) == 0 &&
-        (ldh & 7) == 0 && make_tmap_out_2d(&tmC, false, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 64, 32) == 0 &&
+    // gate | up (M x 2F) and h (M x F): F is a multiple of 64, so no 64-column box straddles the gate / up border
+    if ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0 && (ldc & 7) == 0 && (ldh & 7) == 0 &&
+        (C == nullptr || make_tmap_out_2d(&tmC, false, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 64, 32) == 0) &&
         make_tmap_out_2d(&tmH, false, H, (uint64_t)M, (uint64_t)swiglu_f, (uint64_t)ldh, 64, 32) == 0)
       p.tma_store = 1;
   } else if (g_pair_tma_store && epi == EPI_SWIGLU_BWD) {
@@ -774,6 +798,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
     if (make_tmap_out_2d(&tmC, out_f32, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, out_f32 ? 32 : 64, 32) == 0)
       p.tma_store = 1;
   }
+  if (C == nullptr && !p.tma_store) return -13;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -890,7 +915,7 @@ extern "C" int b200_gemm_bf16_pair_swiglu(const void* A, const void* B, void* C,
                                           const unsigned long long* src_ptrs, void* gather_dst,
                                           unsigned long long shard_bytes, int world, int rank, uint32_t* status,
                                           cudaStream_t stream) {
-  if (F <= 0 || F % P_HALF || (ldc & 7) || (ldh & 7) || H == nullptr) return -12;
+  if (F <= 0 || F % 64 || (ldc & 7) || (ldh & 7) || H == nullptr) return -12;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(H) & 15)) return -10;
   GatherTask g;
   const bool carry = world > 0 && gather_dst != nullptr;

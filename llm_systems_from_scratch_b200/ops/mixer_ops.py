@@ -165,6 +165,8 @@ def glu(a, w, n: int, act: str):
                                       native.EPI_B_STABLE, 2 if act == "relu" else 1, None, _ptr(native.status_word(a.device)),
                                       _stream()), "gemm_few_rows")
         return out
+    if a.dtype == torch.bfloat16 and act == "silu" and native.gemm_glu(a, w, out):
+        return out
     if a.dtype == torch.bfloat16:
         _check(lib.b200_gemm_bf16_grouped(_ptr(a), _ptr(w), _ptr(out), None, m, n, k, a.stride(0), w.stride(0), out.stride(0), 0, None,
                                           0, 2 * n, 1, 0, 0, 2 if act == "relu" else 1, native.EPI_B_STABLE, 0, None,

@@ -502,7 +502,7 @@ def gemm_swiglu(x, wgu, gather=None):
     m, k = x.shape
     two_f = wgu.shape[0]
     f = two_f // 2
-    ok = (USE_PAIR and FUSE_SWIGLU_FWD and (m >= PAIR_MIN_M or FORCE_PAIR) and f % 128 == 0 and x.dtype == torch.bfloat16 and wgu.dtype == torch.bfloat16
+    ok = (USE_PAIR and FUSE_SWIGLU_FWD and (m >= PAIR_MIN_M or FORCE_PAIR) and f % 64 == 0 and x.dtype == torch.bfloat16 and wgu.dtype == torch.bfloat16
           and x.stride(1) == 1 and wgu.stride(1) == 1 and x.stride(0) % 8 == 0 and wgu.stride(0) % 8 == 0)
     if not ok:
         return None
@@ -519,6 +519,21 @@ def gemm_swiglu(x, wgu, gather=None):
     if gargs is not None:
         gather.mark_done(carried=True)
     return gu, h
+
+
+def gemm_glu(x, wgu, out) -> bool:
+    """out (M, F) = silu(gate) * up alone on CTA pairs, F a multiple of 64; False where the kernel for it does not apply."""
+    m, k = x.shape
+    f = wgu.shape[0] // 2
+    if not (USE_PAIR and m >= PAIR_MIN_M and f % 64 == 0 and x.stride(0) % 8 == 0 and wgu.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
+            and (x.data_ptr() | wgu.data_ptr() | out.data_ptr()) % 16 == 0):
+        return False
+    rc = load().b200_gemm_bf16_pair_swiglu(_ptr(x), _ptr(wgu), None, _ptr(out), m, f, k, x.stride(0), wgu.stride(0), 0, out.stride(0),
+                                           None, None, 0, 0, 0, _ptr(status_word(x.device)), _stream())
+    if rc == -13:                      # the TMA-store epilogue is switched off
+        return False
+    _check(rc, "b200_gemm_bf16_pair_swiglu")
+    return True
 
 
 def gemm_swiglu_bwd(dy, wdown, gu, gather=None):

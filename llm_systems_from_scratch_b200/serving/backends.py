@@ -11,7 +11,6 @@ import torch
 
 from .. import ops
 from ..ops import mixer_ops as mo
-from ..ops import native
 from ..ops import serving_ops
 from .kv_cache import LayerCache, PagedKVCache, StateSpec
 
@@ -60,10 +59,7 @@ class TransformerBackend:
         o = attend(qkv, li)
         x = ops.gemm(o, w.wo, "nt", residual=x, b_stable=True)
         h, _ = ops.rmsnorm_fwd(x, w.n2, cfg.eps)
-        if x.is_cuda and native.few_rows(x.shape[0], cfg.d_ff):
-            h = mo.glu(h, w.wgu, cfg.d_ff, "silu")
-        else:
-            h = ops.silu_mul_fwd(ops.gemm(h, w.wgu, "nt", b_stable=True))
+        h = mo.glu(h, w.wgu, cfg.d_ff, "silu") if x.is_cuda else ops.silu_mul_fwd(ops.gemm(h, w.wgu, "nt", b_stable=True))
         return ops.gemm(h, w.wdown, "nt", residual=x, b_stable=True)
 
     def forward(self, batch):

@@ -409,3 +409,31 @@ def test_few_rows(m, n, k):
     for act, f in (("silu", torch.nn.functional.silu), ("relu", torch.relu)):
         assert off(mo.glu(a, b[:2 * half], half, act), f(gu[:, :half]) * gu[:, half:2 * half]) < 2.0 ** -8
     native.check_status()
+
+
+@pytest.mark.parametrize("m,f,k", [(1024, 64, 64), (1030, 192, 136), (1500, 1344, 512), (2048, 5504, 2048)])
+def test_gated_product_on_cta_pairs_with_half_a_tile_left(m, f, k):
+    """F a multiple of 64 but not of the tile's 128: the last tile's gate columns run into the up rows and are not stored.  With and without
+    gate and up as outputs of their own."""
+    from llm_systems_from_scratch_b200.ops import mixer_ops as mo, native
+    g = torch.Generator("cuda").manual_seed(f)
+    x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(2 * f, k, generator=g, device="cuda") / k ** 0.5).bfloat16()
+    want_gu = x.double() @ w.double().T
+    want = torch.nn.functional.silu(want_gu[:, :f]) * want_gu[:, f:]
+    off = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    out = torch.full((m, f + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    assert native.gemm_glu(x, w, out[:, :f])
+    assert off(out[:, :f], want) < 2.0 ** -8 and bool((out[:, f:] == 7.0).all())      # one rounding to bf16 is at most 2^-9
+    assert torch.equal(mo.glu(x, w, f, "silu"), out[:, :f])
+    for on in (True, False):                                                          # both epilogues
+        old = native.set_gemm_tma_store(on)
+        try:
+            gu, h = native.gemm_swiglu(x, w)
+            assert native.gemm_glu(x, w, out[:, :f]) == on
+            assert off(mo.glu(x, w, f, "silu"), want) < 2.0 ** -8
+        finally:
+            native.set_gemm_tma_store(old)
+        # h is made of gate and up rounded to bf16: three roundings
+        assert off(gu, want_gu) < 2.0 ** -8 and off(h, want) < 3 * 2.0 ** -8
+    native.check_status()

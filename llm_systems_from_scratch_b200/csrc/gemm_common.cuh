@@ -55,7 +55,32 @@ struct GatherTask {
   uint32_t* done;
 };
 
+// The QKV projection of a serving step, finished in its epilogue: the Q and K thirds are rotated pair-wise by the angle of the row's
+// position, and the K and V rows go to their slot of the paged cache as well (slot < 0: to none).  cs: (2, ctx, dh / 2) fp32, cos then sin.
+struct QkvAppend {
+  const float* cs;             // null = off
+  const int* positions;
+  const long long* slots;
+  __nv_bfloat16 *k_cache, *v_cache;
+  long long num_slots;
+  int d, dh, ctx;
+};
+
+inline bool qkv_append_ok(const QkvAppend& a) {
+  return a.cs != nullptr && a.positions != nullptr && a.slots != nullptr && a.k_cache != nullptr && a.v_cache != nullptr && a.d > 0 && a.dh > 0 &&
+         a.d % a.dh == 0 && a.dh % 8 == 0 && a.ctx > 0 &&
+         ((reinterpret_cast<uintptr_t>(a.cs) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) & 15) == 0;
+}
+
+__device__ __forceinline__ long long append_slot(const QkvAppend& a, int row, uint32_t* status) {
+  const long long slot = a.slots[row];
+  if (slot < a.num_slots) return slot;
+  if (status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (3u << 8));      // beyond the cache: report, do not write
+  return -1;
+}
+
 struct GemmParams {
+  QkvAppend append;
   GatherTask gather;
   // Optional reduce-scatter (+ scale + sum of squares, or + AdamW) of an earlier FSDP unit's gradient staging, run
   // by the same copy warps after the gather (CTA-pair kernel only); reduce.n == 0 = none.
@@ -124,11 +149,10 @@ __device__ __forceinline__ void report(const GemmParams& p, volatile uint32_t* a
 }
 
 // Interleaved-pair rotation of a 32-column accumulator chunk (16 pairs, all inside one head).
-__device__ __forceinline__ void epilogue_rope(const GemmParams& p, int row, int col0, uint32_t (&acc)[32]) {
-  const int pos = row % p.rope_seq;
-  const int e = col0 % p.rope_dh;                       // multiple of 32
-  const float* cs = p.rope_cs + (size_t)pos * (p.rope_dh / 2) + e / 2;
-  const float* sn = cs + (size_t)p.rope_ctx * (p.rope_dh / 2);
+__device__ __forceinline__ void epilogue_rope(const float* table, int ctx, int dh, int pos, int col0, uint32_t (&acc)[32]) {
+  const int e = col0 % dh;                              // multiple of 32
+  const float* cs = table + (size_t)pos * (dh / 2) + e / 2;
+  const float* sn = cs + (size_t)ctx * (dh / 2);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const float4 c4 = *reinterpret_cast<const float4*>(cs + q * 4);
@@ -206,6 +230,10 @@ __device__ __forceinline__ void epilogue_finish(const GemmParams& p, int col0, i
   }
 }
 
+__device__ __forceinline__ void epilogue_rope(const GemmParams& p, int row, int col0, uint32_t (&acc)[32]) {
+  epilogue_rope(p.rope_cs, p.rope_ctx, p.rope_dh, row % p.rope_seq, col0, acc);
+}
+
 __device__ __forceinline__ float gate_of(float g) { return __fdividef(1.f, 1.f + __expf(-g)); }
 
 // One 32-column chunk of one output row.  `coff` shifts the columns of C and R (one of several problems side by side).
@@ -216,6 +244,8 @@ __device__ __forceinline__ void epilogue_store(const GemmParams& p, int row, int
   if (ncols <= 0) return;
   if (p.finished) epilogue_finish(p, col0, ncols, acc);
   if (p.rope_cs != nullptr && col0 < 2 * p.rope_d && ncols == 32) epilogue_rope(p, row, col0, acc);
+  if (p.append.cs != nullptr && col0 < 2 * p.append.d)        // chunks are whole and inside a head (checked on the host)
+    epilogue_rope(p.append.cs, p.append.ctx, p.append.dh, p.append.positions[row], col0, acc);
   if (p.epi == EPI_SWIGLU_BWD) {
     // as the stand-alone kernel (fast division apart): dh is rounded to bf16 first, gate and up are read as bf16
     const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)row * p.ldr + col0;
@@ -304,6 +334,19 @@ __device__ __forceinline__ void epilogue_store(const GemmParams& p, int row, int
         for (int t = 0; t < 4; ++t)
           o[t] = pack_bf16x2(__uint_as_float(acc[j * 8 + 2 * t]), __uint_as_float(acc[j * 8 + 2 * t + 1]));
         *reinterpret_cast<uint4*>(c + j * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      if (p.append.cs != nullptr && col0 >= p.append.d) {
+        const long long slot = append_slot(p.append, row, p.status);
+        const bool is_k = col0 < 2 * p.append.d;
+        __nv_bfloat16* dst = (is_k ? p.append.k_cache : p.append.v_cache) + slot * p.append.d + (col0 - (is_k ? 1 : 2) * p.append.d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t o[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            o[t] = pack_bf16x2(__uint_as_float(acc[j * 8 + 2 * t]), __uint_as_float(acc[j * 8 + 2 * t + 1]));
+          if (slot >= 0) *reinterpret_cast<uint4*>(dst + j * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
       }
     } else {
 #pragma unroll

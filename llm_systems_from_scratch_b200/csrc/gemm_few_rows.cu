@@ -30,8 +30,55 @@ struct FewRowsParams {
   const void* R;
   long long ldr;
   GemmFinish finish;
+  QkvAppend append;
   uint32_t* status;
 };
+
+// What an output row needs from elsewhere, requested before its sums: four columns of the residual row, or of a row of Q, K or V (see
+// QkvAppend) the angles and the slot.  The four columns lie in one head.
+struct RowNeeds {
+  uint2 res;
+  float2 c, s;
+  long long slot;
+};
+
+__device__ __forceinline__ void fr_need(const FewRowsParams& p, int m, int n, RowNeeds& x) {
+  if (p.epi == EPI_BF16_RES) {
+    const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)m * p.ldr + n;
+    if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(r) & 7) == 0) {
+      x.res = *reinterpret_cast<const uint2*>(r);
+    } else {
+      uint16_t e[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n + j < p.N) e[j] = reinterpret_cast<const uint16_t*>(r)[j];
+      x.res = make_uint2(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16);
+    }
+  }
+  const QkvAppend& a = p.append;
+  if (a.cs == nullptr) return;
+  if (n < 2 * a.d) {
+    const float* cs = a.cs + (size_t)a.positions[m] * (a.dh / 2) + n % a.dh / 2;
+    x.c = *reinterpret_cast<const float2*>(cs);
+    x.s = *reinterpret_cast<const float2*>(cs + (size_t)a.ctx * (a.dh / 2));
+  }
+  x.slot = n >= a.d ? append_slot(a, m, p.status) : -1;
+}
+
+__device__ __forceinline__ void fr_append(const FewRowsParams& p, const RowNeeds& x, int n, float (&v)[4]) {
+  const QkvAppend& a = p.append;
+  if (n < 2 * a.d) {
+    const float x0 = v[0], x1 = v[1], x2 = v[2], x3 = v[3];
+    v[0] = x.c.x * x0 - x.s.x * x1;
+    v[1] = x.s.x * x0 + x.c.x * x1;
+    v[2] = x.c.y * x2 - x.s.y * x3;
+    v[3] = x.s.y * x2 + x.c.y * x3;
+  }
+  if (x.slot < 0) return;
+  const bool is_k = n < 2 * a.d;
+  *reinterpret_cast<uint2*>((is_k ? a.k_cache : a.v_cache) + x.slot * a.d + (n - (is_k ? 1 : 2) * a.d)) =
+      make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+}
 
 __device__ __forceinline__ void fr_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -55,7 +102,7 @@ __device__ __forceinline__ float fr_finish(const FewRowsParams& p, float v, int 
 }
 
 // Four columns of one output row.
-__device__ __forceinline__ void fr_store(const FewRowsParams& p, int m, int n, const float (&v)[4]) {
+__device__ __forceinline__ void fr_store(const FewRowsParams& p, int m, int n, const uint2& res, float (&v)[4]) {
   const long long at = (long long)m * p.ldc + n;
   const bool whole = n + 4 <= p.N;
   if (p.epi == EPI_F32 || p.epi == EPI_F32_ACC) {
@@ -75,20 +122,16 @@ __device__ __forceinline__ void fr_store(const FewRowsParams& p, int m, int n, c
     return;
   }
   __nv_bfloat16* c = reinterpret_cast<__nv_bfloat16*>(p.C) + at;
-  const __nv_bfloat16* r = p.epi == EPI_BF16_RES ? reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)m * p.ldr + n : nullptr;
-  if (whole && ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(r)) & 7) == 0) {
-    float2 a = make_float2(v[0], v[1]), b = make_float2(v[2], v[3]);
-    if (r != nullptr) {
-      const uint2 rv = *reinterpret_cast<const uint2*>(r);
-      const float2 ra = unpack_bf16x2(rv.x), rb = unpack_bf16x2(rv.y);
-      a = make_float2(a.x + ra.x, a.y + ra.y);
-      b = make_float2(b.x + rb.x, b.y + rb.y);
-    }
-    *reinterpret_cast<uint2*>(c) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(b.x, b.y));
+  if (p.epi == EPI_BF16_RES) {
+    const float2 a = unpack_bf16x2(res.x), b = unpack_bf16x2(res.y);
+    v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y;
+  }
+  if (whole && (reinterpret_cast<uintptr_t>(c) & 7) == 0) {
+    *reinterpret_cast<uint2*>(c) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
   } else {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (n + j < p.N) c[j] = __float2bfloat16(r != nullptr ? v[j] + __bfloat162float(r[j]) : v[j]);
+      if (n + j < p.N) c[j] = __float2bfloat16(v[j]);
   }
 }
 
@@ -152,7 +195,8 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   tc_fence_before();
   __syncthreads();          // the CTA holds its tensor memory before the kernel after this one may be placed beside it
   tc_fence_after();
-  pdl_sync();
+  pdl_wait();
+  if (p.append.cs == nullptr) pdl_trigger();      // attention comes next otherwise
   const uint32_t tmem_base = *tmem_holder;
 
   if (warp == 0) {
@@ -234,6 +278,12 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     const int n = n0 + lane * 4, step = p.splits * (FR_THREADS / 32);
     if (n < p.N) {
       for (int m = rank + p.splits * warp; m < p.M; m += ROWS * step) {
+        RowNeeds needs[ROWS];
+        if (HALVES == 1) {
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i)
+            if (m + i * step < p.M) fr_need(p, m + i * step, n, needs[i]);
+        }
         float v[HALVES][ROWS][4] = {};
 #pragma unroll 4
         for (int s = 0; s < p.splits; ++s) {
@@ -263,7 +313,8 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
               v[0][i][j] = fr_finish(p, v[0][i][j], n + j);
             }
           }
-          fr_store(p, m + i * step, n, v[0][i]);
+          if (HALVES == 1 && p.append.cs != nullptr) fr_append(p, needs[i], n, v[0][i]);
+          fr_store(p, m + i * step, n, needs[i].res, v[0][i]);
         }
       }
     }
@@ -347,6 +398,23 @@ static int launch_few_rows(const CUtensorMap& tmX, const CUtensorMap& tmW, FewRo
 }  // namespace b200
 
 using namespace b200;
+
+// QKV projection of a serving step of at most 128 rows (see QkvAppend): C (M x 3 d) bf16.
+extern "C" int b200_gemm_few_rows_append(const void* A, const void* B, void* C, int M, int K, long long lda, long long ldb, long long ldc,
+                                         int epi, const QkvAppend* append, uint32_t* status, cudaStream_t stream) {
+  if (M <= 0 || K <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7)) return -10;
+  if (M > BM || (epi & ~EPI_B_STABLE) != EPI_BF16 || append == nullptr || !qkv_append_ok(*append)) return -11;
+  FewRowsParams p = {};
+  p.M = M; p.N = 3 * append->d; p.K = K; p.xrows = (M + 7) / 8 * 8;
+  p.b_early = (epi & EPI_B_STABLE) ? 1 : 0; p.epi = EPI_BF16; p.C = C; p.ldc = ldc; p.append = *append; p.status = status;
+  CUtensorMap tmX, tmW;
+  int rc = make_tmap_bf16_2d(&tmX, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BK, (uint32_t)p.xrows);
+  if (rc) return -20 + rc;
+  rc = make_tmap_bf16_2d(&tmW, B, (uint64_t)p.N, (uint64_t)K, (uint64_t)ldb, BK, BM);
+  if (rc) return -30 + rc;
+  return launch_few_rows<1>(tmX, tmW, p, stream);
+}
 
 // C (M x N) = act(alpha * (A B^T + bias)) for M <= 128, both operands K-major.  epi: 0, 1, 2 or 3 (see GemmEpilogue), EPI_B_STABLE allowed.
 // gated: 0, or 1 silu, 2 relu: B has 2 N rows, C (bf16) receives act(gate) * up.  finish: as b200_gemm_bf16_finish, without GELU.

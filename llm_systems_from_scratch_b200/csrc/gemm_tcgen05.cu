@@ -17,6 +17,9 @@
 
 namespace b200 {
 
+// Steps of more rows than this are followed by passes over many rows, which are not let in early (see pdl_trigger).
+constexpr int PDL_TRIGGER_M = 2048;
+
 template <int BN, int STAGES>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
@@ -95,7 +98,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_sync();
+  pdl_wait();
+  if (p.append.cs == nullptr && p.M <= PDL_TRIGGER_M) pdl_trigger();
   const uint32_t tmem_base = *tmem_holder;
 
   const int tiles_one = p.num_m_tiles * p.num_n_tiles;
@@ -467,7 +471,7 @@ using namespace b200;
 static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda,
                           long long ldb, long long ldc, long long ldr, int a_mn, int b_mn, int epi, int bn_hint,
                           int max_ctas, int splits, float* ws, uint32_t* tile_counters, uint32_t* status,
-                          cudaStream_t stream, const GemmFinish* finish = nullptr) {
+                          cudaStream_t stream, const GemmFinish* finish = nullptr, const QkvAppend* append = nullptr) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return -10;
@@ -534,6 +538,8 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* R, 
   p.tile_group = nullptr; p.group_rows = 0; p.batch = 1; p.a_step = p.c_step = 0; p.relu = 0; p.head_gate = 0;
   p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;
+  p.append.cs = nullptr;
+  if (append != nullptr) p.append = *append;
 
 #define DISPATCH(BN_)                                                                    \
   if (a_mn && b_mn) return launch_gemm<BN_, true, true>(tmA, tmB, p, max_ctas, stream);   \
@@ -552,6 +558,15 @@ extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, const void*
                               int epi, int bn_hint, int max_ctas, uint32_t* status, cudaStream_t stream) {
   return gemm_bf16_impl(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, bn_hint, max_ctas, 1, nullptr,
                         nullptr, status, stream);
+}
+
+// QKV projection of a serving step (see QkvAppend): C (M x 3 d) bf16, ldc a multiple of 8; d and dh multiples of 32.
+extern "C" int b200_gemm_bf16_append(const void* A, const void* B, void* C, int M, int K, long long lda, long long ldb, long long ldc, int epi,
+                                     const QkvAppend* append, uint32_t* status, cudaStream_t stream) {
+  if (append == nullptr || !qkv_append_ok(*append) || append->d % 32 || append->dh % 32 || (epi & ~EPI_B_STABLE) != EPI_BF16) return -12;
+  if ((reinterpret_cast<uintptr_t>(C) & 15) || (ldc & 7)) return -10;
+  return gemm_bf16_impl(A, B, C, nullptr, M, 3 * append->d, K, lda, ldb, ldc, 0, 0, 0, epi, 0, 0, 1, nullptr, nullptr, status, stream, nullptr,
+                        append);
 }
 
 // K-major operands, epi 0, 1 or 3, accumulators finished first (see GemmFinish).
@@ -697,6 +712,7 @@ extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, con
   p.tile_group = tile_group; p.group_rows = group_rows; p.batch = rows ? 1 : batch; p.a_step = a_step; p.c_step = c_step; p.relu = swiglu == 2;
   p.head_gate = head_gate; p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;
+  p.append.cs = nullptr;
   if (!rows && swiglu) {
     if (bn == 256) return launch_gemm<256, false, false, GROUP_COLS, true>(tmA, tmB, p, 0, stream);
     if (bn == 128) return launch_gemm<128, false, false, GROUP_COLS, true>(tmA, tmB, p, 0, stream);

@@ -25,6 +25,12 @@ def _lib():
         lib.b200_kv_append.restype = I
         lib.b200_rope_kv_append.argtypes = [P, P, P, P, P, P, L, I, I, I, L, P, P]
         lib.b200_rope_kv_append.restype = I
+        lib.b200_gemm_few_rows_append.argtypes = [P, P, P, I, I, L, L, L, I, P, P, P]
+        lib.b200_gemm_few_rows_append.restype = I
+        lib.b200_gemm_bf16_append.argtypes = [P, P, P, I, I, L, L, L, I, P, P, P]
+        lib.b200_gemm_bf16_append.restype = I
+        lib.b200_gemm_bf16_pair_append.argtypes = [P, P, P, I, I, L, L, L, P, P, P]
+        lib.b200_gemm_bf16_pair_append.restype = I
         _declared = True
     return lib
 
@@ -68,6 +74,47 @@ def rope_kv_append(qkv, cos_sin, positions, k_cache, v_cache, slot_mapping, n_he
                                           v_cache.data_ptr(), slot_mapping.data_ptr(), qkv.shape[0], d, dh,
                                           cos_sin.shape[1], num_slots, native.status_word(qkv.device).data_ptr(),
                                           native._stream()), "rope_kv_append")
+
+
+class QkvAppend(ctypes.Structure):
+    """csrc/gemm_common.cuh: QkvAppend."""
+    _fields_ = [("cs", ctypes.c_void_p), ("positions", ctypes.c_void_p), ("slots", ctypes.c_void_p), ("k_cache", ctypes.c_void_p),
+                ("v_cache", ctypes.c_void_p), ("num_slots", ctypes.c_longlong), ("d", ctypes.c_int), ("dh", ctypes.c_int), ("ctx", ctypes.c_int)]
+
+
+def qkv_rope_append(h, wqkv, cos_sin, positions, k_cache, v_cache, slot_mapping, n_heads: int):
+    """qkv = h (R, d) @ wqkv (3 d, d)^T, then what ``rope_kv_append`` does with it, in the product's epilogue where the heads are made of its
+    chunks of columns (Q, K and V are then rounded once, not twice)."""
+    r, k = h.shape
+    d = wqkv.shape[0] // 3
+    dh = d // n_heads
+    few = h.is_cuda and native.few_rows(r, 3 * d)
+    if h.is_cuda and (few or (dh % 32 == 0 and d % 64 == 0)):
+        native._req(h.dtype == torch.bfloat16 and wqkv.dtype == torch.bfloat16 and h.stride(1) == 1 and wqkv.stride(1) == 1
+                    and wqkv.shape[1] == k and dh * n_heads == d, "bad projection")
+        native._req(slot_mapping.dtype == torch.int64 and slot_mapping.numel() == r and slot_mapping.is_contiguous()
+                    and positions.dtype == torch.int32 and positions.numel() == r and positions.is_contiguous(), "bad slot mapping or positions")
+        native._req(k_cache.shape == v_cache.shape and k_cache.shape[-1] == d and k_cache.is_contiguous() and v_cache.is_contiguous()
+                    and k_cache.dtype == v_cache.dtype == torch.bfloat16, "cache shape does not match")
+        native._req(cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.shape[0] == 2 and cos_sin.shape[2] == dh // 2
+                    and dh % 8 == 0, "bad rope cache")
+        out = torch.empty((r, 3 * d), dtype=torch.bfloat16, device=h.device)
+        what = QkvAppend(cos_sin.data_ptr(), positions.data_ptr(), slot_mapping.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                         k_cache.shape[0] * k_cache.shape[1], d, dh, cos_sin.shape[1])
+        args = (h.data_ptr(), wqkv.data_ptr(), out.data_ptr(), r, k, h.stride(0), wqkv.stride(0), 3 * d)
+        tail = (ctypes.byref(what), native.status_word(h.device).data_ptr(), native._stream())
+        if few:
+            native._check(_lib().b200_gemm_few_rows_append(*args, native.EPI_B_STABLE, *tail), "gemm_few_rows_append")
+            return out
+        rc = _lib().b200_gemm_bf16_pair_append(*args, *tail) if native.USE_PAIR and r >= native.PAIR_MIN_M else -13
+        if rc == -13:                      # a small step, or the epilogue that the CTA pairs need is switched off
+            rc = _lib().b200_gemm_bf16_append(*args, native.EPI_B_STABLE, *tail)
+        native._check(rc, "gemm_bf16_append")
+        return out
+    from . import gemm
+    qkv = gemm(h, wqkv, "nt", b_stable=True)
+    rope_kv_append(qkv, cos_sin, positions, k_cache, v_cache, slot_mapping, n_heads)
+    return qkv
 
 
 def choose_splits(rows: int, heads: int, max_context: int, sms: int = 148, head_dim: int = 128) -> int:

@@ -53,9 +53,8 @@ class TransformerBackend:
     def _block(self, x, w, li: int, batch, attend):
         cfg = self.cfg
         h, _ = ops.rmsnorm_fwd(x, w.n1, cfg.eps)
-        qkv = ops.gemm(h, w.wqkv, "nt", b_stable=True)
-        # rotary embedding of Q and K in place and the append of K, V to the paged cache: one kernel on the GPU
-        serving_ops.rope_kv_append(qkv, self.rope, batch.positions, self.cache.k[li], self.cache.v[li], batch.slots, cfg.n_heads)
+        qkv = serving_ops.qkv_rope_append(h, w.wqkv, self.rope, batch.positions, self.cache.k[li], self.cache.v[li], batch.slots,
+                                          cfg.n_heads)
         o = attend(qkv, li)
         x = ops.gemm(o, w.wo, "nt", residual=x, b_stable=True)
         h, _ = ops.rmsnorm_fwd(x, w.n2, cfg.eps)

@@ -187,3 +187,44 @@ def test_cached_tokens_dealt_to_ctas(heads, dh, splits, lens):
     # one rounding of the result to bf16 (2^-9), fp32 sums and exponents otherwise
     assert (got.double().view_as(want) - want).norm() <= 2.0 ** -8 * want.norm()
     assert not got[[i for i, n in enumerate(lens) if n == 0]].any()
+
+
+@pytest.mark.parametrize("rows", [1, 7, 33, 64, 65, 1024, 1030])
+@pytest.mark.parametrize("heads,dh", [(16, 128), (12, 64), (2, 32), (3, 40)])
+def test_qkv_projection_that_rotates_and_appends(rows, heads, dh):
+    """Against the three steps one after the other; rows without a slot, and a slot beyond the cache, which is reported."""
+    from llm_systems_from_scratch_b200.ops import native, serving_ops
+    d, ctx, pages, page = heads * dh, 300, 70, 16
+    g = torch.Generator("cuda").manual_seed(rows)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    h, w = rand(rows, d).bfloat16(), (rand(3 * d, d) / d ** 0.5).bfloat16()
+    angle = torch.arange(ctx)[:, None] * 100.0 ** -(torch.arange(dh // 2) / (dh / 2))
+    table = torch.stack((angle.cos(), angle.sin())).float().cuda()
+    positions = torch.randint(0, ctx, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    slots = torch.randperm(pages * page, generator=g, device="cuda")[:rows]
+    slots[rows // 2] = -1
+    k, v = (rand(pages, page, d).bfloat16() for _ in range(2))
+    k0, v0 = k.clone(), v.clone()
+    native.status_word().zero_()
+    got = serving_ops.qkv_rope_append(h, w, table, positions, k, v, slots, heads)
+    native.check_status()
+    want = h.double() @ w.double().T
+    turn = want[:, :2 * d].reshape(rows, 2 * heads, dh // 2, 2)
+    c, s = (t[positions.long()].double()[:, None] for t in table)
+    want[:, :2 * d] = torch.stack((turn[..., 0] * c - turn[..., 1] * s, turn[..., 0] * s + turn[..., 1] * c), -1).reshape(rows, 2 * d)
+    # one rounding to bf16 is at most 2^-9 (the path in three steps has two)
+    assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+    on = slots >= 0
+    for cache, old, cols in ((k, k0, got[:, d:2 * d]), (v, v0, got[:, 2 * d:])):
+        assert torch.equal(cache.view(-1, d)[slots[on]], cols[on])
+        rest = torch.ones(pages * page, dtype=torch.bool, device="cuda").index_fill_(0, slots[on], False)
+        assert torch.equal(cache.view(-1, d)[rest], old.view(-1, d)[rest])
+    slots[0] = pages * page
+    k.copy_(k0)
+    serving_ops.qkv_rope_append(h, w, table, positions, k, v, slots, heads)
+    torch.cuda.synchronize()
+    with pytest.raises(native.KernelError):
+        native.check_status()
+    on = (slots >= 0) & (slots < pages * page)
+    rest = torch.ones(pages * page, dtype=torch.bool, device="cuda").index_fill_(0, slots[on], False)
+    assert torch.equal(k.view(-1, d)[rest], k0.view(-1, d)[rest])

@@ -19,7 +19,7 @@ def _lib():
     lib = native.load()
     if not _declared:
         P, I, L, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
-        lib.b200_paged_decode.argtypes = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, P, P]
+        lib.b200_paged_decode.argtypes = [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, P, P]
         lib.b200_paged_decode.restype = I
         lib.b200_kv_append.argtypes = [P, P, P, P, L, I, L, P, P]
         lib.b200_kv_append.restype = I
@@ -136,23 +136,12 @@ def choose_splits(rows: int, heads: int, max_context: int, sms: int = 148, head_
     return best
 
 
-LEAST_PIECES = 4       # pieces of eight tokens a CTA takes at least: one request of 2400 tokens 25.5 us with one or two, 17.6 with four
-
-
-def decode_ctas(heads: int, head_dim: int, sms: int = 148) -> int:
-    """CTAs of one wave of the decode kernel: heads * head_dim / 8 threads of 128 registers each."""
-    threads = max(32, -(-heads * head_dim // 8 // 32) * 32)
-    return sms * max(1, min(32, 65536 // (128 * threads)))
-
-
 def paged_decode_attention(qkv, k_cache, v_cache, block_tables, context_lens, n_heads: int, splits: int = 0,
                            scratch=None):
     """One query token per request against its paged KV history.
 
     qkv: (R, 3d) packed (only the query third is read) or (R, d); caches: (num_pages, page_size, d);
     block_tables: (R, max_pages) int32; context_lens: (R,) int32, number of cached tokens to attend to.
-    The cached tokens of all requests are dealt in equal shares to ``splits`` CTAs per request, or (0) to the CTAs that run at
-    once.  ``scratch``: fp32, used where it is large enough.
     Returns (R, d).  The values inside the tables are checked on the device: a length beyond ``max_pages * page`` or
     a page id beyond the cache is skipped and recorded in the status word (``native.check_status`` raises).
     """
@@ -170,18 +159,16 @@ def paged_decode_attention(qkv, k_cache, v_cache, block_tables, context_lens, n_
                 width in (d, 3 * d) and dh * n_heads == d, "cache / query shapes do not match")
     page = k_cache.shape[1]
     max_pages = block_tables.shape[1]
-    ctas = r * splits if splits > 0 else decode_ctas(n_heads, dh)
+    if splits <= 0:
+        splits = choose_splits(r, n_heads, max_pages * page, head_dim=dh)
     out = torch.empty((r, d), dtype=torch.bfloat16, device=qkv.device)
-    parts = ctas + r
-    need = parts * n_heads * (dh + 2) + 2 * r
-    if scratch is None or scratch.numel() < need:
-        scratch = torch.empty(need, dtype=torch.float32, device=qkv.device)
-    part_o = scratch[:parts * n_heads * dh]
-    part_ml = scratch[parts * n_heads * dh:]
-    row_parts = part_ml[parts * n_heads * 2:]
+    if scratch is None:
+        scratch = torch.empty(r * n_heads * splits * (dh + 2), dtype=torch.float32, device=qkv.device)
+    part_o = scratch[:r * n_heads * splits * dh]
+    part_ml = scratch[r * n_heads * splits * dh:]
     native._check(lib.b200_paged_decode(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr(),
                                         context_lens.data_ptr(), out.data_ptr(), part_o.data_ptr(), part_ml.data_ptr(),
-                                        row_parts.data_ptr(), r, qkv.stride(0), n_heads, dh, page, max_pages, ctas, LEAST_PIECES,
-                                        1.0 / math.sqrt(dh), k_cache.shape[0], native.status_word(qkv.device).data_ptr(),
-                                        native._stream()), "paged_decode")
+                                        r, qkv.stride(0), n_heads, dh, page, max_pages, splits, 1.0 / math.sqrt(dh),
+                                        k_cache.shape[0], native.status_word(qkv.device).data_ptr(), native._stream()),
+                  "paged_decode")
     return out

@@ -48,7 +48,7 @@ class TransformerBackend:
         return self.cache
 
     def choose_splits(self, rows: int, max_context: int) -> int:
-        return 0                      # the attention kernel deals the cached tokens to the CTAs that run at once
+        return serving_ops.choose_splits(rows, self.cfg.n_heads, max_context, head_dim=self.cfg.d_model // self.cfg.n_heads)
 
     def _block(self, x, w, li: int, batch, attend):
         cfg = self.cfg

@@ -160,35 +160,6 @@ def test_rope_kv_append_equals_the_two_separate_kernels(heads, dh):
     assert float(kc.view(-1, d)[slots[5]].abs().sum()) == 0.0
 
 
-@pytest.mark.parametrize("heads,dh", [(16, 128), (5, 64), (1, 128)])
-@pytest.mark.parametrize("splits", [0, 1, 3])
-@pytest.mark.parametrize("lens", [[0], [1], [8], [9], [0, 0, 0], [0, 17, 0, 0, 2400, 1, 0], [16] * 70, list(range(0, 400, 3)), [2560, 5, 2560]])
-def test_cached_tokens_dealt_to_ctas(heads, dh, splits, lens):
-    """Shares that end inside a request, at its end and beyond several requests; requests without tokens answer zero."""
-    from llm_systems_from_scratch_b200.ops import native, serving_ops
-    d, page, r = heads * dh, 16, len(lens)
-    g = torch.Generator("cuda").manual_seed(r)
-    n_pages = sum(-(-n // page) for n in lens) + 1
-    kc, vc = (torch.randn(n_pages, page, d, device="cuda", generator=g).bfloat16() for _ in range(2))
-    q = torch.randn(r, d, device="cuda", generator=g).bfloat16()
-    order, at = torch.randperm(n_pages, generator=torch.Generator().manual_seed(r)).int(), 0
-    tables = torch.full((r, 160), 1 << 30, dtype=torch.int32)
-    want = torch.zeros(r, heads, dh, dtype=torch.float64, device="cuda")
-    for i, n in enumerate(lens):
-        pages = order[at:at - (-n // page)]
-        at += len(pages)
-        tables[i, :len(pages)] = pages
-        if n:
-            k, v = (c[pages.long().cuda()].reshape(-1, heads, dh)[:n].double() for c in (kc, vc))
-            p = torch.softmax(torch.einsum("hd,thd->ht", q[i].view(heads, dh).double(), k) * dh ** -0.5, -1)
-            want[i] = torch.einsum("ht,thd->hd", p, v)
-    got = serving_ops.paged_decode_attention(q, kc, vc, tables.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), heads, splits)
-    native.check_status()
-    # one rounding of the result to bf16 (2^-9), fp32 sums and exponents otherwise
-    assert (got.double().view_as(want) - want).norm() <= 2.0 ** -8 * want.norm()
-    assert not got[[i for i, n in enumerate(lens) if n == 0]].any()
-
-
 @pytest.mark.parametrize("rows", [1, 7, 33, 64, 65, 1024, 1030])
 @pytest.mark.parametrize("heads,dh", [(16, 128), (12, 64), (2, 32), (3, 40)])
 def test_qkv_projection_that_rotates_and_appends(rows, heads, dh):

@@ -987,17 +987,23 @@ extern "C" int b200_rmsnorm_set_bwd_rows(int variant) {
 // 0 = always the one-block-per-eight-rows kernel (kept for A/B timing and as the general-width path)
 extern "C" void b200_rmsnorm_set_fwd_rows(int on) { g_rmsnorm_fwd_rows = on; }
 
+// Rows up to which a warp alone in its block, its whole row requested at once, is better than eight warps that read theirs twice (us in a
+// chain of launches, d = 2048: one row 2.4 -> 1.6, 20 2.8 -> 1.7, 592 3.1 -> 2.1, 1184 3.2 -> 3.0, 2331 3.6 -> 4.5).
+constexpr int RMS_FEW_ROWS = 148 * 8;
 extern "C" int b200_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, int d, float eps,
                                 cudaStream_t st) {
   if (d % 8 || !ALIGNED16(x) || !ALIGNED16(w) || !ALIGNED16(y)) return -10;
   if (rows == 0) return 0;
   // widths that are a multiple of 256 up to 2048 with enough rows to fill the GPU: the row-pipelined kernel
   const int nc = d / 256;
-  if (g_rmsnorm_fwd_rows && d % 256 == 0 && nc <= 8 && rows >= 148 * 8 * 2 * 2) {
-    const int grid = 148 * 2;      // two resident blocks per SM at the widest instance (128 registers)
+  // and few rows: a warp alone in its block, which requests its whole row at once (the same sums in the same order)
+  const bool few = rows <= RMS_FEW_ROWS;
+  if (g_rmsnorm_fwd_rows && d % 256 == 0 && nc <= 8 && (few || rows >= 148 * 8 * 2 * 2)) {
+    const int grid = few ? rows : 148 * 2;      // two resident blocks per SM at the widest instance (128 registers)
+    const int threads = few ? 32 : 256;
 #define RMS_FWD_ROWS(NC)                                                                                  \
   case NC:                                                                                                \
-    launch_dep(rmsnorm_fwd_rows_kernel<NC>, grid, 256, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, \
+    launch_dep(rmsnorm_fwd_rows_kernel<NC>, grid, threads, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, \
                (__nv_bfloat16*)y, rstd, rows, eps);                                                       \
     break
     switch (nc) {

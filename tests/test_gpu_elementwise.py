@@ -323,3 +323,17 @@ def test_launches_go_to_the_current_stream():
     with torch.cuda.stream(side):
         assert native._stream() == side.cuda_stream == torch.cuda.current_stream().cuda_stream
     assert native._stream() != side.cuda_stream
+
+
+@pytest.mark.parametrize("rows", [1, 9, 1184, 1185])
+@pytest.mark.parametrize("d", [8, 256, 264, 768, 2048, 2304, 5120])
+def test_rmsnorm_of_few_rows(rows, d):
+    """The borders of a warp alone in its block (1184 rows, multiples of 256 up to 2048 columns)."""
+    from llm_systems_from_scratch_b200.ops import native
+    g = torch.Generator("cuda").manual_seed(d)
+    x, w = torch.randn(rows, d, generator=g, device="cuda").bfloat16(), torch.randn(d, generator=g, device="cuda").bfloat16()
+    y, rstd = native.rmsnorm_fwd(x, w, 1e-5)
+    want = torch.rsqrt(x.double().square().mean(-1) + 1e-5)
+    assert ((rstd.double() - want) / want).abs().max().item() < 1e-5               # fp32 sum of d squares, then rsqrt
+    want = x.double() * want[:, None] * w.double()
+    assert ((y.double() - want).norm() / want.norm()).item() < 2.0 ** -8           # one rounding to bf16 is at most 2^-9

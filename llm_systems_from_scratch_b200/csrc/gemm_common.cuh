@@ -234,6 +234,18 @@ __device__ __forceinline__ void epilogue_rope(const GemmParams& p, int row, int 
   epilogue_rope(p.rope_cs, p.rope_ctx, p.rope_dh, row % p.rope_seq, col0, acc);
 }
 
+// The same for QkvAppend: the sums are rounded to bf16 first and rotated as rope_kv_append_kernel does, so that a step's values do not
+// depend on whether it takes this path.
+__device__ __forceinline__ void epilogue_append_rope(const QkvAppend& a, int row, int col0, uint32_t (&acc)[32]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float2 v = unpack_bf16x2(pack_bf16x2(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1])));
+    acc[2 * j] = __float_as_uint(v.x);
+    acc[2 * j + 1] = __float_as_uint(v.y);
+  }
+  epilogue_rope(a.cs, a.ctx, a.dh, a.positions[row], col0, acc);
+}
+
 __device__ __forceinline__ float gate_of(float g) { return __fdividef(1.f, 1.f + __expf(-g)); }
 
 // One 32-column chunk of one output row.  `coff` shifts the columns of C and R (one of several problems side by side).
@@ -245,7 +257,7 @@ __device__ __forceinline__ void epilogue_store(const GemmParams& p, int row, int
   if (p.finished) epilogue_finish(p, col0, ncols, acc);
   if (p.rope_cs != nullptr && col0 < 2 * p.rope_d && ncols == 32) epilogue_rope(p, row, col0, acc);
   if (p.append.cs != nullptr && col0 < 2 * p.append.d)        // chunks are whole and inside a head (checked on the host)
-    epilogue_rope(p.append.cs, p.append.ctx, p.append.dh, p.append.positions[row], col0, acc);
+    epilogue_append_rope(p.append, row, col0, acc);
   if (p.epi == EPI_SWIGLU_BWD) {
     // as the stand-alone kernel (fast division apart): dh is rounded to bf16 first, gate and up are read as bf16
     const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)row * p.ldr + col0;

@@ -1,83 +1,46 @@
-// bf16 product of at most 128 rows with a weight matrix, D[m, n] = sum_k A(m, k) B(n, k): decode steps, which stream the weights once.
+// bf16 product of at most 128 rows with a weight matrix, D[m, n] = sum_k A(m, k) B(n, k), whose contraction is cut in slices: the long
+// products of decode steps, which stream the weights once.
 //
 // The weights are the 128-row operand of the MMA and the rows of A its columns, so a k-block of 64 costs four MMAs for 16 KB of weights
-// however few rows there are.  (With A as the 128-row operand and 32 or 64 weight rows as columns, as the general kernel has it, a
-// k-block takes 0.175 us for 4 or 8 KB of weights, from L2 as from DRAM: its copies and MMAs take as long to issue as ones of full size.)
-// There are few tiles of 128 weight rows, so K is cut in slices, one for each CTA of a cluster; a CTA leaves its sums in its shared
-// memory and then adds its share of the output rows over the cluster's CTAs, in slice order.  No workspace in global memory.
+// however few rows there are.  (With A as the 128-row operand and 64 weight rows as columns, as the general kernel has it, a k-block
+// takes 0.175 us for 8 KB of weights, from L2 as from DRAM: its copies and MMAs take as long to issue as ones of full size.)
+// Each CTA of a cluster has a slice of K; it leaves its sums in its shared memory and then adds its share of the output rows over the
+// cluster's CTAs, in slice order.  No workspace in global memory.  The slices are those of the general kernel's plan and are added in
+// the same order, so the results are the same bits.
 //
 //   warp 0      TMA producer     warp 1      MMA issuer     warps 2-9   accumulator -> shared memory     all warps   sums and output
-//
-// HALVES == 2: the gated product.  B holds gate rows, then up rows; a tile is 128 of each and the output act(gate) * up.
 #include "gemm_common.cuh"
 
 namespace b200 {
 
 int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_cols, uint32_t box_rows);
 
-// M up to 64 is where this beats the general kernel (both in us, one / 20 / 64 rows): N x K = 6144 x 2048 7.3 / 7.9 / 9.2 for 9.3 / 9.4 /
-// 9.5, 2048 x 2048 4.5 / 4.9 / 6.0 for 8.4 / 8.5 / 8.6, 2048 x 5504 7.5 / 7.9 / 9.3 for 11.0 / 11.0 / 11.1; at 128 rows 6144 x 2048 takes
-// 11.0 for 9.9.  With more tiles than SMs (a vocabulary) the general kernel is level or better: the caller keeps those there.
+// us, one / 20 / 64 rows, N x K = 2048 x 5504 in four slices: the general kernel 11.8 / 12.5 / 13.0, this 9.1 / 9.9 / 10.9.  Clusters of four and
+// more do not fill the chip (16 tiles in eight slices 12.0 us): the caller keeps to those that run at once.
 constexpr int FR_MAX_STAGES = 16, FR_THREADS = 320, FR_W_BYTES = BM * BK * 2;
 constexpr int FR_SMEM = 227 * 1024;
 
 struct FewRowsParams {
-  int M, N, K;                // N: columns of the output (rows of one half of B)
+  int M, N, K;                
   int xrows;                  // rows of A that are copied: M rounded up to 8
-  int stages, splits, b_early, epi, relu, finished;
+  int stages, splits, b_early, epi, finished;
   void* C;
   long long ldc;
   const void* R;
   long long ldr;
   GemmFinish finish;
-  QkvAppend append;
   uint32_t* status;
 };
 
-// What an output row needs from elsewhere, requested before its sums: four columns of the residual row, or of a row of Q, K or V (see
-// QkvAppend) the angles and the slot.  The four columns lie in one head.
-struct RowNeeds {
-  uint2 res;
-  float2 c, s;
-  long long slot;
-};
-
-__device__ __forceinline__ void fr_need(const FewRowsParams& p, int m, int n, RowNeeds& x) {
-  if (p.epi == EPI_BF16_RES) {
-    const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)m * p.ldr + n;
-    if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(r) & 7) == 0) {
-      x.res = *reinterpret_cast<const uint2*>(r);
-    } else {
-      uint16_t e[4] = {0, 0, 0, 0};
+// Four columns of the residual row, requested before the sums.
+__device__ __forceinline__ uint2 fr_residual(const FewRowsParams& p, int m, int n) {
+  const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)m * p.ldr + n;
+  if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(r) & 7) == 0) return *reinterpret_cast<const uint2*>(r);
+  uint16_t e[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (n + j < p.N) e[j] = reinterpret_cast<const uint16_t*>(r)[j];
-      x.res = make_uint2(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16);
-    }
-  }
-  const QkvAppend& a = p.append;
-  if (a.cs == nullptr) return;
-  if (n < 2 * a.d) {
-    const float* cs = a.cs + (size_t)a.positions[m] * (a.dh / 2) + n % a.dh / 2;
-    x.c = *reinterpret_cast<const float2*>(cs);
-    x.s = *reinterpret_cast<const float2*>(cs + (size_t)a.ctx * (a.dh / 2));
-  }
-  x.slot = n >= a.d ? append_slot(a, m, p.status) : -1;
-}
-
-__device__ __forceinline__ void fr_append(const FewRowsParams& p, const RowNeeds& x, int n, float (&v)[4]) {
-  const QkvAppend& a = p.append;
-  if (n < 2 * a.d) {
-    const float x0 = v[0], x1 = v[1], x2 = v[2], x3 = v[3];
-    v[0] = x.c.x * x0 - x.s.x * x1;
-    v[1] = x.s.x * x0 + x.c.x * x1;
-    v[2] = x.c.y * x2 - x.s.y * x3;
-    v[3] = x.s.y * x2 + x.c.y * x3;
-  }
-  if (x.slot < 0) return;
-  const bool is_k = n < 2 * a.d;
-  *reinterpret_cast<uint2*>((is_k ? a.k_cache : a.v_cache) + x.slot * a.d + (n - (is_k ? 1 : 2) * a.d)) =
-      make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+  for (int j = 0; j < 4; ++j)
+    if (n + j < p.N) e[j] = reinterpret_cast<const uint16_t*>(r)[j];
+  return make_uint2(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16);
 }
 
 __device__ __forceinline__ void fr_cluster_sync() {
@@ -140,7 +103,6 @@ __device__ __forceinline__ void fr_report(const FewRowsParams& p, volatile uint3
   if (p.status != nullptr) atomicCAS(p.status, 0u, code | (blockIdx.x << 8));
 }
 
-template <int HALVES>
 __global__ void __launch_bounds__(FR_THREADS)
 gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const FewRowsParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -153,7 +115,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   uint8_t* smem_x = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1024 + 1023) & ~uintptr_t(1023));
   const int x_bytes = p.xrows * (BK * 2), stages = p.stages;
   uint8_t* smem_w = smem_x + stages * x_bytes;
-  float* part = reinterpret_cast<float*>(smem_x);             // (HALVES, M, 128) sums, when the ring is read no more
+  float* part = reinterpret_cast<float*>(smem_x);             // (M, 128) sums, when the ring is read no more
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = blockIdx.x / p.splits, rank = blockIdx.x - tile * p.splits;
@@ -162,14 +124,10 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   const int kb_lo = rank * num_kb / p.splits, kb_hi = (rank + 1) * num_kb / p.splits;
   const int cols = (p.M + 15) / 16 * 16;
   uint32_t tmem_cols = 32;
-  while (tmem_cols < (uint32_t)(HALVES * cols)) tmem_cols *= 2;
-  const uint32_t stage_bytes = x_bytes + HALVES * FR_W_BYTES;
+  while (tmem_cols < (uint32_t)cols) tmem_cols *= 2;
+  const uint32_t stage_bytes = x_bytes + FR_W_BYTES;
 
-  auto load_w = [&](int stage, int kb) {
-#pragma unroll
-    for (int h = 0; h < HALVES; ++h)
-      tma_load_2d(smem_w + (stage * HALVES + h) * FR_W_BYTES, &tmW, &full_bar[stage], kb * BK, n0 + h * p.N);
-  };
+  auto load_w = [&](int stage, int kb) { tma_load_2d(smem_w + stage * FR_W_BYTES, &tmW, &full_bar[stage], kb * BK, n0); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -195,8 +153,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   tc_fence_before();
   __syncthreads();          // the CTA holds its tensor memory before the kernel after this one may be placed beside it
   tc_fence_after();
-  pdl_wait();
-  if (p.append.cs == nullptr) pdl_trigger();      // attention comes next otherwise
+  pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
 
   if (warp == 0) {
@@ -233,13 +190,11 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
           break;
         }
         tc_fence_after();
-        const uint32_t x_base = smem_u32(smem_x + stage * x_bytes), w_base = smem_u32(smem_w + stage * HALVES * FR_W_BYTES);
+        const uint32_t x_base = smem_u32(smem_x + stage * x_bytes), w_base = smem_u32(smem_w + stage * FR_W_BYTES);
 #pragma unroll
-        for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_f16_ss(tmem_base + h * cols, make_smem_desc(w_base + h * FR_W_BYTES + k * (UMMA_K * 2), 16, 1024),
-                        make_smem_desc(x_base + k * (UMMA_K * 2), 16, 1024), idesc, (kb > kb_lo || k > 0) ? 1u : 0u);
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_f16_ss(tmem_base, make_smem_desc(w_base + k * (UMMA_K * 2), 16, 1024), make_smem_desc(x_base + k * (UMMA_K * 2), 16, 1024), idesc,
+                      (kb > kb_lo || k > 0) ? 1u : 0u);
         umma_commit(&empty_bar[stage]);
         if (++stage == stages) {
           stage = 0;
@@ -253,17 +208,15 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     if (mbar_wait(done_bar, 0, abort_word)) {
       tc_fence_after();
 #pragma unroll 1
-      for (int h = 0; h < HALVES; ++h)
-#pragma unroll 1
-        for (int m0 = (warp - 2) / 4 * 16; m0 < p.M; m0 += 32) {
-          uint32_t r[16];
-          tmem_ld_32x16(tmem_base + (uint32_t(quarter * 32) << 16) + h * cols + m0, r);
-          tmem_ld_wait();
-          float* dst = part + (h * p.M + m0) * BM + quarter * 32 + lane;
+      for (int m0 = (warp - 2) / 4 * 16; m0 < p.M; m0 += 32) {
+        uint32_t r[16];
+        tmem_ld_32x16(tmem_base + (uint32_t(quarter * 32) << 16) + m0, r);
+        tmem_ld_wait();
+        float* dst = part + m0 * BM + quarter * 32 + lane;
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (m0 + j < p.M) dst[j * BM] = __uint_as_float(r[j]);
-        }
+        for (int j = 0; j < 16; ++j)
+          if (m0 + j < p.M) dst[j * BM] = __uint_as_float(r[j]);
+      }
       tc_fence_before();
     } else if (lane == 0) {
       fr_report(p, abort_word, ERR_WAIT_TMEM_FULL);
@@ -273,48 +226,34 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   fr_cluster_sync();        // all slices' sums are in place
   {
     // rows of this CTA: every splits-th, dealt to the warps; a warp adds ROWS of them at a time, a lane four columns of each
-    constexpr int ROWS = HALVES == 1 ? 4 : 2;
+    constexpr int ROWS = 4;
     const uint32_t base = smem_u32(part) + lane * 16;
     const int n = n0 + lane * 4, step = p.splits * (FR_THREADS / 32);
     if (n < p.N) {
       for (int m = rank + p.splits * warp; m < p.M; m += ROWS * step) {
-        RowNeeds needs[ROWS];
-        if (HALVES == 1) {
+        uint2 res[ROWS];
+        float v[ROWS][4] = {};
 #pragma unroll
-          for (int i = 0; i < ROWS; ++i)
-            if (m + i * step < p.M) fr_need(p, m + i * step, n, needs[i]);
-        }
-        float v[HALVES][ROWS][4] = {};
+        for (int i = 0; i < ROWS; ++i)
+          if (p.epi == EPI_BF16_RES && m + i * step < p.M) res[i] = fr_residual(p, m + i * step, n);
 #pragma unroll 4
         for (int s = 0; s < p.splits; ++s) {
-          float4 t[HALVES][ROWS];
+          float4 t[ROWS];
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h)
+          for (int i = 0; i < ROWS; ++i)
+            if (m + i * step < p.M) t[i] = fr_remote(base + (m + i * step) * (BM * 4), s);
 #pragma unroll
-            for (int i = 0; i < ROWS; ++i)
-              if (m + i * step < p.M) t[h][i] = fr_remote(base + (h * p.M + m + i * step) * (BM * 4), s);
-#pragma unroll
-          for (int h = 0; h < HALVES; ++h)
-#pragma unroll
-            for (int i = 0; i < ROWS; ++i)
-              if (m + i * step < p.M) {
-                v[h][i][0] += t[h][i].x; v[h][i][1] += t[h][i].y; v[h][i][2] += t[h][i].z; v[h][i][3] += t[h][i].w;
-              }
+          for (int i = 0; i < ROWS; ++i)
+            if (m + i * step < p.M) {
+              v[i][0] += t[i].x; v[i][1] += t[i].y; v[i][2] += t[i].z; v[i][3] += t[i].w;
+            }
         }
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) {
           if (m + i * step >= p.M) break;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (HALVES == 2) {
-              const float g = v[0][i][j];
-              v[0][i][j] = (p.relu ? fmaxf(g, 0.f) : __fdividef(g, 1.f + __expf(-g))) * v[HALVES - 1][i][j];
-            } else {
-              v[0][i][j] = fr_finish(p, v[0][i][j], n + j);
-            }
-          }
-          if (HALVES == 1 && p.append.cs != nullptr) fr_append(p, needs[i], n, v[0][i]);
-          fr_store(p, m + i * step, n, needs[i].res, v[0][i]);
+          for (int j = 0; j < 4; ++j) v[i][j] = fr_finish(p, v[i][j], n + j);
+          fr_store(p, m + i * step, n, res[i], v[i]);
         }
       }
     }
@@ -333,51 +272,22 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   }
 }
 
-static int fr_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      return 148;
-    }
-    sms = n;
-  }
-  return sms;
-}
-
-// Slices of K, one for each CTA of a cluster.  Each slice keeps at least eight k-blocks (four where there are few CTAs), so that a
-// cluster's two barriers and the sums are the smaller part; all CTAs run at once.  Clusters of four and more do not fill the chip (the
-// SMs of a processing cluster are no multiple of them): 16 tiles in eight slices take 10.0 us, in six 7.5, in four 9.0 (N x K = 2048 x
-// 5504, one row; without slices 17.2).  48 tiles (6144 x 2048): two slices 7.3 us, three 10.8, one 9.8.
-static int fr_splits(int N, int K) {
-  const int tiles = (N + BM - 1) / BM, num_kb = (K + BK - 1) / BK;
-  const int cand[5] = {8, 6, 4, 3, 2};
-  for (int i = 0; i < 5; ++i) {
-    const int s = cand[i], ctas = tiles * s;
-    if (ctas <= (s >= 4 ? fr_sms() * 2 / 3 : fr_sms() * 9 / 10) && num_kb >= s * (ctas <= 64 ? 4 : 8)) return s;
-  }
-  return 1;
-}
-
-template <int HALVES>
 static int launch_few_rows(const CUtensorMap& tmX, const CUtensorMap& tmW, FewRowsParams p, cudaStream_t stream) {
-  auto kern = gemm_few_rows_kernel<HALVES>;
+  auto kern = gemm_few_rows_kernel;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FR_SMEM) != cudaSuccess) return -3;
     configured = true;
   }
   const int tiles = (p.N + BM - 1) / BM, num_kb = (p.K + BK - 1) / BK;
-  p.splits = fr_splits(p.N, p.K);
-  const int mine = (num_kb + p.splits - 1) / p.splits, stage = p.xrows * BK * 2 + HALVES * FR_W_BYTES;
+  const int mine = (num_kb + p.splits - 1) / p.splits, stage = p.xrows * BK * 2 + FR_W_BYTES;
   int stages = (FR_SMEM - 2048) / stage;
   if (stages > FR_MAX_STAGES) stages = FR_MAX_STAGES;
   if (stages > mine) stages = mine;
   if (stages < 2) stages = 2;
   p.stages = stages;
   int ring = stages * stage;
-  const int sums = HALVES * p.M * BM * 4;
+  const int sums = p.M * BM * 4;
   if (ring < sums) ring = sums;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * p.splits);
@@ -399,45 +309,28 @@ static int launch_few_rows(const CUtensorMap& tmX, const CUtensorMap& tmW, FewRo
 
 using namespace b200;
 
-// QKV projection of a serving step of at most 128 rows (see QkvAppend): C (M x 3 d) bf16.
-extern "C" int b200_gemm_few_rows_append(const void* A, const void* B, void* C, int M, int K, long long lda, long long ldb, long long ldc,
-                                         int epi, const QkvAppend* append, uint32_t* status, cudaStream_t stream) {
-  if (M <= 0 || K <= 0) return 0;
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7)) return -10;
-  if (M > BM || (epi & ~EPI_B_STABLE) != EPI_BF16 || append == nullptr || !qkv_append_ok(*append)) return -11;
-  FewRowsParams p = {};
-  p.M = M; p.N = 3 * append->d; p.K = K; p.xrows = (M + 7) / 8 * 8;
-  p.b_early = (epi & EPI_B_STABLE) ? 1 : 0; p.epi = EPI_BF16; p.C = C; p.ldc = ldc; p.append = *append; p.status = status;
-  CUtensorMap tmX, tmW;
-  int rc = make_tmap_bf16_2d(&tmX, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BK, (uint32_t)p.xrows);
-  if (rc) return -20 + rc;
-  rc = make_tmap_bf16_2d(&tmW, B, (uint64_t)p.N, (uint64_t)K, (uint64_t)ldb, BK, BM);
-  if (rc) return -30 + rc;
-  return launch_few_rows<1>(tmX, tmW, p, stream);
-}
-
-// C (M x N) = act(alpha * (A B^T + bias)) for M <= 128, both operands K-major.  epi: 0, 1, 2 or 3 (see GemmEpilogue), EPI_B_STABLE allowed.
-// gated: 0, or 1 silu, 2 relu: B has 2 N rows, C (bf16) receives act(gate) * up.  finish: as b200_gemm_bf16_finish, without GELU.
+// C (M x N) = act(alpha * (A B^T + bias)) for M <= 128, both operands K-major, K in `splits` slices (2 to 8, two k-blocks each at least).
+// epi: 0, 1, 2 or 3 (see GemmEpilogue), EPI_B_STABLE allowed.  finish: as b200_gemm_bf16_finish, without GELU.
 extern "C" int b200_gemm_few_rows(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
-                                  long long ldc, long long ldr, int epi, int gated, const GemmFinish* finish, uint32_t* status,
+                                  long long ldc, long long ldr, int epi, int splits, const GemmFinish* finish, uint32_t* status,
                                   cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7)) return -10;
   const int b_early = (epi & EPI_B_STABLE) ? 1 : 0;
   epi &= ~EPI_B_STABLE;
-  if (M > BM || gated < 0 || gated > 2 || (gated && (epi != EPI_BF16 || finish != nullptr))) return -11;
+  if (M > BM || splits < 2 || splits > 8 || (K + BK - 1) / BK < 2 * splits) return -11;
   if (epi != EPI_BF16 && epi != EPI_F32 && epi != EPI_BF16_RES && epi != EPI_F32_ACC) return -11;
   if (epi == EPI_BF16_RES && R == nullptr) return -11;
   if (finish != nullptr && finish->act == ACT_GELU) return -11;
   FewRowsParams p = {};
-  p.M = M; p.N = N; p.K = K; p.xrows = (M + 7) / 8 * 8;
-  p.b_early = b_early; p.epi = epi; p.relu = gated == 2; p.finished = finish != nullptr;
+  p.M = M; p.N = N; p.K = K; p.xrows = (M + 7) / 8 * 8; p.splits = splits;
+  p.b_early = b_early; p.epi = epi; p.finished = finish != nullptr;
   p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.status = status;
   if (finish != nullptr) p.finish = *finish;
   CUtensorMap tmX, tmW;
   int rc = make_tmap_bf16_2d(&tmX, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BK, (uint32_t)p.xrows);
   if (rc) return -20 + rc;
-  rc = make_tmap_bf16_2d(&tmW, B, (uint64_t)(gated ? 2 : 1) * N, (uint64_t)K, (uint64_t)ldb, BK, BM);
+  rc = make_tmap_bf16_2d(&tmW, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, BK, BM);
   if (rc) return -30 + rc;
-  return gated ? launch_few_rows<2>(tmX, tmW, p, stream) : launch_few_rows<1>(tmX, tmW, p, stream);
+  return launch_few_rows(tmX, tmW, p, stream);
 }

@@ -571,9 +571,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               epilogue_rope(p, row, col + 32, r1);
             }
             if (p.append.cs != nullptr && col < 2 * p.append.d && row < p.M) {
-              const int pos = p.append.positions[row];
-              epilogue_rope(p.append.cs, p.append.ctx, p.append.dh, pos, col, r0);
-              epilogue_rope(p.append.cs, p.append.ctx, p.append.dh, pos, col + 32, r1);
+              epilogue_append_rope(p.append, row, col, r0);
+              epilogue_append_rope(p.append, row, col + 32, r1);
             }
             if (p.epi == EPI_BF16_RES && row < p.M) {
               const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)row * p.ldr + col;

@@ -160,11 +160,6 @@ def glu(a, w, n: int, act: str):
         return mixer_torch.glu(a, w, n, act, out)
     lib = _lib()
     m, k = a.shape
-    if a.dtype == torch.bfloat16 and native.few_rows(m, n):
-        _check(lib.b200_gemm_few_rows(_ptr(a), _ptr(w), _ptr(out), None, m, n, k, a.stride(0), w.stride(0), out.stride(0), 0,
-                                      native.EPI_B_STABLE, 2 if act == "relu" else 1, None, _ptr(native.status_word(a.device)),
-                                      _stream()), "gemm_few_rows")
-        return out
     if a.dtype == torch.bfloat16 and act == "silu" and native.gemm_glu(a, w, out):
         return out
     if a.dtype == torch.bfloat16:

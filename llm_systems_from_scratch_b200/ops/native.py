@@ -399,8 +399,9 @@ def gemm(a, b, layout: str, out=None, out_dtype=None, residual=None, accumulate=
         return out
     if b_stable and layout == "nt":
         epi |= EPI_B_STABLE
-    if layout == "nt" and bn_hint == 0 and max_ctas == 0 and few_rows(m, n) and (finish is None or finish.act != ACT_GELU):
-        _check(lib.b200_gemm_few_rows(_ptr(a), _ptr(b), _ptr(out), _ptr(residual), m, n, k, lda, ldb, out.stride(0), ldr, epi, 0,
+    few = few_rows(m, n, k) if layout == "nt" and bn_hint == 0 and max_ctas == 0 and USE_SPLITK else 0
+    if few and (finish is None or finish.act != ACT_GELU):
+        _check(lib.b200_gemm_few_rows(_ptr(a), _ptr(b), _ptr(out), _ptr(residual), m, n, k, lda, ldb, out.stride(0), ldr, epi, few,
                                       None if finish is None else ctypes.byref(finish), _ptr(status_word(a.device)), _stream()),
                "b200_gemm_few_rows")
         return out
@@ -456,14 +457,18 @@ def _splitk_scratch(device):
     return got
 
 
-# The kernel for few rows of A (csrc/gemm_few_rows.cu), by size alone: its tiles are 128 output columns, and they have to leave it room to
-# cut K in slices (74 tiles in two slices are one CTA on each of 148 SMs).
-FEW_ROWS_MAX_M, FEW_ROWS_MAX_TILES = 64, 74
+FEW_ROWS_MAX_M = 64
 ACT_GELU = 1
 
 
-def few_rows(m: int, n: int) -> bool:
-    return m <= FEW_ROWS_MAX_M and -(-n // 128) <= FEW_ROWS_MAX_TILES
+@functools.lru_cache(maxsize=4096)
+def few_rows(m: int, n: int, k: int) -> int:
+    """K slices of the kernel for few rows of A (csrc/gemm_few_rows.cu), 0 where it does not apply: those of the split-K plan, whose results it
+    gives bit for bit, as long as all clusters run at once (two CTAs of three SMs for clusters of four and more)."""
+    if m > FEW_ROWS_MAX_M or k < SPLITK_MIN_K_DEFAULT:
+        return 0
+    _, s = splitk_plan(m, n, k)
+    return s if s > 1 and -(-n // 128) * s <= (98 if s > 3 else 132) and -(-k // 64) >= 2 * s else 0
 
 
 def splitk_plan(m: int, n: int, k: int) -> tuple[int, int]:

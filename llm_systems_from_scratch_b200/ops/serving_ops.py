@@ -25,8 +25,6 @@ def _lib():
         lib.b200_kv_append.restype = I
         lib.b200_rope_kv_append.argtypes = [P, P, P, P, P, P, L, I, I, I, L, P, P]
         lib.b200_rope_kv_append.restype = I
-        lib.b200_gemm_few_rows_append.argtypes = [P, P, P, I, I, L, L, L, I, P, P, P]
-        lib.b200_gemm_few_rows_append.restype = I
         lib.b200_gemm_bf16_append.argtypes = [P, P, P, I, I, L, L, L, I, P, P, P]
         lib.b200_gemm_bf16_append.restype = I
         lib.b200_gemm_bf16_pair_append.argtypes = [P, P, P, I, I, L, L, L, P, P, P]
@@ -84,12 +82,12 @@ class QkvAppend(ctypes.Structure):
 
 def qkv_rope_append(h, wqkv, cos_sin, positions, k_cache, v_cache, slot_mapping, n_heads: int):
     """qkv = h (R, d) @ wqkv (3 d, d)^T, then what ``rope_kv_append`` does with it, in the product's epilogue where the heads are made of its
-    chunks of columns (Q, K and V are then rounded once, not twice)."""
+    chunks of columns and its contraction is not cut in slices.  The same values either way."""
     r, k = h.shape
     d = wqkv.shape[0] // 3
     dh = d // n_heads
-    few = h.is_cuda and native.few_rows(r, 3 * d)
-    if h.is_cuda and (few or (dh % 32 == 0 and d % 64 == 0)):
+    sliced = native.USE_SPLITK and r <= native.SPLITK_MAX_M and k >= native.SPLITK_MIN_K
+    if h.is_cuda and dh % 32 == 0 and d % 64 == 0 and not sliced:
         native._req(h.dtype == torch.bfloat16 and wqkv.dtype == torch.bfloat16 and h.stride(1) == 1 and wqkv.stride(1) == 1
                     and wqkv.shape[1] == k and dh * n_heads == d, "bad projection")
         native._req(slot_mapping.dtype == torch.int64 and slot_mapping.numel() == r and slot_mapping.is_contiguous()
@@ -103,9 +101,6 @@ def qkv_rope_append(h, wqkv, cos_sin, positions, k_cache, v_cache, slot_mapping,
                          k_cache.shape[0] * k_cache.shape[1], d, dh, cos_sin.shape[1])
         args = (h.data_ptr(), wqkv.data_ptr(), out.data_ptr(), r, k, h.stride(0), wqkv.stride(0), 3 * d)
         tail = (ctypes.byref(what), native.status_word(h.device).data_ptr(), native._stream())
-        if few:
-            native._check(_lib().b200_gemm_few_rows_append(*args, native.EPI_B_STABLE, *tail), "gemm_few_rows_append")
-            return out
         rc = _lib().b200_gemm_bf16_pair_append(*args, *tail) if native.USE_PAIR and r >= native.PAIR_MIN_M else -13
         if rc == -13:                      # a small step, or the epilogue that the CTA pairs need is switched off
             rc = _lib().b200_gemm_bf16_append(*args, native.EPI_B_STABLE, *tail)

@@ -20,6 +20,7 @@ class TransformerBackend:
 
     splits_prompts = False
     page_size = 16
+    GATED_MIN_ROWS = 128              # steps of more rows multiply gate and up in their product's epilogue
 
     def __init__(self, model):
         model.use_custom_triton = True
@@ -58,7 +59,9 @@ class TransformerBackend:
         o = attend(qkv, li)
         x = ops.gemm(o, w.wo, "nt", residual=x, b_stable=True)
         h, _ = ops.rmsnorm_fwd(x, w.n2, cfg.eps)
-        h = mo.glu(h, w.wgu, cfg.d_ff, "silu") if x.is_cuda else ops.silu_mul_fwd(ops.gemm(h, w.wgu, "nt", b_stable=True))
+        # decode steps round gate and up before they are multiplied, whatever their rows
+        fused = x.is_cuda and x.shape[0] > self.GATED_MIN_ROWS
+        h = mo.glu(h, w.wgu, cfg.d_ff, "silu") if fused else ops.silu_mul_fwd(ops.gemm(h, w.wgu, "nt", b_stable=True))
         return ops.gemm(h, w.wdown, "nt", residual=x, b_stable=True)
 
     def forward(self, batch):

@@ -183,8 +183,10 @@ def test_qkv_projection_that_rotates_and_appends(rows, heads, dh):
     turn = want[:, :2 * d].reshape(rows, 2 * heads, dh // 2, 2)
     c, s = (t[positions.long()].double()[:, None] for t in table)
     want[:, :2 * d] = torch.stack((turn[..., 0] * c - turn[..., 1] * s, turn[..., 0] * s + turn[..., 1] * c), -1).reshape(rows, 2 * d)
-    # one rounding to bf16 is at most 2^-9 (the path in three steps has two)
-    assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+    assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8             # two roundings to bf16 of at most 2^-9
+    three, k3, v3 = native.gemm(h, w, "nt", b_stable=True), k0.clone(), v0.clone()
+    serving_ops.rope_kv_append(three, table, positions, k3, v3, slots, heads)
+    assert torch.equal(got, three) and torch.equal(k, k3) and torch.equal(v, v3)
     on = slots >= 0
     for cache, old, cols in ((k, k0, got[:, d:2 * d]), (v, v0, got[:, 2 * d:])):
         assert torch.equal(cache.view(-1, d)[slots[on]], cols[on])

@@ -201,3 +201,38 @@ def test_qkv_projection_that_rotates_and_appends(rows, heads, dh):
     on = (slots >= 0) & (slots < pages * page)
     rest = torch.ones(pages * page, dtype=torch.bool, device="cuda").index_fill_(0, slots[on], False)
     assert torch.equal(k.view(-1, d)[rest], k0.view(-1, d)[rest])
+
+
+@pytest.mark.parametrize("rows", [100, 129, 200])
+def test_decode_steps_of_any_size_round_gate_and_up(rows, monkeypatch):
+    """Logits of a step of single tokens, and tokens of the captured step of its bucket (128 or 256 rows), against the four launches one after
+    the other: the same bits, below and above the rows that a tile has."""
+    from llm_systems_from_scratch_b200 import ops
+    from llm_systems_from_scratch_b200.models.transformer import TransformerLM
+    from llm_systems_from_scratch_b200.ops import mixer_ops as mo, native
+    from llm_systems_from_scratch_b200.serving import ServingEngine
+    torch.manual_seed(0)
+    cfg = dict(vocab_size=503, context_length=64, d_model=256, num_layers=2, num_heads=4, d_ff=704, rope_theta=10000.0)
+    model = TransformerLM(**cfg, use_custom_triton=True).cuda().eval()
+    g = torch.Generator().manual_seed(rows)
+    prompts, singles = torch.randint(0, 503, (2, rows, 3), generator=g).tolist()
+
+    def steps():
+        eng = ServingEngine(model, page_size=16, max_batch=256, max_context=64)
+        reqs = [eng.open(i) for i in range(rows)]
+        eng.extend([(r, p, []) for r, p in zip(reqs, prompts)])
+        # from here on there are single tokens only
+        with monkeypatch.context() as at:
+            if plain:
+                at.setattr(mo, "glu", lambda h, w, n, act: ops.silu_mul_fwd(ops.gemm(h, w, "nt", b_stable=True)))
+            logits = [eng.extend([(r, [t[i]], [0]) for r, t in zip(reqs, singles)]) for i in range(2)]
+            for r in reqs:
+                r.output, r.prompt = [7], list(range(r.fed))
+                eng.sched.grow(r, r.fed + 2)
+            return logits, eng.decode(reqs)
+    plain = False
+    got, tokens = steps()
+    plain = True
+    want, expected = steps()
+    native.check_status()
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and tokens == expected

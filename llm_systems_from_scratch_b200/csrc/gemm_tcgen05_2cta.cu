@@ -142,7 +142,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     fence_barrier_init();
     prefetch_tensormap(&tmA);
     prefetch_tensormap(&tmB);
-    if (p.tma_store) prefetch_tensormap(&tmC);
+    if (p.tma_store && p.C != nullptr) prefetch_tensormap(&tmC);          // without C its map was never made
     if (p.tma_store && (p.swiglu_f > 0 || p.epi == EPI_SWIGLU_BWD)) prefetch_tensormap(&tmH);
   }
   if (warp == 1) {

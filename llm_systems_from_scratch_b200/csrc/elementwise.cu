@@ -638,8 +638,9 @@ __device__ __forceinline__ float2 exp_below2(float2 x, float minus_m) {
   const float2 t = __fmul2_rn(__fadd2_rn(x, make_float2(minus_m, minus_m)), make_float2(L2E, L2E));
   return make_float2(ex2(t.x), ex2(t.y));
 }
+// A NaN on either side is the maximum.
 __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
-  const __nv_bfloat162 m = __hmax2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  const __nv_bfloat162 m = __hmax2_nan(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&m);
 }
 
@@ -672,6 +673,10 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
     for (int u = 0; u < XENT_DEPTH; ++u)
       top = max_bf16x2(top, max_bf16x2(max_bf16x2(v[u].x, v[u].y), max_bf16x2(v[u].z, v[u].w)));
     const float2 t2 = unpack_bf16x2(top);
+    if (t2.x != t2.x || t2.y != t2.y) {
+      s = NAN;                            // the row's, whatever follows: no pass and no maximum drops it
+      continue;
+    }
     const float nm = fmaxf(m, fmaxf(t2.x, t2.y));
     if (nm == -INFINITY) continue;
     float2 add[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -687,12 +692,12 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
   for (int c = nvec * 8 + threadIdx.x; c < vocab; c += XENT_THREADS) {
     const float f = __bfloat162float(lr[c]);
     const float nm = fmaxf(m, f);
-    if (nm == -INFINITY) continue;
+    if (nm == -INFINITY && f == f) continue;
     s = s * __expf(m - nm) + __expf(f - nm);
     m = nm;
   }
   const float gm = block_max(m, red);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
+  if (m != -INFINITY) s *= __expf(m - gm);          // else no term (0) or a NaN
   const float gs = block_sum(s, red);
   const float lse = gm + logf(gs);
   const float nv = *n_valid;

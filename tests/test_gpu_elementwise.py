@@ -119,7 +119,7 @@ def test_xent(rows, v, ld):
 
 @pytest.mark.parametrize("rows,v", [(5, 1), (5, 7), (5, 8), (9, 4095), (9, 16384), (3, 16392), (3, 50257)])
 def test_xent_of_rows_of_any_length(rows, v):
-    """Ends of the passes of 16384 columns and of 8; logits of the lowest value, of minus infinity, and one that leads by far."""
+    """Ends of the passes of 8192 columns and of 8; logits of the lowest value, of minus infinity, and one that leads by far."""
     from llm_systems_from_scratch_b200.ops import native
     ld = -(-v // 8) * 8 + 8
     buf = (4 * torch.randn(rows, ld, generator=torch.Generator().manual_seed(v))).bfloat16().cuda()
@@ -141,6 +141,30 @@ def test_xent_of_rows_of_any_length(rows, v):
     diff = (buf[:, :v].double() - logits.grad).norm(dim=1)
     assert bool((diff <= 2.0 ** -8 * logits.grad.norm(dim=1) + 1e-7).all()), diff
     assert torch.equal(buf[:, v:], keep)
+
+
+@pytest.mark.parametrize("v", [1, 7, 8, 2056, 8192, 16392, 50257])
+def test_xent_keeps_a_nan(v):
+    """A NaN anywhere in a row is in its loss and gradients: alone, in all of the row, or as all that one thread sees in a pass (columns
+    [0, 8), [2048, 2056), [4096, 4104) and [6144, 6152)), beside minus infinity or finite values in later passes."""
+    from llm_systems_from_scratch_b200.ops import native
+    ld = -(-v // 8) * 8
+    buf = (4 * torch.randn(6, ld, generator=torch.Generator().manual_seed(v))).bfloat16().cuda()
+    first = torch.cat([torch.arange(a, a + 8) for a in range(0, 8192, 2048)])
+    first = first[first < v].cuda()
+    buf[0, v - 1] = torch.nan
+    buf[1, :v] = torch.nan
+    buf[2, first] = torch.nan
+    buf[3, first] = -torch.inf
+    buf[3, first[-1]] = torch.nan
+    buf[4, :v] = -torch.inf
+    buf[4, 0] = torch.nan
+    for row in range(6):
+        for fn in (native.xent_fwd, lambda *a, **k: native.xent_fwd_bwd(a[0], a[1], 1.0, **k)):
+            x = buf[row:row + 1].clone()
+            loss = fn(x, torch.tensor([v // 2], device="cuda"), valid_cols=v)
+            assert bool(loss.isnan()) == (row < 5)
+        assert bool(x[:, :v].isnan().all()) == (row < 5) and bool(x[:, :v].isnan().any()) == (row < 5)
 
 
 def test_argmax():

@@ -720,14 +720,16 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 f = exp_below2(unpack_bf16x2(w[i]), -lse);
-        e[2 * i] = f.x * k;
-        e[2 * i + 1] = f.y * k;
+        e[2 * i] = f.x;
+        e[2 * i + 1] = f.y;
       }
       if (at == tgt_vec) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-          if (at * 8 + i == tgt) e[i] -= k;
+          if (at * 8 + i == tgt) e[i] -= 1.f;          // before the factor: exact where the row is sure of its target
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) e[i] *= k;
       store8(lr + at * 8, e);
     }
   }

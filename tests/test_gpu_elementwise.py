@@ -167,6 +167,24 @@ def test_xent_keeps_a_nan(v):
         assert bool(x[:, :v].isnan().all()) == (row < 5) and bool(x[:, :v].isnan().any()) == (row < 5)
 
 
+def test_xent_of_a_row_sure_of_its_target():
+    """The target's gradient is (p - 1) k wherever the target lies: of p close to one the difference is exact, and a product with k before it is
+    not.  Columns 0 - 7 are read as a vector, 8 - 10 one by one; the rows hold the same two finite logits."""
+    from llm_systems_from_scratch_b200.ops import native
+    other = torch.arange(-15.0, -7.0, 0.0625, device="cuda")
+    got = []
+    for tgt, beside in ((0, 1), (5, 2), (10, 9)):
+        x = torch.full((other.numel(), 16), -torch.inf, device="cuda")
+        x[:, tgt], x[:, beside] = 0.0, other
+        x = x.bfloat16()
+        native.xent_fwd_bwd(x, torch.full((other.numel(),), tgt, device="cuda"), 1.0 / 3.0, valid_cols=11)
+        got.append(x[:, tgt].clone())
+    assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[2])
+    want = -torch.sigmoid(other.double()) / 3.0 / other.numel()
+    # p carries the roundings of the sum's logarithm and of the exponential, two units of 2^-23 each at most, then one rounding to bf16
+    assert bool(((got[0].double() - want).abs() <= 2.0 ** -21 / 3.0 / other.numel() + 2.0 ** -8 * want.abs()).all())
+
+
 def test_argmax():
     from llm_systems_from_scratch_b200.ops import native
     x = torch.randn(37, 50264, device="cuda").bfloat16()

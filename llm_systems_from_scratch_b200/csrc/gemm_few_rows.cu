@@ -1,4 +1,4 @@
-// bf16 product of at most 128 rows with a weight matrix, D[m, n] = sum_k A(m, k) B(n, k), whose contraction is cut in slices: the long
+// bf16 product of at most 64 rows with a weight matrix, D[m, n] = sum_k A(m, k) B(n, k), whose contraction is cut in slices: the long
 // products of decode steps, which stream the weights once.
 //
 // The weights are the 128-row operand of the MMA and the rows of A its columns, so a k-block of 64 costs four MMAs for 16 KB of weights
@@ -17,11 +17,11 @@ int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, uint64_t rows, uint64_t 
 
 // us, one / 20 / 64 rows, N x K = 2048 x 5504 in four slices: the general kernel 11.8 / 12.5 / 13.0, this 9.1 / 9.9 / 10.9.  Clusters of four and
 // more do not fill the chip (16 tiles in eight slices 12.0 us): the caller keeps to those that run at once.
-constexpr int FR_MAX_STAGES = 16, FR_THREADS = 320, FR_W_BYTES = BM * BK * 2;
+constexpr int FR_MAX_M = 64, FR_MAX_STAGES = 16, FR_THREADS = 320, FR_W_BYTES = BM * BK * 2;
 constexpr int FR_SMEM = 227 * 1024;
 
 struct FewRowsParams {
-  int M, N, K;                
+  int M, N, K;
   int xrows;                  // rows of A that are copied: M rounded up to 8
   int stages, splits, b_early, epi, finished;
   void* C;
@@ -309,7 +309,7 @@ static int launch_few_rows(const CUtensorMap& tmX, const CUtensorMap& tmW, FewRo
 
 using namespace b200;
 
-// C (M x N) = act(alpha * (A B^T + bias)) for M <= 128, both operands K-major, K in `splits` slices (2 to 8, two k-blocks each at least).
+// C (M x N) = act(alpha * (A B^T + bias)) for M <= 64, both operands K-major, K in `splits` slices (2 to 8, two k-blocks each at least).
 // epi: 0, 1, 2 or 3 (see GemmEpilogue), EPI_B_STABLE allowed.  finish: as b200_gemm_bf16_finish, without GELU.
 extern "C" int b200_gemm_few_rows(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                                   long long ldc, long long ldr, int epi, int splits, const GemmFinish* finish, uint32_t* status,
@@ -318,7 +318,7 @@ extern "C" int b200_gemm_few_rows(const void* A, const void* B, void* C, const v
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7)) return -10;
   const int b_early = (epi & EPI_B_STABLE) ? 1 : 0;
   epi &= ~EPI_B_STABLE;
-  if (M > BM || splits < 2 || splits > 8 || (K + BK - 1) / BK < 2 * splits) return -11;
+  if (M > FR_MAX_M || splits < 2 || splits > 8 || (K + BK - 1) / BK < 2 * splits) return -11;
   if (epi != EPI_BF16 && epi != EPI_F32 && epi != EPI_BF16_RES && epi != EPI_F32_ACC) return -11;
   if (epi == EPI_BF16_RES && R == nullptr) return -11;
   if (finish != nullptr && finish->act == ACT_GELU) return -11;

@@ -110,28 +110,29 @@ def bench_gemm_decode():
         return timeit(g.replay, iters=10, warm=2) * 1e3 / len(ws)
 
     for m in (64, 128, 256):
-        tot = {"plain": 0.0, "splitk": 0.0, "cublas": 0.0}
+        tot = {"plain": 0.0, "splitk": 0.0, "default": 0.0, "cublas": 0.0}
         for name, n, k, reps in shapes:
             a = torch.randn(m, k, device="cuda").bfloat16()
             out = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
-            prev = native.USE_SPLITK
-            native.USE_SPLITK = False
+            prev, few = native.USE_SPLITK, native.FEW_ROWS_MAX_M
+            t_default = graph_us(lambda w: native.gemm(a, w, "nt", out=out), weights[name])
+            native.USE_SPLITK, native.FEW_ROWS_MAX_M = False, 0
             t_plain = graph_us(lambda w: native.gemm(a, w, "nt", out=out), weights[name])
             native.USE_SPLITK = True
             native.SPLITK_MIN_K = 0
             t_split = graph_us(lambda w: native.gemm(a, w, "nt", out=out), weights[name])
-            native.USE_SPLITK = prev
+            native.USE_SPLITK, native.FEW_ROWS_MAX_M = prev, few
             native.SPLITK_MIN_K = native.SPLITK_MIN_K_DEFAULT
             t_lib = graph_us(lambda w: torch.matmul(a, w.t(), out=out), weights[name])
             native.check_status()
             bn, splits = native.splitk_plan(m, n, k)
             w_us = n * k * 2 / 6541.8e3
             per_step = 1 if name == "lm_head" else 24
-            for key, t in (("plain", t_plain), ("splitk", t_split), ("cublas", t_lib)):
+            for key, t in (("plain", t_plain), ("splitk", t_split), ("default", t_default), ("cublas", t_lib)):
                 tot[key] += per_step * t / 1e3
             print(json.dumps({"op": "gemm-decode", "name": name, "m": m, "n": n, "k": k, "split_tile_n": bn,
                               "k_slices": splits, "plain_us": round(t_plain, 2), "splitk_us": round(t_split, 2),
-                              "cublas_us": round(t_lib, 2), "weights_at_copy_bw_us": round(w_us, 2)}), flush=True)
+                              "default_us": round(t_default, 2), "cublas_us": round(t_lib, 2), "weights_at_copy_bw_us": round(w_us, 2)}), flush=True)
         print(json.dumps({"op": "gemm-decode-step", "m": m, "layers": 24,
                           **{k + "_ms": round(v, 3) for k, v in tot.items()}}), flush=True)
 

@@ -236,6 +236,12 @@ USE_PAIR = os.environ.get("B200_GEMM_PAIR", "1") == "1"
 FORCE_PAIR = os.environ.get("B200_GEMM_FORCE_PAIR", "0") == "1"
 
 
+@functools.lru_cache(maxsize=1)
+def _sms() -> int:
+    """SMs of the current device; a B200's on a machine without one."""
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count if torch.cuda.is_available() else 148
+
+
 def _pair_pays(m: int, n: int, sms: int = 148) -> bool:
     """Wave model of the two tensor-core kernels.  A 256x256 tile on a CTA pair is the unit of time; a 128x128
     tile on one SM is a quarter of the work on half the hardware at about 0.8 of the efficiency.  Small weight
@@ -256,7 +262,7 @@ def pair_tail_plan(m: int, n: int, k: int) -> tuple[int, int, bool]:
     fn.restype, fn.argtypes = c_ll, [c_int, c_int, c_int, c_void_p, c_void_p]
     splits, cost = c_int(1), ctypes.c_double(0.0)
     floats = int(fn(m, n, k, ctypes.byref(splits), ctypes.byref(cost)))
-    waves = -(-(-(-m // 128) * -(-n // 128)) // 148)
+    waves = -(-(-(-m // 128) * -(-n // 128)) // _sms())
     return splits.value, floats, cost.value <= waves * 0.625 * -(-k // 64) + 8
 
 
@@ -457,18 +463,28 @@ def _splitk_scratch(device):
     return got
 
 
+# Rows up to which a product whose contraction is sliced takes the kernel for few rows (csrc/gemm_few_rows.cu): those of the decode buckets up
+# to 64, which it was brought in for (0 switches it off).  N x K = 2048 x 5504, general kernel -> this one, us: one row 11.9 -> 9.1, 20 rows
+# 12.5 -> 9.7, 64 rows 12.9 -> 10.6.  Steps of 65 to 128 rows stay with the general kernel, although it is not the faster one there either
+# (13.6 at 128 rows, 11.8 with this kernel's tiles of 128).
 FEW_ROWS_MAX_M = 64
 ACT_GELU = 1
 
 
-@functools.lru_cache(maxsize=4096)
 def few_rows(m: int, n: int, k: int) -> int:
-    """K slices of the kernel for few rows of A (csrc/gemm_few_rows.cu), 0 where it does not apply: those of the split-K plan, whose results it
-    gives bit for bit, as long as all clusters run at once (two CTAs of three SMs for clusters of four and more)."""
-    if m > FEW_ROWS_MAX_M or k < SPLITK_MIN_K_DEFAULT:
+    """K slices of the kernel for few rows of A, 0 where it does not apply: those of the split-K plan, whose results it gives bit for bit.
+    Contractions below ``SPLITK_MIN_K`` are not sliced; where that switch is lowered, to time or test the general kernel's slices, the general
+    kernel takes them."""
+    if m > FEW_ROWS_MAX_M or k < max(SPLITK_MIN_K, SPLITK_MIN_K_DEFAULT):
         return 0
+    return _few_rows_slices(m, n, k)
+
+
+@functools.lru_cache(maxsize=4096)
+def _few_rows_slices(m: int, n: int, k: int) -> int:
+    # all clusters have to run at once: clusters of four and more fill two SMs of three (98 of 148), smaller ones nine of ten
     _, s = splitk_plan(m, n, k)
-    return s if s > 1 and -(-n // 128) * s <= (98 if s > 3 else 132) and -(-k // 64) >= 2 * s else 0
+    return s if s > 1 and -(-n // 128) * s <= _sms() * (98 if s > 3 else 132) // 148 and -(-k // 64) >= 2 * s else 0
 
 
 def splitk_plan(m: int, n: int, k: int) -> tuple[int, int]:

@@ -251,3 +251,20 @@ def test_split_k_plan_for_decode_shapes():
             assert s == 1 or (tiles * s * 128 * bn <= ws_floats and tiles * 4 <= counters and s <= (k + 63) // 64)
     assert native.splitk_plan(128, 2048, 5504)[1] > 1
     assert native.splitk_plan(128, 50264, 2048)[1] == 1
+
+
+def test_slicing_switches_govern_the_kernel_for_few_rows(monkeypatch):
+    """One threshold for all sliced products: raising it turns the kernel for few rows off as well.  Lowering it leaves short contractions to
+    the general kernel's slices, and 0 rows switches the kernel off."""
+    from llm_systems_from_scratch_b200.ops import native
+    monkeypatch.setattr(native, "splitk_plan", lambda m, n, k: (64, 4))
+    native._few_rows_slices.cache_clear()
+    assert native.few_rows(1, 2048, 5504) == native.few_rows(64, 2048, 5504) == 4
+    assert not native.few_rows(65, 2048, 5504) and not native.few_rows(1, 2048, 4032)
+    monkeypatch.setattr(native, "SPLITK_MIN_K", 8192)
+    assert not native.few_rows(1, 2048, 5504) and native.few_rows(1, 2048, 8192) == 4
+    monkeypatch.setattr(native, "SPLITK_MIN_K", 0)
+    assert native.few_rows(1, 2048, 5504) == 4 and not native.few_rows(1, 2048, 2048)
+    monkeypatch.setattr(native, "FEW_ROWS_MAX_M", 0)
+    assert not native.few_rows(1, 2048, 5504)
+    native._few_rows_slices.cache_clear()

@@ -1168,8 +1168,12 @@ extern "C" int b200_xent(void* logits, const long long* targets, float* loss, fl
 extern "C" int b200_argmax(const void* logits, long long rows, long long ld, int vocab, int f32, long long* out,
                            cudaStream_t st) {
   if (rows == 0) return 0;
-  if (f32) launch_dep(argmax_kernel<float>, (unsigned)rows, 1024, 0, st, (const float*)logits, ld, vocab, out);
-  else launch_dep(argmax_kernel<__nv_bfloat16>, (unsigned)rows, 1024, 0, st, (const __nv_bfloat16*)logits, ld, vocab, out);
+  // A thread for every 16 bytes of a row, up to 1024 where the rows alone do not fill the chip and 256 where two blocks per SM do: threads
+  // beyond that only wait for the others.  4096 rows, 1024 threads -> now, us: 503 columns 36 -> 4.6, 50257 columns 115 -> 68.
+  const int vecs = vocab / (f32 ? 4 : 8), most = rows > 148 * 2 ? 256 : 1024;
+  const int threads = vecs >= most ? most : vecs <= 64 ? 64 : (vecs + 31) / 32 * 32;
+  if (f32) launch_dep(argmax_kernel<float>, (unsigned)rows, threads, 0, st, (const float*)logits, ld, vocab, out);
+  else launch_dep(argmax_kernel<__nv_bfloat16>, (unsigned)rows, threads, 0, st, (const __nv_bfloat16*)logits, ld, vocab, out);
   CHECK_LAUNCH();
 }
 

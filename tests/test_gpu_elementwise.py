@@ -192,6 +192,22 @@ def test_argmax():
     assert torch.equal(got, x[:, :50257].float().argmax(-1))
 
 
+@pytest.mark.parametrize("rows", [296, 297])
+@pytest.mark.parametrize("cols", [1, 7, 519, 520, 1032, 2056, 8200])
+def test_argmax_of_many_rows(rows, cols):
+    """Block sizes by columns and rows: rows that start anywhere, ties and the ends of what the threads take."""
+    from llm_systems_from_scratch_b200.ops import native
+    for dtype in (torch.bfloat16, torch.float32):
+        x = torch.randn(rows, cols + 9, generator=torch.Generator().manual_seed(cols)).to(dtype).cuda()[:, 1:]
+        x[:, cols:] = 99.0
+        at = torch.randint(0, cols, (2, rows), generator=torch.Generator().manual_seed(rows)).cuda()
+        x.scatter_(1, at.T, 50.0)
+        at[:, 0], at[:, 1] = cols - 1, 0
+        x[0, :cols], x[1, :cols] = 0.0, -torch.inf
+        x[0, cols - 1], x[1, 0] = 50.0, 50.0
+        assert torch.equal(native.argmax_rows(x, valid_cols=cols), at.amin(0))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("cols", [1, 3, 8, 9, 1023, 8191, 32768, 32775])
 @pytest.mark.parametrize("start", [0, 1, 7])

@@ -487,15 +487,18 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ tokens, const
 }
 
 // Deterministic variant: `order` lists the token rows sorted by token id (stable), `sorted_tokens` the ids in that
-// order.  The sorted rows are cut into segments of EMB_SEG; one warp per segment and 256 columns adds its rows in order in
-// fp32 registers, eight rows in flight.  A run of equal ids that lies inside a segment is written to its table row at once; what
+// order.  The sorted rows are cut into segments of SEG; one warp per segment and 256 columns adds its rows in order in
+// fp32 registers, up to eight rows in flight.  A run of equal ids that lies inside a segment is written to its table row at once; what
 // a run leaves in a segment that it enters from the left, or goes on from to the right, goes to `parts` (two rows per segment), and
 // embedding_bwd_join_kernel adds those in segment order.  No atomics: bitwise reproducible.
 // Bound by reading dx once.  Text repeats few ids often (with Zipf's law one id in sixteen is the most frequent one), and one warp per
 // run, as it was, spent the whole launch on the longest run: 1630 us at 16384 x 2048 and a vocabulary of 50257, now 29 + 16 us.
 // OUT = float: the fp32 gradient table; OUT = __nv_bfloat16: a bf16 staging table (multi-GPU gradient staging),
 // written once per row from the fp32 sum of the run (accumulate is not offered there).
-constexpr int EMB_SEG = 16;
+// SEG is 16, and 4 up to 2048 rows, where a warp's table rows, one after the other, are the launch (us with the sort, SEG 16 -> 4: 64 rows x 512
+// 19.0 -> 15.5, 1024 x 2048 39 -> 35; 2048 rows of one id 46 -> 69, by the join).
+constexpr int EMB_FEW_ROWS = 2048;
+static int emb_seg(long long rows) { return rows <= EMB_FEW_ROWS ? 4 : 16; }
 
 template <typename OUT>
 __device__ __forceinline__ void emb_store(OUT* dst, const float (&acc)[8], int accumulate) {
@@ -514,17 +517,18 @@ __device__ __forceinline__ void emb_store(OUT* dst, const float (&acc)[8], int a
   }
 }
 
-template <typename OUT>
+template <int SEG, typename OUT>
 __global__ void __launch_bounds__(256)
 embedding_bwd_sorted_kernel(const long long* __restrict__ sorted_tokens, const long long* __restrict__ order,
                             const __nv_bfloat16* __restrict__ dx, OUT* __restrict__ grad_table, float* __restrict__ parts,
                             long long rows, int d, int vocab, int accumulate) {
   pdl_sync();
+  constexpr int IN = SEG < 8 ? SEG : 8;       // rows in flight
   const int lane = threadIdx.x & 31;
   const long long seg = blockIdx.x * 8ll + (threadIdx.x >> 5);
-  const long long j0 = seg * EMB_SEG;
+  const long long j0 = seg * SEG;
   if (j0 >= rows) return;
-  const int n = (int)min((long long)EMB_SEG, rows - j0);
+  const int n = (int)min((long long)SEG, rows - j0);
   const int c = blockIdx.y * 256 + lane * 8;
   // lanes [0, n): the segment's ids and rows; lane n: the id behind it (an id of no token past the end)
   const long long tok = lane < n || (lane == n && j0 + n < rows) ? sorted_tokens[j0 + lane] : -1;
@@ -535,16 +539,16 @@ embedding_bwd_sorted_kernel(const long long* __restrict__ sorted_tokens, const l
 #pragma unroll
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
 #pragma unroll
-  for (int half = 0; half < EMB_SEG / 8; ++half) {
-    uint4 v[8];
+  for (int half = 0; half < SEG / IN; ++half) {
+    uint4 v[IN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const long long r = __shfl_sync(0xffffffffu, src, half * 8 + i);
-      if (half * 8 + i < n && c < d) v[i] = *reinterpret_cast<const uint4*>(dx + (size_t)r * d + c);
+    for (int i = 0; i < IN; ++i) {
+      const long long r = __shfl_sync(0xffffffffu, src, half * IN + i);
+      if (half * IN + i < n && c < d) v[i] = *reinterpret_cast<const uint4*>(dx + (size_t)r * d + c);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int at = half * 8 + i;
+    for (int i = 0; i < IN; ++i) {
+      const int at = half * IN + i;
       const long long t = __shfl_sync(0xffffffffu, tok, at), next = __shfl_sync(0xffffffffu, tok, at + 1);
       if (at >= n) continue;
       const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
@@ -569,28 +573,28 @@ embedding_bwd_sorted_kernel(const long long* __restrict__ sorted_tokens, const l
 }
 
 // One warp per segment in which a run begins that goes on behind it: row 1 of the segment, then row 0 of every segment that the run reaches.
-template <typename OUT>
+template <int SEG, typename OUT>
 __global__ void __launch_bounds__(256)
 embedding_bwd_join_kernel(const long long* __restrict__ sorted_tokens, const float* __restrict__ parts, OUT* __restrict__ grad_table,
                           long long rows, int d, int vocab, int accumulate) {
   pdl_sync();
   const int lane = threadIdx.x & 31;
   const long long seg = blockIdx.x * 8ll + (threadIdx.x >> 5);
-  const long long j0 = seg * EMB_SEG, j1 = j0 + EMB_SEG;
+  const long long j0 = seg * SEG, j1 = j0 + SEG;
   if (j1 >= rows) return;
   const long long t = sorted_tokens[j1 - 1];
   if (t < 0 || t >= vocab || sorted_tokens[j1] != t) return;
   if (j0 > 0 && sorted_tokens[j0] == t && sorted_tokens[j0 - 1] == t) return;        // the run began earlier
   long long reach = 1;                                             // segments behind this one that the run fills to their end
   for (;; reach += 32) {
-    const long long end = (seg + reach + lane + 1) * EMB_SEG;      // one behind the last row of that segment
+    const long long end = (seg + reach + lane + 1) * SEG;          // one behind the last row of that segment
     const unsigned on = __ballot_sync(0xffffffffu, end <= rows && sorted_tokens[end - 1] == t);
     if (on != 0xffffffffu) {
       reach += __ffs(~on) - 1;
       break;
     }
   }
-  const long long tail = (seg + reach) * EMB_SEG;                  // the run may end inside the segment behind those
+  const long long tail = (seg + reach) * SEG;                      // the run may end inside the segment behind those
   const long long count = tail < rows && sorted_tokens[tail] == t ? reach + 1 : reach;
   const int c = blockIdx.y * 256 + lane * 8;
   if (c >= d) return;
@@ -1114,25 +1118,32 @@ extern "C" int b200_embedding_bwd(const long long* tokens, const void* dx, float
   CHECK_LAUNCH();
 }
 
-// Deterministic embedding backward.  sorted_tokens / order: the token ids sorted ascending (stable) and the row
-// index of each; the table rows of tokens that occur are overwritten (accumulate = 0: the caller zeroes the rest)
-// or added to (accumulate = 1).  d must be a multiple of 8.
 // Floats of scratch that b200_embedding_bwd_sorted needs: two rows per segment.
-extern "C" long long b200_embedding_bwd_parts(long long rows, int d) { return 2 * ((rows + EMB_SEG - 1) / EMB_SEG) * (long long)d; }
+extern "C" long long b200_embedding_bwd_parts(long long rows, int d) { return 2 * ((rows + emb_seg(rows) - 1) / emb_seg(rows)) * (long long)d; }
+
+template <int SEG, typename OUT>
+static int embedding_bwd_segments(const long long* sorted_tokens, const long long* order, const void* dx, OUT* grad_table, float* parts,
+                                  long long rows, int d, int vocab, int accumulate, cudaStream_t st) {
+  const long long segs = (rows + SEG - 1) / SEG;
+  const dim3 grid((unsigned)((segs + 7) / 8), (unsigned)((d + 255) / 256));
+  launch_dep(embedding_bwd_sorted_kernel<SEG, OUT>, grid, 256, 0, st, sorted_tokens, order, (const __nv_bfloat16*)dx, grad_table, parts, rows, d,
+             vocab, accumulate);
+  launch_dep(embedding_bwd_join_kernel<SEG, OUT>, grid, 256, 0, st, sorted_tokens, parts, grad_table, rows, d, vocab, accumulate);
+  CHECK_LAUNCH();
+}
 
 template <typename OUT>
 static int embedding_bwd_sorted(const long long* sorted_tokens, const long long* order, const void* dx, OUT* grad_table, float* parts,
                                 long long rows, int d, int vocab, int accumulate, cudaStream_t st) {
   if (d % 8 || !ALIGNED16(dx) || !ALIGNED16(grad_table) || !ALIGNED16(parts)) return -10;
   if (rows == 0) return 0;
-  const long long segs = (rows + EMB_SEG - 1) / EMB_SEG;
-  const dim3 grid((unsigned)((segs + 7) / 8), (unsigned)((d + 255) / 256));
-  launch_dep(embedding_bwd_sorted_kernel<OUT>, grid, 256, 0, st, sorted_tokens, order, (const __nv_bfloat16*)dx, grad_table, parts, rows, d, vocab,
-                                                         accumulate);
-  launch_dep(embedding_bwd_join_kernel<OUT>, grid, 256, 0, st, sorted_tokens, parts, grad_table, rows, d, vocab, accumulate);
-  CHECK_LAUNCH();
+  return emb_seg(rows) == 4 ? embedding_bwd_segments<4>(sorted_tokens, order, dx, grad_table, parts, rows, d, vocab, accumulate, st)
+                            : embedding_bwd_segments<16>(sorted_tokens, order, dx, grad_table, parts, rows, d, vocab, accumulate, st);
 }
 
+// Deterministic embedding backward.  sorted_tokens / order: the token ids sorted ascending (stable) and the row
+// index of each; the table rows of tokens that occur are overwritten (accumulate = 0: the caller zeroes the rest)
+// or added to (accumulate = 1).  d must be a multiple of 8.
 extern "C" int b200_embedding_bwd_sorted(const long long* sorted_tokens, const long long* order, const void* dx,
                                          float* grad_table, float* parts, long long rows, int d, int vocab, int accumulate,
                                          cudaStream_t st) {

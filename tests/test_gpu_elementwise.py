@@ -341,21 +341,26 @@ def test_rmsnorm_bwd_variants_agree(rows, d):
     assert torch.equal(again[0], got[1][0]) and torch.equal(again[1], got[1][2])
 
 
-@pytest.mark.parametrize("runs", [(1,), (16,), (17,), (1, 15, 16, 17, 1), (7, 33, 8), (15, 1, 16, 600, 5), (3, 16, 16, 530), (16, 15, 2, 1)])
+@pytest.mark.parametrize("runs", [((0, 1),), ((39, 16),), ((7, 17),), ((0, 4),), ((-1, 16),), ((-1, 21),), ((77, 40),),
+                                  ((-3, 1), (2, 15), (5, 16), (6, 17), (77, 1)), ((-1, 7), (2, 33), (39, 8)),
+                                  ((2, 15), (5, 1), (6, 16), (39, 600), (77, 5)), ((-1, 3), (2, 16), (5, 16), (39, 530)),
+                                  ((-3, 16), (-1, 15), (0, 2), (77, 1)), ((-1, 4), (0, 4), (1, 8), (39, 3))])
+@pytest.mark.parametrize("more", [0, 2064])
 @pytest.mark.parametrize("d", [8, 264])
-def test_embedding_backward_segments(runs, d):
-    """Runs of equal ids that begin, end and lie anywhere in the segments the kernel works by, ids outside the table among them."""
+def test_embedding_backward_segments(runs, more, d):
+    """Runs (id, length) of equal ids that begin, end and lie anywhere in the segments the kernel works by, ids outside the table before, behind and
+    without others among them.  ``more`` rows of an id in the middle take the segments from 4 rows to 16."""
     from llm_systems_from_scratch_b200.ops import native
     v = 40
-    ids = torch.tensor([-3, 2, 5, 6, 39, 77][:len(runs) + 1][-len(runs):] if len(runs) > 3 else [0, 7, 39][:len(runs)])
-    tok = ids.repeat_interleave(torch.tensor(runs))
+    runs = runs + ((20, more),)
+    tok = torch.tensor([i for i, _ in runs]).repeat_interleave(torch.tensor([n for _, n in runs]))
     tok = tok[torch.randperm(tok.numel(), generator=torch.Generator().manual_seed(1))].cuda()
     dx = torch.randn(tok.numel(), d, device="cuda").bfloat16()
     seen = (tok >= 0) & (tok < v)
     want = torch.zeros(v, d, dtype=torch.float64, device="cuda").index_add_(0, tok[seen], dx[seen].double())
     size = torch.zeros(v, d, dtype=torch.float64, device="cuda").index_add_(0, tok[seen], dx[seen].double().abs())
     got = native.embedding_bwd(dx, tok, torch.empty(v, d, device="cuda"))
-    bound = size * max(runs) * 2.0 ** -24                        # fp32 sums in any order
+    bound = size * max(n for _, n in runs) * 2.0 ** -24                        # fp32 sums in any order
     assert bool(((got.double() - want).abs() <= bound).all())
     more = native.embedding_bwd(dx, tok, got.clone(), accumulate=True)
     assert bool(((more.double() - 2 * want).abs() <= 2 * bound + 2.0 ** -23 * want.abs()).all())

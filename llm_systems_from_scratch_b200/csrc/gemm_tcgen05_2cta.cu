@@ -570,10 +570,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               epilogue_rope(p, row, col, r0);
               epilogue_rope(p, row, col + 32, r1);
             }
-            if (p.append.cs != nullptr && col < 2 * p.append.d && row < p.M) {
-              epilogue_append_rope(p.append, row, col, r0);
-              epilogue_append_rope(p.append, row, col + 32, r1);
-            }
             if (p.epi == EPI_BF16_RES && row < p.M) {
               const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)row * p.ldr + col;
               if (col + 64 <= p.N && (p.ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(p.R) & 15) == 0) {
@@ -604,16 +600,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
           }
           emit(&tmC, col, o, p.epi == EPI_F32_ACC);
-          if (p.append.cs != nullptr && col >= p.append.d && row < p.M) {       // 64 columns of K or V, the d columns a multiple of 64
-            const long long slot = append_slot(p.append, row, p.status);
-            if (slot >= 0) {
-              const bool is_k = col < 2 * p.append.d;
-              uint4* dst = reinterpret_cast<uint4*>((is_k ? p.append.k_cache : p.append.v_cache) + slot * p.append.d +
-                                                    (col - (is_k ? 1 : 2) * p.append.d));
-#pragma unroll
-              for (int j = 0; j < 8; ++j) dst[j] = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-            }
-          }
         }
       } else {
 #pragma unroll 1
@@ -750,7 +736,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
                           uint32_t* status, cudaStream_t stream, const float* rope_cs = nullptr, int rope_seq = 0,
                           int rope_d = 0, int rope_dh = 0, int rope_ctx = 0, int swiglu_f = 0, void* H = nullptr,
                           long long ldh = 0, const ReduceTask* reduce = nullptr, const GemmFinish* finish = nullptr, int splits = 1,
-                          float* ws = nullptr, const QkvAppend* append = nullptr) {
+                          float* ws = nullptr) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return -10;
@@ -779,7 +765,6 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;
   p.append.cs = nullptr;
-  if (append != nullptr) p.append = *append;
   p.wait_counter = wait_counter; p.wait_value = wait_value; p.wait_limit_ns = g_counter_wait_limit_ns;
   p.rope_cs = rope_cs; p.rope_seq = rope_seq; p.rope_d = rope_d; p.rope_dh = rope_dh; p.rope_ctx = rope_ctx;
   p.swiglu_f = swiglu_f; p.H = H; p.ldh = ldh;
@@ -815,7 +800,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
     if (make_tmap_out_2d(&tmC, out_f32, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, out_f32 ? 32 : 64, 32) == 0)
       p.tma_store = 1;
   }
-  if ((C == nullptr || append != nullptr) && !p.tma_store) return -13;
+  if (C == nullptr && !p.tma_store) return -13;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -922,15 +907,6 @@ extern "C" int b200_gemm_bf16_pair_rope(const void* A, const void* B, void* C, i
   if (reinterpret_cast<uintptr_t>(cos_sin) & 15) return -10;
   return gemm_pair_impl(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, 0, 0, EPI_BF16, nullptr, nullptr, 0, status, stream,
                         cos_sin, seq, d, dh, ctx);
-}
-
-// QKV projection of a serving step (see QkvAppend): C (M x 3 d) bf16.  d a multiple of 64, dh of 32.  -13: the TMA-store epilogue it needs
-// is switched off or C does not suit it.
-extern "C" int b200_gemm_bf16_pair_append(const void* A, const void* B, void* C, int M, int K, long long lda, long long ldb, long long ldc,
-                                          const QkvAppend* append, uint32_t* status, cudaStream_t stream) {
-  if (append == nullptr || !qkv_append_ok(*append) || append->d % 64 || append->dh % 32) return -12;
-  return gemm_pair_impl(A, B, C, nullptr, M, 3 * append->d, K, lda, ldb, ldc, 0, 0, 0, EPI_BF16, nullptr, nullptr, 0, status, stream, nullptr, 0,
-                        0, 0, 0, 0, nullptr, 0, nullptr, nullptr, 1, nullptr, append);
 }
 
 // Merged gate|up projection with SwiGLU in the epilogue: C (M x 2F) = A * B^T (gate columns, then up columns) and

@@ -27,8 +27,6 @@ def _lib():
         lib.b200_rope_kv_append.restype = I
         lib.b200_gemm_bf16_append.argtypes = [P, P, P, I, I, L, L, L, I, P, P, P]
         lib.b200_gemm_bf16_append.restype = I
-        lib.b200_gemm_bf16_pair_append.argtypes = [P, P, P, I, I, L, L, L, P, P, P]
-        lib.b200_gemm_bf16_pair_append.restype = I
         _declared = True
     return lib
 
@@ -80,14 +78,22 @@ class QkvAppend(ctypes.Structure):
                 ("v_cache", ctypes.c_void_p), ("num_slots", ctypes.c_longlong), ("d", ctypes.c_int), ("dh", ctypes.c_int), ("ctx", ctypes.c_int)]
 
 
+# Rows x width x width up to which a layer takes the device less time than its launches take the host (about 100 us): there a launch less is
+# worth more than the time that rotating and appending takes a product's epilogue, whose rows lie scattered (rows x width, us a launch, fused and as
+# three launches: 256 x 768 7.5, 8.6; 512 x 2048 27.7, 20.3; 2048 x 1024 25.0, 22.4).  Whole prompts, us, three launches -> fused: 256 x 2048
+# 2831 -> 2693, 1536 x 1024 1686 -> 1619, 4096 x 512 963 -> 937; beyond the limit 512 x 2048 3163 -> 3278, 4096 x 768 2002 -> 2138,
+# 8192 x 2048 18230 -> 20200.  Captured decode steps, all within the limit: 16 x 2048 1833 -> 1765, 128 x 768 869 -> 860, 256 x 2048 4739 -> 4746.
+APPEND_MAX_WORK = 1.6e9
+
+
 def qkv_rope_append(h, wqkv, cos_sin, positions, k_cache, v_cache, slot_mapping, n_heads: int):
-    """qkv = h (R, d) @ wqkv (3 d, d)^T, then what ``rope_kv_append`` does with it, in the product's epilogue where the heads are made of its
-    chunks of columns and its contraction is not cut in slices.  The same values either way."""
+    """qkv = h (R, d) @ wqkv (3 d, d)^T, then what ``rope_kv_append`` does with it, in the product's epilogue where the step is short
+    (``APPEND_MAX_WORK``), the heads are made of its chunks of columns and its contraction is not cut in slices.  The same values either way."""
     r, k = h.shape
     d = wqkv.shape[0] // 3
     dh = d // n_heads
     sliced = native.USE_SPLITK and r <= native.SPLITK_MAX_M and k >= native.SPLITK_MIN_K
-    if h.is_cuda and dh % 32 == 0 and d % 64 == 0 and not sliced:
+    if h.is_cuda and r * k * d <= APPEND_MAX_WORK and dh % 32 == 0 and d % 64 == 0 and not sliced:
         native._req(h.dtype == torch.bfloat16 and wqkv.dtype == torch.bfloat16 and h.stride(1) == 1 and wqkv.stride(1) == 1
                     and wqkv.shape[1] == k and dh * n_heads == d, "bad projection")
         native._req(slot_mapping.dtype == torch.int64 and slot_mapping.numel() == r and slot_mapping.is_contiguous()
@@ -99,11 +105,8 @@ def qkv_rope_append(h, wqkv, cos_sin, positions, k_cache, v_cache, slot_mapping,
         out = torch.empty((r, 3 * d), dtype=torch.bfloat16, device=h.device)
         what = QkvAppend(cos_sin.data_ptr(), positions.data_ptr(), slot_mapping.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                          k_cache.shape[0] * k_cache.shape[1], d, dh, cos_sin.shape[1])
-        args = (h.data_ptr(), wqkv.data_ptr(), out.data_ptr(), r, k, h.stride(0), wqkv.stride(0), 3 * d)
-        tail = (ctypes.byref(what), native.status_word(h.device).data_ptr(), native._stream())
-        rc = _lib().b200_gemm_bf16_pair_append(*args, *tail) if native.USE_PAIR and r >= native.PAIR_MIN_M else -13
-        if rc == -13:                      # a small step, or the epilogue that the CTA pairs need is switched off
-            rc = _lib().b200_gemm_bf16_append(*args, native.EPI_B_STABLE, *tail)
+        rc = _lib().b200_gemm_bf16_append(h.data_ptr(), wqkv.data_ptr(), out.data_ptr(), r, k, h.stride(0), wqkv.stride(0), 3 * d,
+                                          native.EPI_B_STABLE, ctypes.byref(what), native.status_word(h.device).data_ptr(), native._stream())
         native._check(rc, "gemm_bf16_append")
         return out
     from . import gemm

@@ -160,11 +160,13 @@ def test_rope_kv_append_equals_the_two_separate_kernels(heads, dh):
     assert float(kc.view(-1, d)[slots[5]].abs().sum()) == 0.0
 
 
-@pytest.mark.parametrize("rows", [1, 7, 33, 64, 65, 1024, 1030])
-@pytest.mark.parametrize("heads,dh", [(16, 128), (12, 64), (2, 32), (3, 40)])
-def test_qkv_projection_that_rotates_and_appends(rows, heads, dh):
-    """Against the three steps one after the other; rows without a slot, and a slot beyond the cache, which is reported."""
+@pytest.mark.parametrize("rows", [1, 7, 33, 64, 65, 1024, 1030, 129, 200, 256, 257, 1023])
+@pytest.mark.parametrize("heads,dh", [(16, 128), (12, 64), (2, 32), (3, 40), (32, 128)])
+def test_qkv_projection_that_rotates_and_appends(rows, heads, dh, monkeypatch):
+    """Against the three steps one after the other, whichever the rule on rows and widths would take: rows of one and two short tiles and of whole
+    ones, contractions that are sliced (4096 columns, up to 256 rows); rows without a slot, and a slot beyond the cache, which is reported."""
     from llm_systems_from_scratch_b200.ops import native, serving_ops
+    monkeypatch.setattr(serving_ops, "APPEND_MAX_WORK", float("inf"))
     d, ctx, pages, page = heads * dh, 300, 70, 16
     g = torch.Generator("cuda").manual_seed(rows)
     rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
@@ -236,3 +238,17 @@ def test_decode_steps_of_any_size_round_gate_and_up(rows, monkeypatch):
     want, expected = steps()
     native.check_status()
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and tokens == expected
+
+
+@pytest.mark.parametrize("rows,width,fused", [(1, 2048, True), (256, 2048, True), (381, 2048, True), (382, 2048, False), (512, 2048, False),
+                                              (8192, 2048, False), (1525, 1024, True), (1526, 1024, False), (300, 4096, False)])
+def test_long_steps_leave_rotation_and_append_to_a_launch_of_their_own(rows, width, fused, monkeypatch):
+    """Rotating and appending in the product's epilogue takes the device longer than a pass of its own (512 rows of 2048 columns 27.7 us, 20.3)."""
+    from llm_systems_from_scratch_b200.ops import serving_ops
+    apart = []
+    monkeypatch.setattr(serving_ops, "rope_kv_append", lambda *a: apart.append(len(a)))
+    h, w = (torch.randn(n, width, device="cuda").bfloat16() for n in (rows, 3 * width))
+    cache = torch.zeros(1, 16, width, device="cuda", dtype=torch.bfloat16)
+    serving_ops.qkv_rope_append(h, w, torch.ones(2, 4, 32, device="cuda"), torch.zeros(rows, device="cuda", dtype=torch.int32), cache, cache.clone(),
+                                torch.full((rows,), -1, device="cuda"), width // 64)
+    assert bool(apart) != fused

@@ -149,10 +149,15 @@ def has(symbol: str) -> bool:
     return lib is not None and hasattr(lib, symbol)
 
 
+_RAW_STREAM, _DEVICE = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
     """The current stream of the current device.  ``torch.cuda.current_stream`` makes a stream object of it, 4 us of the 18 a launch takes
-    on the host."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    on the host; it is asked where this torch does not tell the handle alone."""
+    if _RAW_STREAM is None or _DEVICE is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _RAW_STREAM(_DEVICE())
 
 
 def _ptr(t) -> int:

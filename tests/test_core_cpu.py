@@ -253,6 +253,19 @@ def test_split_k_plan_for_decode_shapes():
     assert native.splitk_plan(128, 50264, 2048)[1] == 1
 
 
+def test_stream_handle_of_a_torch_without_the_raw_call(monkeypatch):
+    from types import SimpleNamespace
+    from llm_systems_from_scratch_b200.ops import native
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=77))
+    for name in ("_RAW_STREAM", "_DEVICE"):
+        with monkeypatch.context() as at:
+            at.setattr(native, "_RAW_STREAM", lambda device: 100 + device)
+            at.setattr(native, "_DEVICE", lambda: 3)
+            assert native._stream() == 103
+            at.setattr(native, name, None)
+            assert native._stream() == 77
+
+
 def test_slicing_switches_govern_the_kernel_for_few_rows(monkeypatch):
     """One threshold for all sliced products: raising it turns the kernel for few rows off as well.  Lowering it leaves short contractions to
     the general kernel's slices, and 0 rows switches the kernel off."""

@@ -729,6 +729,18 @@ extern "C" int b200_gemm_set_tma_store(int on) {
   return old;
 }
 
+// SMs of the current device, asked once; a B200's where there is none (plans made on a machine without a GPU).
+static int pair_sms() {
+  static int known = 0;
+  int dev = 0;
+  if (known == 0 && (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&known, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)) {
+    cudaGetLastError();
+    known = 0;
+    return 148;
+  }
+  return known;
+}
+
 // Same contract as b200_gemm_bf16 (gemm_tcgen05.cu); tiles are 256 x 256 on CTA pairs.
 static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda,
                           long long ldb, long long ldc, long long ldr, int a_mn, int b_mn, int epi,
@@ -801,9 +813,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
       p.tma_store = 1;
   }
   if (C == nullptr && !p.tma_store) return -13;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = pair_sms();
   if (splits > 1 && p.tma_store) {
     const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN), rest = tiles % (sms / 2);
     if (rest > 0 && make_tmap_out_2d(&tmH, true, ws, (uint64_t)rest * splits * 256, P_BN, P_BN, 32, 32) == 0) {
@@ -822,38 +832,42 @@ extern "C" int b200_gemm_bf16_pair(const void* A, const void* B, void* C, const 
   return gemm_pair_impl(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, epi, nullptr, nullptr, 0, status, stream);
 }
 
+constexpr int TAIL_MAX_SLICES = 24;
+static long long tail_floats(int M, int N, int splits) {
+  const int rest = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN) % (pair_sms() / 2);
+  return splits > 1 ? (long long)rest * splits * 256 * P_BN : 0;
+}
+
 // Slices of K for the tiles of the last wave of a launch (1 = leave them whole) and the floats of workspace they need.  The estimate counts
 // k-blocks of 64 (0.27 us on a pair): a wave of slices, a pipeline fill of 8 per unit, and for the second launch 14 and 0.2 per partial tile.
 // Measured, us per weight gradient over 16384 rows, before (on one SM per 128 x 128 tile where that was better) -> now: 512 x 512 46 -> 18,
 // 768 x 2048 59 -> 44, 2304 x 768 58 -> 51, 2048 x 5504 319 -> 289, 6144 x 2048 342 -> 314.
 // cost_out (may be null): the launch's estimate in k-blocks.
 extern "C" long long b200_gemm_pair_tail_plan(int M, int N, int K, int* splits_out, double* cost_out) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  const int pairs = sms / 2, num_kb = (K + BK - 1) / BK;
+  const int pairs = pair_sms() / 2, num_kb = (K + BK - 1) / BK;
   const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN), rest = tiles % pairs;
   double best = rest > 0 ? num_kb + 8 : 0;
   *splits_out = 1;
   if (rest > 0 && N % 4 == 0)
-    for (int s = 2; s <= 24 && s <= num_kb / 4; ++s) {
+    for (int s = 2; s <= TAIL_MAX_SLICES && s <= num_kb / 4; ++s) {
       const int units = rest * s;
       const double cost = ((units + pairs - 1) / pairs) * ((double)num_kb / s + 8) + 14 + 0.2 * units;
       if (cost < 0.95 * best) { best = cost; *splits_out = s; }
     }
   if (cost_out != nullptr) *cost_out = best + (tiles / pairs) * (double)num_kb;
-  return *splits_out > 1 ? (long long)rest * *splits_out * 256 * P_BN : 0;
+  return tail_floats(M, N, *splits_out);
 }
 
-// b200_gemm_bf16_pair (epi 0, 1 or 3) whose last wave is contracted in `splits` slices, as planned above; `ws` (16-byte aligned) belongs to
+// b200_gemm_bf16_pair (epi 0, 1 or 3) whose last wave is contracted in `splits` slices (the plan's, which the caller keeps); `ws` (16-byte aligned) belongs to
 // this launch until it ends.
 extern "C" int b200_gemm_bf16_pair_tail(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                                         long long ldc, int a_mn, int b_mn, int epi, int splits, float* ws, long long ws_floats,
                                         uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (epi != EPI_BF16 && epi != EPI_F32 && epi != EPI_F32_ACC) return -11;
-  int planned = 1;
-  const long long need = b200_gemm_pair_tail_plan(M, N, K, &planned, nullptr);
-  if (splits != planned || (splits > 1 && (ws == nullptr || (reinterpret_cast<uintptr_t>(ws) & 15) || ws_floats < need))) return -12;
+  if (splits < 1 || (splits > 1 && (splits > TAIL_MAX_SLICES || splits > (K + BK - 1) / BK / 4 || N % 4 || ws == nullptr ||
+                                    (reinterpret_cast<uintptr_t>(ws) & 15) || ws_floats < tail_floats(M, N, splits))))
+    return -12;
   return gemm_pair_impl(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, a_mn, b_mn, epi, nullptr, nullptr, 0, status, stream, nullptr, 0, 0, 0,
                         0, 0, nullptr, 0, nullptr, nullptr, splits, ws);
 }
@@ -886,9 +900,7 @@ extern "C" int b200_gemm_bf16_pair_gather(const void* A, const void* B, void* C,
   g.shard_vec = shard_bytes / 16;
   g.world = world; g.rank = rank; g.done = done_counter;
   if (ctas_out != nullptr) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = pair_sms();
     const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN);
     int pairs = sms / 2;
     if (tiles < pairs) pairs = tiles;

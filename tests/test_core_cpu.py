@@ -253,6 +253,20 @@ def test_split_k_plan_for_decode_shapes():
     assert native.splitk_plan(128, 50264, 2048)[1] == 1
 
 
+def test_sliced_last_wave_refuses_what_its_workspace_does_not_hold():
+    """Argument checks of the entry, before anything is launched: 176 tiles leave 28 on 74 pairs, each with a partial tile of 256 x 256 per slice."""
+    from llm_systems_from_scratch_b200.ops import native
+    if native.load(required=False) is None:
+        pytest.skip("kernel library not built")
+    lib, at = native.load(), 1 << 20
+    m, n, k = 2048, 5504, 16384
+    slices, floats, _ = native.pair_tail_plan(m, n, k)
+    assert slices > 1 and floats == 28 * slices * 65536
+    call = lambda s, ws, have, n=n, k=k: lib.b200_gemm_bf16_pair_tail(at, at, at, m, n, k, m, n, n, 1, 1, 1, s, ws, have, None, None)
+    assert [call(slices, at, floats - 1), call(slices, at + 4, floats), call(slices, None, floats), call(0, at, floats), call(25, at, 1 << 40),
+            call(slices + 1, at, floats), call(4, at, 1 << 40, k=960), call(2, at, 1 << 40, n=5502)] == [-12] * 8
+
+
 def test_stream_handle_of_a_torch_without_the_raw_call(monkeypatch):
     from types import SimpleNamespace
     from llm_systems_from_scratch_b200.ops import native

@@ -978,8 +978,8 @@ using namespace b200;
 namespace b200 {
 int g_pdl_enabled = 0;
 }
-// 1 = kernels of the decode path (norm, GEMM, rotary embedding, KV append, paged attention, SiLU, embedding, argmax)
-// are launched as programmatic dependents of the kernel before them; returns the previous setting.
+// 1 = kernels of training and serving steps (all that are launched through launch_dep) are programmatic dependents of the kernel before
+// them; returns the previous setting.
 extern "C" int b200_set_pdl(int on) {
   const int old = b200::g_pdl_enabled;
   b200::g_pdl_enabled = on ? 1 : 0;

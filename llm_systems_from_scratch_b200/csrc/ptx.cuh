@@ -321,7 +321,8 @@ __device__ __forceinline__ void pdl_sync() {
 }
 // Who lets the next kernel in early also shares its SMs' memory with it: beside a kernel with 200 KB of shared memory an SM has almost no
 // L1, where loads in flight are held, and keeps that division until it is empty.  A product in front of a kernel that streams from memory
-// therefore waits without letting it in (decode attention of 20 requests behind the QKV projection: 8.5 us a layer).
+// therefore waits without letting it in (decode attention behind the QKV projection, 24 layers, us, let in -> not: one request 1605 -> 1618,
+// eight 2528 -> 2303, 20 3067 -> 3064, 64 5030 -> 4963, 128 7196 -> 7076).
 
 extern int g_pdl_enabled;   // host switch (b200_set_pdl); defined in elementwise.cu
 

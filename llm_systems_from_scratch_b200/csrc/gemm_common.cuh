@@ -114,7 +114,7 @@ struct GemmParams {
   // B (the weights) does not depend on the kernel before this one: as a programmatic dependent the kernel requests
   // its first B tiles before it waits for that kernel, so the weights' DRAM latency overlaps the predecessor's tail.
   int b_early;
-  // Several problems in one launch (single-CTA kernel, K-major operands):
+  // Several problems in one launch (K-major operands; by columns: single-CTA kernel only):
   //   by rows    (`tile_group`): 128-row tile m multiplies with rows [group * group_rows, ...) of B, group = tile_group[m]
   //              (a mixture of experts whose tokens are sorted by expert); a negative group skips the tile
   //   by columns (`batch` > 1): problem g reads A columns from g * a_step, B rows from g * group_rows and writes C (and
@@ -133,14 +133,17 @@ struct GemmParams {
   uint32_t* tile_counters;    // four per tile (one per 32-row quarter), zero between launches (the last warp resets its own)
 };
 
-__device__ __forceinline__ void tile_coords(int tile, const GemmParams& p, int& m_blk, int& n_blk) {
+__device__ __forceinline__ void tile_coords(int tile, const GemmParams& p, int num_m_tiles, int& m_blk, int& n_blk) {
   const int per_group = p.group_m * p.num_n_tiles;
   const int g = tile / per_group;
   const int first_m = g * p.group_m;
-  const int gm = min(p.group_m, p.num_m_tiles - first_m);
+  const int gm = min(p.group_m, num_m_tiles - first_m);
   const int r = tile - g * per_group;
   m_blk = first_m + r % gm;
   n_blk = r / gm;
+}
+__device__ __forceinline__ void tile_coords(int tile, const GemmParams& p, int& m_blk, int& n_blk) {
+  tile_coords(tile, p, p.num_m_tiles, m_blk, n_blk);
 }
 
 __device__ __forceinline__ void report(const GemmParams& p, volatile uint32_t* abort_word, uint32_t code) {

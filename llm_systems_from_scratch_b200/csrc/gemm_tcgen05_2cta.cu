@@ -12,6 +12,10 @@
 //   tmem_empty[a]  lives in the leader; the 2 x 128 epilogue threads of the pair arrive on it
 // TMA loads are ordinary (non-multicast) loads.  Every wait is bounded (see ptx.cuh).
 //
+// Grouped rows (experts' products of prompts): a pair takes two neighbouring 128-row tiles of the same group, the 256 columns as above.  Single
+// CTAs are held up by their shared memory as described; a prompt of 8192 rows, top 2 of 8 experts of 2752 x 2048: 1175 -> 1330 TFLOP/s in
+// the step.  What it cannot use is the second half of a group's last pair (4 of 68 on average there).
+//
 // Last wave (weight gradients): with T tiles on P pairs, the T % P tiles of the last wave are contracted in `splits` slices of K each, on all
 // pairs; the partial tiles go to a workspace and pair_tail_sum_kernel adds them in slice order (no atomics: reproducible).
 #include "gemm_common.cuh"
@@ -41,7 +45,10 @@ constexpr int P_SLAB = 32 * 128;
 constexpr int P_STAGING = 4 * 2 * P_SLAB;   // 32 KB
 constexpr int P_BARS = 2 * P_STAGES + 4;
 constexpr int P_SMEM = P_DATA + P_STAGING + P_BARS * 8 + 16 + 160 + 1024;   // 160: ReduceSmem of the copy warps
-static_assert(P_SMEM <= 232448, "shared memory budget of one CTA");
+// Grouped launches: up to P_LIST pairs of row tiles, two bytes each, and their number.
+constexpr int P_LIST = 800;
+constexpr int P_SMEM_GROUPED = P_SMEM + P_LIST * 2 + 16;
+static_assert(P_SMEM_GROUPED <= 232448, "shared memory budget of one CTA");
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -105,7 +112,35 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
       : "memory");
 }
 
-template <bool A_MN, bool B_MN>
+// The row tiles that one pair works on together: two neighbours of the same group, or (P_ALONE) the last one of a group with an odd number of
+// them, which both CTAs then load and one stores.  Called by one warp; entries go to `list`, their number is returned.
+constexpr uint32_t P_ALONE = 0x8000;
+__device__ __forceinline__ int list_pairs(const int* __restrict__ tile_group, int tiles, uint16_t* list) {
+  const int lane = threadIdx.x & 31;
+  int count = 0, run = 0, before = -1;      // first tile of the current run; group of the tile in front
+  for (int t0 = 0; t0 < tiles; t0 += 32) {
+    const int t = t0 + lane;
+    const int g = t < tiles ? tile_group[t] : -1, next = t + 1 < tiles ? tile_group[t + 1] : -1;
+    int prev = __shfl_up_sync(0xffffffffu, g, 1);
+    if (lane == 0) prev = before;
+    int start = g != prev ? t : lane == 0 ? run : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int other = __shfl_up_sync(0xffffffffu, start, o);
+      if (lane >= o) start = max(start, other);
+    }
+    const bool first = g >= 0 && ((t - start) & 1) == 0;
+    const uint32_t those = __ballot_sync(0xffffffffu, first);
+    if (first) list[count + __popc(those & ((1u << lane) - 1u))] = (uint16_t)(t | (next != g ? P_ALONE : 0u));
+    count += __popc(those);
+    run = __shfl_sync(0xffffffffu, start, 31);
+    before = __shfl_sync(0xffffffffu, g, 31);
+  }
+  return count;
+}
+
+// GROUPED: the 128-row tiles of A belong to the groups of rows of B in p.tile_group (negative: skipped); see list_pairs.
+template <bool A_MN, bool B_MN, bool GROUPED = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmH,
@@ -158,7 +193,26 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   pdl_wait();
   const uint32_t tmem_base = *tmem_holder;
 
-  const int num_tiles = p.num_m_tiles * p.num_n_tiles;   // tiles of 256 x 256
+  int num_m_tiles = p.num_m_tiles;
+  uint16_t* pair_list = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(tmem_holder) + 176);
+  int* pair_count = reinterpret_cast<int*>(pair_list + P_LIST);
+  if (GROUPED) {
+    if (warp == 2) {
+      const int n = list_pairs(p.tile_group, p.M / BM, pair_list);
+      if (lane == 0) *pair_count = n;
+    }
+    __syncthreads();
+    num_m_tiles = *pair_count;
+  }
+  // first row of this CTA's row tile of a unit, and whether it stores its rows
+  auto tile_row = [&](int m_blk, bool& stored) {
+    stored = true;
+    if (!GROUPED) return m_blk * 256 + (int)rank * BM;
+    const uint32_t e = pair_list[m_blk];
+    stored = rank == 0 || !(e & P_ALONE);
+    return (int)((e & (P_ALONE - 1)) + (stored ? rank : 0)) * BM;
+  };
+  const int num_tiles = num_m_tiles * p.num_n_tiles;   // tiles of 256 x 256
   const int num_kb = (p.K + BK - 1) / BK;
   // work unit: a whole tile, or behind the first full_tiles of them a slice of K of a tile (`part`: which partial tile it leaves, else -1)
   const int full_tiles = p.splits > 1 ? p.full_tiles : num_tiles;
@@ -195,10 +249,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       for (int unit = pair; unit < num_units && ok; unit += num_pairs) {
         int m_blk, n_blk, kb_lo, kb_hi, part;
-        tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, m_blk, n_blk);
-        const int m0 = m_blk * 256 + (int)rank * BM;
+        tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, num_m_tiles, m_blk, n_blk);
+        bool stored;
+        const int m0 = tile_row(m_blk, stored);
         // SwiGLU mode: the leader loads 128 gate rows, its peer the matching 128 up rows (F rows further down)
-        const int n0 = p.swiglu_f > 0 ? n_blk * P_HALF + (int)rank * p.swiglu_f : n_blk * P_BN + (int)rank * P_HALF;
+        int n0 = p.swiglu_f > 0 ? n_blk * P_HALF + (int)rank * p.swiglu_f : n_blk * P_BN + (int)rank * P_HALF;
+        if (GROUPED) n0 += __ldg(p.tile_group + m0 / BM) * p.group_rows;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) {
             report(p, abort_word, ERR_WAIT_EMPTY);
@@ -333,7 +389,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     bool ok = true;
     for (int unit = pair; unit < num_units && ok; unit += num_pairs, ++local) {
       int m_blk, n_blk, kb_lo, kb_hi, part;
-      tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, m_blk, n_blk);
+      tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, num_m_tiles, m_blk, n_blk);
       const int acc = local & 1;
       if (!mbar_wait(&tmem_full[acc], acc_phase[acc], abort_word)) {
         if (lane == 0) report(p, abort_word, ERR_WAIT_TMEM_FULL);
@@ -342,14 +398,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       acc_phase[acc] ^= 1;
       tc_fence_after();
-      const int row = m_blk * 256 + (int)rank * BM + quarter * 32 + lane;
+      bool stored;
+      const int row0 = tile_row(m_blk, stored) + quarter * 32;
+      const int row = stored ? row0 + lane : p.M;
       const int n0 = n_blk * P_BN;
       const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc * P_BN;
       // registers -> swizzled slab in shared memory -> TMA store (or TMA add).  Row `lane` of a slab is one 128-byte
       // line; its 16-byte pieces are permuted by (row & 7) as the 128-byte swizzle of the tensor maps expects, which
       // also makes the st.shared.v4 of a quarter warp conflict-free.  A warp alternates between its two slabs and
       // waits, before refilling one, until the store that last used it has read it.
-      const int row0 = m_blk * 256 + (int)rank * BM + quarter * 32;
       const int y0 = part < 0 ? row0 : part * 256 + (int)rank * BM + quarter * 32;      // row of the output or of the workspace
       auto emit = [&](const CUtensorMap* tm, int x, const uint32_t (&o)[32], bool add) {
         uint8_t* slab = smem_out + ((warp - 2) * 2 + (out_slab & 1)) * P_SLAB;
@@ -363,7 +420,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (row0 < p.M) {
+          if (row0 < p.M && stored) {
             if (add) tma_reduce_add_2d(tm, slab, x, y0);
             else tma_store_2d(tm, slab, x, y0);
           }
@@ -678,23 +735,24 @@ pair_tail_sum_kernel(const float4* __restrict__ ws, OUT* __restrict__ C, const G
   }
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool GROUPED = false>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmH,
                        GemmParams p, int sms, cudaStream_t stream) {
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN>;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, GROUPED>;
+  constexpr int SMEM = GROUPED ? P_SMEM_GROUPED : P_SMEM;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -3;
     configured = true;
   }
   p.num_m_tiles = (p.M + 255) / 256;
   p.num_n_tiles = p.swiglu_f > 0 ? (p.swiglu_f + P_HALF - 1) / P_HALF : (p.N + P_BN - 1) / P_BN;
   p.group_m = 8;
-  const int tiles = p.num_m_tiles * p.num_n_tiles;
+  const int tiles = (GROUPED ? 2 : 1) * p.num_m_tiles * p.num_n_tiles;      // grouped: up to one pair per row tile
   int pairs = sms / 2;
   const int units = p.splits > 1 ? p.full_tiles + (tiles - p.full_tiles) * p.splits : tiles;
   if (units < pairs) pairs = units;
-  launch_dep(kern, pairs * 2, P_THREADS, P_SMEM, stream, tmA, tmB, tmC, tmH, p);
+  launch_dep(kern, pairs * 2, P_THREADS, SMEM, stream, tmA, tmB, tmC, tmH, p);
   if (p.splits > 1) {
     const unsigned grid = (unsigned)(tiles - p.full_tiles) * 32;
     if (p.epi == EPI_BF16) launch_dep(pair_tail_sum_kernel<__nv_bfloat16>, grid, 256, 0, stream, (const float4*)p.ws, (__nv_bfloat16*)p.C, p);
@@ -748,7 +806,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
                           uint32_t* status, cudaStream_t stream, const float* rope_cs = nullptr, int rope_seq = 0,
                           int rope_d = 0, int rope_dh = 0, int rope_ctx = 0, int swiglu_f = 0, void* H = nullptr,
                           long long ldh = 0, const ReduceTask* reduce = nullptr, const GemmFinish* finish = nullptr, int splits = 1,
-                          float* ws = nullptr) {
+                          float* ws = nullptr, const int* tile_group = nullptr, int n_groups = 1) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return -10;
@@ -763,7 +821,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
                 : make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 64, BM);
   if (rc) return -20 + rc;
   rc = b_mn ? make_tmap_bf16_2d(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, 64)
-            : make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, P_HALF);
+            : make_tmap_bf16_2d(&tmB, B, (uint64_t)N * n_groups, (uint64_t)K, (uint64_t)ldb, 64, P_HALF);
   if (rc) return -30 + rc;
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
@@ -777,6 +835,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   p.finished = finish != nullptr;
   if (finish != nullptr) p.finish = *finish;
   p.append.cs = nullptr;
+  p.tile_group = tile_group; p.group_rows = N;
   p.wait_counter = wait_counter; p.wait_value = wait_value; p.wait_limit_ns = g_counter_wait_limit_ns;
   p.rope_cs = rope_cs; p.rope_seq = rope_seq; p.rope_d = rope_d; p.rope_dh = rope_dh; p.rope_ctx = rope_ctx;
   p.swiglu_f = swiglu_f; p.H = H; p.ldh = ldh;
@@ -814,6 +873,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   }
   if (C == nullptr && !p.tma_store) return -13;
   const int sms = pair_sms();
+  if (tile_group != nullptr) return p.tma_store ? launch_pair<false, false, true>(tmA, tmB, tmC, tmH, p, sms, stream) : -13;
   if (splits > 1 && p.tma_store) {
     const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN), rest = tiles % (sms / 2);
     if (rest > 0 && make_tmap_out_2d(&tmH, true, ws, (uint64_t)rest * splits * 256, P_BN, P_BN, 32, 32) == 0) {
@@ -943,6 +1003,22 @@ extern "C" int b200_gemm_bf16_pair_swiglu(const void* A, const void* B, void* C,
   }
   return gemm_pair_impl(A, B, C, nullptr, M, 2 * F, K, lda, ldb, ldc, 0, 0, 0, EPI_BF16, carry ? &g : nullptr, nullptr, 0,
                         status, stream, nullptr, 0, 0, 0, 0, F, H, ldh);
+}
+
+// Grouped product on CTA pairs (see b200_gemm_bf16_grouped with `tile_group`; bf16 output): the same values, for the many rows of a prompt.
+// gate: silu(gate) * up of groups of 2 N rows, N a multiple of 64.  -13: an output that TMA stores do not reach, -14: too many row tiles
+// (the caller then takes the other kernel).
+extern "C" int b200_gemm_bf16_pair_grouped(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                                           long long ldc, const int* tile_group, int n_groups, int gate, const GemmFinish* finish,
+                                           uint32_t* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M % BM || n_groups <= 0 || tile_group == nullptr || (gate && (finish != nullptr || N % 64))) return -12;
+  if (M / BM > P_LIST) return -14;
+  if (gate)
+    return gemm_pair_impl(A, B, nullptr, nullptr, M, 2 * N, K, lda, ldb, 0, 0, 0, 0, EPI_BF16, nullptr, nullptr, 0, status, stream, nullptr,
+                          0, 0, 0, 0, N, C, ldc, nullptr, nullptr, 1, nullptr, tile_group, n_groups);
+  return gemm_pair_impl(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, 0, 0, EPI_BF16, nullptr, nullptr, 0, status, stream, nullptr, 0, 0, 0,
+                        0, 0, nullptr, 0, nullptr, finish, 1, nullptr, tile_group, n_groups);
 }
 
 int b200_make_reduce_task(const B200ReduceDesc* d, uint32_t* status, bool carried, ReduceTask* out);

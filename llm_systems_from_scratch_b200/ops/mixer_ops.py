@@ -16,6 +16,12 @@ from . import mixer_torch, native
 from .native import _check, _ptr, _req, _stream
 
 TILE = 128                 # rows of an expert tile (csrc/mixer_elementwise.cu: PLAN_TILE)
+# Rows of the buffer per group from which a grouped product runs on CTA pairs (gated, plain): below, there are too few tiles for all pairs and
+# more pairs that work for one tile.  Eight groups, us on single CTAs -> pairs, gated and plain, 2 x 2752 x 2048 and 2048 x 2752: 160 rows
+# 41 -> 45, 24 -> 23; 256 56 -> 46, 26 -> 24; 512 80 -> 71, 43 -> 39; 1152 168 -> 144, 83 -> 74; 2176 289 -> 256, 155 -> 171 alone, but the prompt
+# step with both on pairs is the faster one (22.8 ms; gated 22.4; both 21.8).  2 x 1344 x 768 and 768 x 1344: 192 23 -> 23, 12 -> 21; 256
+# 29 -> 23, 14 -> 22; 384 37 -> 16, 10 -> 14; 512 32 -> 20, 14 -> 14; 1616 73 -> 45, 32 -> 23.
+PAIR_GROUP_ROWS = (256, 512)
 _declared = False
 
 
@@ -33,6 +39,7 @@ def _lib():
             "b200_gate_sigmoid": [P, P, L, I, I, L, L, I, P],
             "b200_gemm_f32": [P, P, P, I, I, I, L, L, L, I, P, I, I, I, I, P, P],
             "b200_gemm_bf16_grouped": [P, P, P, P, I, I, I, L, L, L, L, P, I, I, I, I, I, I, I, I, P, P, P],
+            "b200_gemm_bf16_pair_grouped": [P, P, P, I, I, I, L, L, L, P, I, I, P, P, P],
             "b200_moe_route": [P, L, P, P, P, P, P, P, P, I, I, I, I, I, P],
             "b200_moe_route_rows": [P, L, P, L, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
             "b200_moe_dispatch": [P, L, P, L, P, P, P, P, P, I, I, I, I, I, I, I, P],
@@ -138,6 +145,13 @@ def gemm_rows(a, w, tile_group, n: int, swiglu: bool, act: str | None = None):
     finish = _finish(None, 1.0, act, 0.0)
     if a.dtype == torch.bfloat16:
         out = rows_buffer(p, n, a.dtype, a.device)
+        if native.USE_PAIR and p >= PAIR_GROUP_ROWS[not swiglu] * (w.shape[0] // rows) and not (swiglu and n % 64):
+            rc = lib.b200_gemm_bf16_pair_grouped(_ptr(a), _ptr(w), _ptr(out), p, n, k, a.stride(0), w.stride(0), out.stride(0),
+                                                 _ptr(tile_group), w.shape[0] // rows, int(swiglu), _ref(finish),
+                                                 _ptr(native.status_word(a.device)), _stream())
+            if rc not in (-13, -14):           # an output for plain stores, or more tiles than the kernel lists
+                _check(rc, "gemm_pair_grouped")
+                return out
         _check(lib.b200_gemm_bf16_grouped(_ptr(a), _ptr(w), _ptr(out), None, p, n, k, a.stride(0), w.stride(0), out.stride(0),
                                           0, _ptr(tile_group), w.shape[0] // rows, rows, 1, 0, 0, int(swiglu), 0, 0, _ref(finish),
                                           _ptr(native.status_word(a.device)), _stream()), "gemm_grouped")

@@ -434,3 +434,46 @@ def test_gated_product_on_cta_pairs_with_half_a_tile_left(m, f, k):
         # h is made of gate and up rounded to bf16: three roundings
         assert off(gu, want_gu) < 2.0 ** -8 and off(h, want) < 3 * 2.0 ** -8
     native.check_status()
+
+
+@pytest.mark.parametrize("tiles", [[1], [2], [0, 3, 0, 1], [5, 4, 2, 1], [31, 2, 33], [1] * 40, [-2, 3, -1, 2]])
+@pytest.mark.parametrize("n,k,act", [(64, 64, "silu"), (192, 136, "silu"), (1344, 512, "silu"), (8, 64, None), (200, 136, None), (768, 1344, "gelu")])
+def test_grouped_products_on_cta_pairs(tiles, n, k, act, monkeypatch):
+    """Groups of odd and even numbers of row tiles, none, and skipped tiles (negative counts): the single-CTA kernel's results bit for bit, and
+    nothing outside the tiles that belong to a group."""
+    from llm_systems_from_scratch_b200.ops import mixer_ops as mo, native
+    groups = len(tiles)
+    of = [e if t > 0 else -1 for e, t in enumerate(tiles) for _ in range(abs(t))] + [-1, -1]
+    tile_group = torch.tensor(of, dtype=torch.int32, device="cuda")
+    g = torch.Generator("cuda").manual_seed(n)
+    gated = act == "silu"
+    x = torch.randn(len(of) * 128, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(groups * n * (2 if gated else 1), k, generator=g, device="cuda") / k ** 0.5).bfloat16()
+    made = []
+
+    def rows_buffer(rows, cols, dtype, device):
+        made.append(torch.full((rows, cols), 7.0, dtype=dtype, device=device))
+        return made[-1]
+    monkeypatch.setattr(mo, "rows_buffer", rows_buffer)
+    out = []
+    for least in (0, 1 << 30):
+        monkeypatch.setattr(mo, "PAIR_GROUP_ROWS", (least, least))
+        out.append(mo.gemm_rows(x, w, tile_group, n, gated, None if gated else act))
+    assert torch.equal(out[0], out[1])
+    mine = torch.tensor([e >= 0 for e in of], device="cuda").repeat_interleave(128)
+    assert bool((out[0][~mine] == 7.0).all()) and (not mine.any() or bool((out[0][mine] != 7.0).any()))
+    native.check_status()
+
+
+def test_more_row_tiles_than_a_pair_lists(monkeypatch):
+    """Beyond 800 row tiles the grouped product stays on single CTAs; 800 are still listed."""
+    from llm_systems_from_scratch_b200.ops import mixer_ops as mo, native
+    w = torch.randn(2 * 64, 64, device="cuda").bfloat16()
+    for count in (800, 801):
+        x = torch.randn(count * 128, 64, device="cuda").bfloat16()
+        tile_group = (torch.arange(count, device="cuda") >= count - 3).int()
+        got = mo.gemm_rows(x, w, tile_group, 64, False)
+        with monkeypatch.context() as at:
+            at.setattr(mo, "PAIR_GROUP_ROWS", (1 << 30, 1 << 30))
+            assert torch.equal(got, mo.gemm_rows(x, w, tile_group, 64, False))
+    native.check_status()

@@ -208,6 +208,11 @@ def _check(rc: int, name: str):
     _LAUNCHES += _KERNELS_PER_CALL.get(name, 1)
 
 
+def count_launches(n: int):
+    global _LAUNCHES
+    _LAUNCHES += n
+
+
 def _req(cond: bool, msg: str):
     if not cond:
         raise ValueError(msg)
@@ -269,6 +274,17 @@ def pair_tail_plan(m: int, n: int, k: int) -> tuple[int, int, bool]:
     floats = int(fn(m, n, k, ctypes.byref(splits), ctypes.byref(cost)))
     waves = -(-(-(-m // 128) * -(-n // 128)) // _sms())
     return splits.value, floats, cost.value <= waves * 0.625 * -(-k // 64) + 8
+
+
+def nt_route(m: int, n: int, k: int, device) -> tuple[int, int]:
+    """Kernel of a plain 'nt' product, as ``gemm`` chooses it: (0 single CTAs, 1 CTA pairs, 2 sliced through the workspace, 3 few rows; K slices
+    of the last)."""
+    if USE_PAIR and (FORCE_PAIR or (m >= PAIR_MIN_M and n >= 256 and _pair_pays(m, n))):
+        return 1, 0
+    few = few_rows(m, n, k) if USE_SPLITK else 0
+    if few:
+        return 3, few
+    return (2 if USE_SPLITK and m <= SPLITK_MAX_M and k >= SPLITK_MIN_K and _splitk_scratch(device) is not None else 0), 0
 
 
 def set_gemm_tma_store(on: bool) -> bool:

@@ -27,6 +27,8 @@ def _lib():
         lib.b200_rope_kv_append.restype = I
         lib.b200_gemm_bf16_append.argtypes = [P, P, P, I, I, L, L, L, I, P, P, P]
         lib.b200_gemm_bf16_append.restype = I
+        lib.b200_lm_layers.argtypes = [P, P]
+        lib.b200_lm_layers.restype = I
         _declared = True
     return lib
 
@@ -86,14 +88,18 @@ class QkvAppend(ctypes.Structure):
 APPEND_MAX_WORK = 1.6e9
 
 
+def _appends_in_product(r: int, k: int, d: int, dh: int) -> bool:
+    sliced = native.USE_SPLITK and r <= native.SPLITK_MAX_M and k >= native.SPLITK_MIN_K
+    return r * k * d <= APPEND_MAX_WORK and dh % 32 == 0 and d % 64 == 0 and not sliced
+
+
 def qkv_rope_append(h, wqkv, cos_sin, positions, k_cache, v_cache, slot_mapping, n_heads: int):
     """qkv = h (R, d) @ wqkv (3 d, d)^T, then what ``rope_kv_append`` does with it, in the product's epilogue where the step is short
     (``APPEND_MAX_WORK``), the heads are made of its chunks of columns and its contraction is not cut in slices.  The same values either way."""
     r, k = h.shape
     d = wqkv.shape[0] // 3
     dh = d // n_heads
-    sliced = native.USE_SPLITK and r <= native.SPLITK_MAX_M and k >= native.SPLITK_MIN_K
-    if h.is_cuda and r * k * d <= APPEND_MAX_WORK and dh % 32 == 0 and d % 64 == 0 and not sliced:
+    if h.is_cuda and _appends_in_product(r, k, d, dh):
         native._req(h.dtype == torch.bfloat16 and wqkv.dtype == torch.bfloat16 and h.stride(1) == 1 and wqkv.stride(1) == 1
                     and wqkv.shape[1] == k and dh * n_heads == d, "bad projection")
         native._req(slot_mapping.dtype == torch.int64 and slot_mapping.numel() == r and slot_mapping.is_contiguous()
@@ -170,3 +176,90 @@ def paged_decode_attention(qkv, k_cache, v_cache, block_tables, context_lens, n_
                                         k_cache.shape[0], native.status_word(qkv.device).data_ptr(), native._stream()),
                   "paged_decode")
     return out
+
+
+# ------------------------------------------------------------------------------------------------------- all layers of a step
+class LmProduct(ctypes.Structure):
+    """csrc/lm_layers.cu: LmProduct."""
+    _fields_ = [("kind", ctypes.c_int), ("slices", ctypes.c_int)]
+
+
+class LmLayer(ctypes.Structure):
+    """csrc/lm_layers.cu: LmLayer."""
+    _fields_ = [(n, ctypes.c_void_p) for n in ("wqkv", "wo", "wgu", "wdown", "n1", "n2", "k", "v")]
+
+
+class LmStep(ctypes.Structure):
+    """csrc/lm_layers.cu: LmStep."""
+    _fields_ = [(n, ctypes.c_void_p) for n in ("layers", "x", "y", "h", "qkv", "o", "gu", "act", "rstd", "cos_sin", "positions", "slots", "cu",
+                                               "tables", "ctx_lens", "part_o", "part_ml", "ws", "counters", "status")] + \
+               [(n, ctypes.c_longlong) for n in ("num_slots", "ws_floats")] + \
+               [(n, ctypes.c_int) for n in ("n_layers", "rows", "d", "heads", "ff", "rope_ctx", "batch", "max_seq", "page_size", "max_pages",
+                                            "splits", "num_pages", "n_counters", "append", "glu")] + \
+               [("eps", ctypes.c_float), ("scale", ctypes.c_float)] + [(n, LmProduct) for n in ("pqkv", "po", "pgu", "pdown")]
+
+
+_PAIR, _GROUPED, _ROUNDED = 0, 1, 2          # csrc/lm_layers.cu: LmGlu
+
+
+def transformer_layers(x, layers, n_heads: int, d_ff: int, eps: float, cos_sin, positions, slots, k_cache, v_cache, fused: bool, cu=None,
+                       max_seq: int = 0, tables=None, context_lens=None, splits: int = 0):
+    """All layers of a serving step over the residual stream x (R, d), from one call into the kernel library: what the ops make of it one by one,
+    launch by launch.  ``layers``: ``models.engine.BlockWeights``; caches (layers, pages, page size, d).  Attention among the step's rows
+    (``cu``, ``max_seq``) or through the cache (``tables``, ``context_lens``).  ``fused``: gate and up are multiplied unrounded.
+    Returns x, which then holds the result, or None for what only the single ops take (widths and heads that they pad)."""
+    rows, d = x.shape
+    dh = d // n_heads
+    bf16, dev = torch.bfloat16, x.device
+    if rows == 0 or not layers or d % 8 or d_ff % 8 or dh not in ((32, 64, 128) if cu is not None else (64, 128)) or d > 4096 and cu is None:
+        return None
+    req = native._req
+    req(x.dtype == bf16 and x.is_contiguous() and dh * n_heads == d, "the residual stream must be contiguous bf16")
+    req(positions.dtype == torch.int32 and positions.numel() == rows and positions.is_contiguous()
+        and slots.dtype == torch.int64 and slots.numel() == rows and slots.is_contiguous(), "bad slot mapping or positions")
+    req(k_cache.dtype == bf16 and v_cache.dtype == bf16 and k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.shape == v_cache.shape
+        and k_cache.dim() == 4 and k_cache.shape[0] == len(layers) and k_cache.shape[3] == d, "cache shape does not match")
+    req(cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.shape[0] == 2 and cos_sin.shape[2] == dh // 2, "bad rope cache")
+    shapes = ((3 * d, d), (d, d), (2 * d_ff, d), (d, d_ff), (d,), (d,))
+    table, step = (LmLayer * len(layers))(), k_cache.stride(0) * 2
+    kp, vp = k_cache.data_ptr(), v_cache.data_ptr()
+    for i, w in enumerate(layers):
+        for t, shape in zip(w, shapes):
+            req(t.shape == shape and t.dtype == bf16 and t.is_contiguous() and t.device == dev, "layer weights must be contiguous bf16")
+        table[i] = LmLayer(*[t.data_ptr() for t in w], kp + i * step, vp + i * step)
+    new = lambda *shape, dtype=bf16: torch.empty(shape, dtype=dtype, device=dev)
+    s = LmStep(layers=ctypes.addressof(table), n_layers=len(layers), rows=rows, d=d, heads=n_heads, ff=d_ff, rope_ctx=cos_sin.shape[1], eps=eps,
+               scale=1.0 / math.sqrt(dh), cos_sin=cos_sin.data_ptr(), positions=positions.data_ptr(), slots=slots.data_ptr(),
+               num_slots=k_cache.shape[1] * k_cache.shape[2], page_size=k_cache.shape[2], num_pages=k_cache.shape[1],
+               status=native.status_word(dev).data_ptr())
+    held = [new(rows, d), new(rows, d), new(rows, 3 * d), new(rows, d), new(rows, d_ff), new(rows, dtype=torch.float32)]
+    s.x = x.data_ptr()
+    s.y, s.h, s.qkv, s.o, s.act, s.rstd = (t.data_ptr() for t in held)
+    if cu is not None:
+        req(cu.dtype == torch.int32 and cu.is_cuda and cu.is_contiguous(), "cu_seqlens must be int32 on the device")
+        s.cu, s.batch, s.max_seq = cu.data_ptr(), cu.numel() - 1, max_seq
+    else:
+        req(tables.dtype == torch.int32 and context_lens.dtype == torch.int32 and tables.dim() == 2 and tables.is_contiguous()
+            and tables.shape[0] >= rows and context_lens.is_contiguous() and context_lens.numel() >= rows, "one table row and one length per request")
+        s.tables, s.ctx_lens, s.max_pages = tables.data_ptr(), context_lens.data_ptr(), tables.shape[1]
+        s.splits = splits if splits > 0 else choose_splits(rows, n_heads, s.max_pages * s.page_size, head_dim=dh)
+        held.append(new(rows * n_heads * s.splits * (dh + 2), dtype=torch.float32))
+        s.part_o = held[-1].data_ptr()
+        s.part_ml = s.part_o + rows * n_heads * s.splits * dh * 4
+    route = lambda n, k: LmProduct(*native.nt_route(rows, n, k, dev))
+    s.append = int(_appends_in_product(rows, d, d, dh))
+    s.pqkv, s.po, s.pdown = route(3 * d, d), route(d, d), route(d, d_ff)
+    if fused:
+        s.glu = _PAIR if native.USE_PAIR and rows >= native.PAIR_MIN_M and d_ff % 64 == 0 else _GROUPED
+    else:
+        s.glu, s.pgu = _ROUNDED, route(2 * d_ff, d)
+        held.append(new(rows, 2 * d_ff))
+        s.gu = held[-1].data_ptr()
+    scratch = native._splitk_scratch(dev) if 2 in (s.pqkv.kind, s.po.kind, s.pgu.kind, s.pdown.kind) else None
+    if scratch is not None:
+        ws, counters = scratch
+        s.ws, s.ws_floats, s.counters, s.n_counters = ws.data_ptr(), ws.numel(), counters.data_ptr(), counters.numel()
+    launches = _lib().b200_lm_layers(ctypes.byref(s), native._stream())
+    native._check(min(launches, 0), "lm_layers")
+    native.count_launches(launches - 1)
+    return x

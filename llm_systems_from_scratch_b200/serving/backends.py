@@ -86,6 +86,13 @@ class TransformerBackend:
             return ops.torch_impl.varlen_attention_fwd(qkv, batch.cu, heads)
 
         x = ops.embedding_fwd(batch.tokens, self.head.emb)
+        if x.is_cuda:
+            cfg = self.cfg
+            attention = dict(cu=batch.cu, max_seq=batch.max_portion) if tables is None else dict(tables=tables, context_lens=ctx, splits=batch.splits)
+            done = serving_ops.transformer_layers(x, self.layers, heads, cfg.d_ff, cfg.eps, self.rope, batch.positions, batch.slots, self.cache.k,
+                                                  self.cache.v, batch.n_single != batch.n_rows, **attention)
+            if done is not None:
+                return done
         for li, w in enumerate(self.layers):
             x = self._block(x, w, li, batch, attend)
         return x

@@ -252,3 +252,42 @@ def test_long_steps_leave_rotation_and_append_to_a_launch_of_their_own(rows, wid
     serving_ops.qkv_rope_append(h, w, torch.ones(2, 4, 32, device="cuda"), torch.zeros(rows, device="cuda", dtype=torch.int32), cache, cache.clone(),
                                 torch.full((rows,), -1, device="cuda"), width // 64)
     assert bool(apart) != fused
+
+
+@pytest.mark.parametrize("heads,dh,ff", [(4, 64, 704), (2, 128, 688), (16, 128, 5504)])
+def test_all_layers_from_one_call(heads, dh, ff, monkeypatch):
+    """Prompts (short, and long enough for CTA pairs), a portion that continues beside single tokens, steps of single tokens and a captured
+    step: logits and caches are those of the ops one by one, bit for bit, with as many launches; what only the ops take is left to them."""
+    from llm_systems_from_scratch_b200.models.transformer import TransformerLM
+    from llm_systems_from_scratch_b200.ops import native, serving_ops
+    from llm_systems_from_scratch_b200.serving import ServingEngine
+    torch.manual_seed(0)
+    model = TransformerLM(503, 1088, heads * dh, 2, heads, ff, 10000.0, use_custom_triton=True).cuda().eval()
+    g = torch.Generator().manual_seed(heads)
+    ids = lambda n: torch.randint(0, 503, (n,), generator=g).tolist()
+    lengths = [1, 70, 200, 1030]
+    prompts, more, singles = [ids(n) for n in lengths], ids(40), ids(4)
+    taken = []
+    real = serving_ops.transformer_layers
+
+    def steps():
+        eng = ServingEngine(model, page_size=16, max_batch=8, max_context=1088)
+        native.reset_launch_count()
+        reqs = [eng.open(i) for i in range(4)]
+        logits = [eng.extend([(reqs[i], prompts[i], [lengths[i] - 1])]) for i in range(3)]
+        logits.append(eng.extend([(reqs[3], prompts[3], [0, 1029])]))
+        logits.append(eng.extend([(reqs[1], more, [39]), (reqs[2], [singles[2]], [0])]))
+        logits.append(eng.extend([(r, [t], [0]) for r, t in zip(reqs, singles)]))
+        for r in reqs:
+            r.output, r.prompt = [7], list(range(r.fed))
+            eng.sched.grow(r, r.fed + 2)
+        return logits, eng.decode(reqs), [eng.cache.k.clone(), eng.cache.v.clone()], native.launch_count()
+    monkeypatch.setattr(serving_ops, "transformer_layers", lambda *a, **k: taken.append(real(*a, **k)) or taken[-1])
+    got = steps()
+    assert taken and all(t is not None for t in taken)
+    monkeypatch.setattr(serving_ops, "transformer_layers", lambda *a, **k: None)
+    want = steps()
+    assert all(torch.equal(a, b) for a, b in zip(got[0] + got[2], want[0] + want[2])) and got[1] == want[1] and got[3] == want[3]
+    narrow = torch.zeros(3, heads * 8, dtype=torch.bfloat16, device="cuda")
+    assert real(narrow, [None], heads, ff, 1e-5, None, None, None, None, None, False) is None           # heads of 8 columns
+    native.check_status()

@@ -3,16 +3,15 @@
 // Replaces the library SDPA call of the reference (llm-core/llm_core/model.py:381-382) and its
 // naive masked-softmax path (model.py:308-325).
 //
-// One CTA owns TWO 128-query tiles (A, B) of one (batch, head) and walks the key/value tiles up to the
-// diagonal.  The two tiles take turns on the tensor pipe, so the softmax of one overlaps the MMAs of the other:
-//   warp 0      TMA producer: Q_A, Q_B once, then K_j / V_j into two-stage rings (128B swizzle)
-//   warp 1      MMA issuer:   S_X = Q_X K_j^T (TMEM, 128 fp32 columns per tile)  and  O_X += P_X V_j
-//   warps 2-5   softmax of tile A, warps 6-9 softmax of tile B: one thread per query row, no exchange between
-//               threads.  Two passes over the row in tensor memory (row max, then exp2 / sum / bf16 pack); P is
-//               written back over the S columns it came from (tcgen05.st) and is the A operand of the P V MMA
-//               straight from tensor memory.  O is rescaled in TMEM only when the running max moved by more
-//               than 2^8 (vote per warp).
-// Tensor-pipe order per key tile j: P_A V_j, S_A(j+1), P_B V_j, S_B(j+1).
+// A CTA owns two 128-query tiles (A, B) of one (batch, head), or one (see FwdShape), and walks the key/value tiles up to the diagonal.  The
+// tiles of an SM take turns on the tensor pipe, so the softmax of one overlaps the MMAs of the other:
+//   TMA warp       Q_A, Q_B once, then K_j / V_j into two-stage rings (128B swizzle)
+//   MMA warp       S_X = Q_X K^T (TMEM, 128 fp32 columns per tile)  and  O_X += P_X V
+//   softmax warps  four per tile: one thread per query row, no exchange between threads.  A row's scores of a step are loaded once from tensor
+//                  memory (row max, then exp2 / sum / bf16 pack); P is written back over the S columns it came from (tcgen05.st) and is
+//                  the A operand of the P V MMA straight from tensor memory.  O is rescaled in TMEM only when the running max moved by
+//                  more than 2^8 (vote per warp).
+// Tensor-pipe order per key tile j and query tile X: P_X V_j, S_X(j+1); in steps of 64 keys half by half.
 //
 // WINDOW instances (b200_flash_window_fwd) serve portions of prompts under a sliding window: queries and keys come from
 // separate matrices, a sequence has more keys than queries (the earlier tokens its first queries can still see), tile X
@@ -46,19 +45,6 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   return r;
 }
 
-// 2^x on the FMA and integer pipes (no special-function unit): round x to the nearest integer n with the
-// 1.5 * 2^23 trick, evaluate a cubic on the remainder in [-0.5, 0.5] (relative error 8e-5, far below bf16
-// rounding of the result) and add n to the exponent field.  x must be <= 127; x below -126 gives 2^-126.
-__device__ __forceinline__ float fa_exp2_poly(float x) {
-  x = fmaxf(x, -126.f);
-  const float t = x + 12582912.f;
-  const float f = x - (t - 12582912.f);
-  float pl = fmaf(f, 0.05508868f, 0.24260405f);
-  pl = fmaf(pl, f, 0.69327624f);
-  pl = fmaf(pl, f, 0.99992894f);
-  return __int_as_float(__float_as_int(pl) + (__float_as_int(t) << 23));
-}
-
 // Packed fp32 pairs: one FMA-pipe instruction for two elements.
 __device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, float b, float c) {
   asm("{\n\t"
@@ -84,18 +70,33 @@ __device__ __forceinline__ void add2(float& d0, float& d1, float a0, float a1) {
       : "f"(a0), "f"(a1));
 }
 
-constexpr int FA_POLY_PER_8 = 0;   // of every 8 exponentials, this many are evaluated by fa_exp2_poly
+constexpr int FA_BQ = 128;   // queries per tile
+constexpr int FA_BK = 128;   // keys per tile of the K and V rings
 
-constexpr int FA_BQ = 128;   // queries per tile (two tiles per CTA)
-constexpr int FA_BK = 128;   // keys per step
-constexpr int FA_THREADS = 64 + 256;   // TMA warp, MMA warp, 4 + 4 softmax warps
+// Heads of 128 (and ROPE): two query tiles per CTA, one CTA per SM, steps of 128 keys.  A row of 128 scores stays in registers, for which the
+// issuing warpgroup gives up some (80 + 2 * 208 <= 3 * 168, the registers at launch).
+// Heads of 64 and 32: one query tile and half of the tensor memory per CTA, two CTAs per SM, which also hide each other's first loads and
+// epilogues; steps of 64 keys, so that S of the next step is made while the softmax works on this one.
+// Forward, us, (batch x seq x heads x head): two tiles, scores read twice from tensor memory -> these.  64 x 256 x 16 x 32 50.0 -> 40.5,
+// 16 x 1024 x 12 x 64 79.9 -> 66.9, 3 x 777 x 12 x 64 18.8 -> 16.1; 8 x 2048 x 16 x 128 176 -> 169, 2 x 4096 x 32 x 128 293 -> 277.  Heads of 128 in steps
+// of 64 keys: 171 and 287; heads of 64 with two tiles in registers 77.1, in steps of 64 keys 76.4.
+template <int DH, bool ROPE>
+struct FwdShape {
+  static constexpr bool TWO = DH == 64 && !ROPE;
+  static constexpr int CTAS = TWO ? 2 : 1, TILES = TWO ? 1 : 2;
+  static constexpr int STEP = TWO ? 64 : 128, BUFS = 128 / STEP; // keys per step; S buffers of a tile
+  static constexpr int FIRST = TWO ? 2 : 4;                      // first softmax warp: behind TMA and MMA warp, or their warpgroup
+  static constexpr int THREADS = FIRST * 32 + 128 * TILES;       // 4 softmax warps per tile
+  static constexpr int REGS_ISSUE = 80, REGS_SOFTMAX = 208;      // with TWO: as launched
+  static constexpr int TMEM = 256 * TILES, TM_O = 128 * TILES;   // columns; S of the tiles, then O of the tiles, 128 apart
+};
 
 struct FlashFwdParams {
   __nv_bfloat16* o;      // (rows, d)
   float* lse;            // (batch, heads, seq)
   const int* cu_seqlens; // optional (batch+1) row offsets for packed variable-length sequences
   int batch, seq, heads, d;  // d = heads * dh; seq = max sequence length when cu_seqlens is given
-  int n_qblk;            // 128-query tiles per sequence; a CTA takes two of them
+  int n_qblk;            // 128-query tiles per sequence
   float scale_log2;      // softmax scale * log2(e)
   uint32_t* status;
   // WINDOW instances only
@@ -127,20 +128,21 @@ struct FlashFwdSmem {
   static constexpr int QK_BYTES = TILE_BYTES + (ROPE ? 16384 : 0);      // Q or K tile
   static constexpr int V_STAGES = ROPE && DH == 128 ? 1 : 2;
   static constexpr int OFF_Q = 0;                     // Q_A, Q_B
-  static constexpr int OFF_K = OFF_Q + 2 * QK_BYTES;
+  static constexpr int OFF_K = OFF_Q + FwdShape<DH, ROPE>::TILES * QK_BYTES;
   static constexpr int OFF_V = OFF_K + 2 * QK_BYTES;
   static constexpr int OFF_BAR = OFF_V + V_STAGES * TILE_BYTES;
-  static constexpr int NUM_BARS = 1 + 4 + 4 + 2 + 4 + 2;  // q, k full/empty, v full/empty, s_full[2], p_full[2][2], o_full[2]
+  static constexpr int NUM_BARS = 1 + 4 + 4 + 4 + 4 + 2 + 2;  // q, k full/empty, v full/empty, s_full[2][2], p_full[2][2], pv_done[2], o_full[2]
   static constexpr int TOTAL = OFF_BAR + NUM_BARS * 8 + 16 + 1024;
 };
 
 template <int DH, bool WINDOW, bool ROPE, int HW>
-__global__ void __launch_bounds__(FA_THREADS, 1)
+__global__ void __launch_bounds__(FwdShape<DH, ROPE>::THREADS, FwdShape<DH, ROPE>::CTAS)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_kv,
                  const __grid_constant__ CUtensorMap tm_kr, const FlashFwdParams p) {
   static_assert((WINDOW || !ROPE) && (HW == DH || (DH == 64 && !WINDOW)), "");
   using L = FlashFwdSmem<DH, ROPE>;
-  constexpr int VS = L::V_STAGES;
+  using F = FwdShape<DH, ROPE>;
+  constexpr int VS = L::V_STAGES, NT = F::TILES, STEP = F::STEP, BUFS = F::BUFS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
@@ -149,9 +151,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   uint64_t* k_empty = bars + 3;   // [2]  both tiles' S MMAs on this K stage have been issued and completed
   uint64_t* v_full = bars + 5;    // [2]
   uint64_t* v_empty = bars + 7;   // [2]  both tiles' P V MMAs on this V stage have completed
-  uint64_t* s_full = bars + 9;    // [2]  per tile: S_X(j) is in tensor memory (and P_X V_{j-1} has completed)
-  uint64_t* p_full = bars + 11;   // [2][2]  per tile and half of the key tile: P_X(j) is in tensor memory (128 arrivals)
-  uint64_t* o_full = bars + 15;   // [2]  per tile: the last P V MMA has completed
+  uint64_t* s_full = bars + 9;    // [2][2]  per tile and buffer: S_X(t) is in tensor memory
+  uint64_t* p_full = bars + 13;   // [2][2]  per tile and half of the key tile: P_X is in tensor memory (128 arrivals)
+  uint64_t* pv_done = bars + 17;  // [2]  per tile: P_X(t) V has completed (O_X may be rescaled)
+  uint64_t* o_full = bars + 19;   // [2]  per tile: the last P V MMA has completed
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + L::NUM_BARS);
   volatile uint32_t* abort_word = tmem_holder + 1;
 
@@ -159,7 +162,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
 
   // Work assignment: longest-first over the whole grid (latest query tiles = most key steps), so the tail of the
   // launch is made of short CTAs; the (b, h) index varies fastest.
-  const int n_pair = (p.n_qblk + 1) >> 1;
+  const int n_pair = (p.n_qblk + NT - 1) / NT;
   const int bh = blockIdx.x % (p.batch * p.heads);
   const int pair = n_pair - 1 - blockIdx.x / (p.batch * p.heads);
   const int b = bh / p.heads, h = bh % p.heads;
@@ -179,14 +182,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   }
   // CTA-uniform tile geometry: tile X covers queries [q0[X], q0[X] + 128) and key tiles lo_t[X] .. n_kv_t[X] - 1.  Tile A's
   // range starts and ends no later than tile B's and the two ranges leave no gap, so the CTA walks lo_t[0] .. n_kv - 1.
-  const int q0_t[2] = {pair * 2 * FA_BQ, pair * 2 * FA_BQ + FA_BQ};
-  int n_kv_t[2], lo_t[2];
+  int q0_t[NT], n_kv_t[NT], lo_t[NT];
 #pragma unroll
-  for (int x = 0; x < 2; ++x) {
+  for (int x = 0; x < NT; ++x) {
+    q0_t[x] = (pair * NT + x) * FA_BQ;
     n_kv_t[x] = q0_t[x] < seq_len ? (min(q0_t[x] + FA_BQ, seq_len) + shift + FA_BK - 1) / FA_BK : 0;
     lo_t[x] = (WINDOW && n_kv_t[x] > 0) ? max(0, q0_t[x] + shift - p.window + 1) / FA_BK : 0;
   }
-  const int n_kv = max(n_kv_t[0], n_kv_t[1]);
+  const int n_kv = max(n_kv_t[0], n_kv_t[NT - 1]);
   const int j0 = lo_t[0];
   const bool active = n_kv > 0;
 
@@ -197,7 +200,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1);
+      mbar_init(&s_full[2 * i], 1);
+      mbar_init(&s_full[2 * i + 1], 1);
+      mbar_init(&pv_done[i], 1);
       mbar_init(&p_full[2 * i], 128);
       mbar_init(&p_full[2 * i + 1], 128);
       mbar_init(&o_full[i], 1);
@@ -209,7 +214,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     if (ROPE) prefetch_tensormap(&tm_kr);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_holder, 512);
+    tmem_alloc(tmem_holder, F::TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -217,7 +222,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   tc_fence_after();
   pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
-  // columns: S_A [0,128)  S_B [128,256)  O_A [256,256+DH)  O_B [384,384+DH); P_X overlays the first 64 columns of S_X
+  // columns: S_X [128 X, 128 X + 128), two halves; O_X from TM_O + 128 X; P_X overlays the first 32 columns of a half
 
   const int col_q = h * (WINDOW ? p.q_step : HW), col_k = WINDOW ? h * p.k_step : p.d + h * HW,
             col_v = WINDOW ? p.v_off + h * p.v_step : 2 * p.d + h * HW;
@@ -225,13 +230,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   const int ksteps = WINDOW ? (p.dim + 15) / 16 : DH / 16;
   const CUtensorMap* const map_kv = WINDOW ? &tm_kv : &tm_qkv;
 
+  if (warp < F::FIRST) {
+  if (!F::TWO) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F::REGS_ISSUE));
   if (warp == 0) {
     if (active && elect_one()) {   // elect.sync keeps the issuing code warp-uniform (descriptors in uniform registers)
       // rows past the end of the tensor are zero-filled by TMA; rows of a following packed sequence are masked or unused
       const uint32_t qk_bytes = (uint32_t)(pd + (ROPE ? 1 : 0)) * 16384u;
-      mbar_expect_tx(q_full, 2 * qk_bytes);
+      mbar_expect_tx(q_full, NT * qk_bytes);
 #pragma unroll
-      for (int x = 0; x < 2; ++x) {
+      for (int x = 0; x < NT; ++x) {
 #pragma unroll
         for (int pn = 0; pn < L::PANELS; ++pn)
           if (pn < pd)
@@ -262,95 +269,102 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     if (active && elect_one()) {
       const int lane = 0;   // the tracing macro stamps from the issuing thread
       (void)lane;
-      constexpr uint32_t idesc_qk = make_idesc_bf16(128, FA_BK, false, false);
+      constexpr uint32_t idesc_qk = make_idesc_bf16(128, STEP, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, DH, false, true);
-      auto issue_s = [&](int x, int j) {   // S_X(j) = Q_X K_j^T
+      auto issue_s = [&](int x, int t) {   // S_X(t) = Q_X K(t)^T, into buffer t % BUFS of the tile's columns
+        const int buf = t % BUFS;
+        const uint32_t d_tmem = tmem_base + x * 128 + buf * STEP;
         const uint64_t q_desc = make_smem_desc(smem_u32(smem + L::OFF_Q + x * L::QK_BYTES), 16, 1024);
-        const uint64_t k_desc = make_smem_desc(smem_u32(smem + L::OFF_K + ((j - j0) & 1) * L::QK_BYTES), 16, 1024);
+        const uint64_t k_desc = make_smem_desc(smem_u32(smem + L::OFF_K + ((t / BUFS - j0) & 1) * L::QK_BYTES + buf * STEP * 128), 16, 1024);
         if (ROPE) {
           const int rsteps = (p.rot + 15) / 16;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             if (k >= rsteps) break;
             const uint32_t off = (L::TILE_BYTES + k * 32) >> 4;
-            umma_f16_ss(tmem_base + x * 128, q_desc + off, k_desc + off, idesc_qk, k > 0 ? 1u : 0u);
+            umma_f16_ss(d_tmem, q_desc + off, k_desc + off, idesc_qk, k > 0 ? 1u : 0u);
           }
         }
 #pragma unroll
         for (int k = 0; k < HW / 16; ++k) {
           if (WINDOW && k >= ksteps) break;
           const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4;
-          umma_f16_ss(tmem_base + x * 128, q_desc + off, k_desc + off, idesc_qk, (ROPE || k > 0) ? 1u : 0u);
+          umma_f16_ss(d_tmem, q_desc + off, k_desc + off, idesc_qk, (ROPE || k > 0) ? 1u : 0u);
         }
-        umma_commit(&s_full[x]);
+        umma_commit(&s_full[2 * x + buf]);
       };
-      // O_X += P_X(j) V_j, one half of the key tile at a time (the softmax warps publish P in two halves):
-      // A = P from tensor memory (16 keys = 8 packed columns), B = V MN-major (dh contiguous, keys are rows of
-      // 128 B): 16 keys = 2048 B; dh panels 16384 B apart.
+      // O_X += P_X V over one half of key tile j: A = P from tensor memory (16 keys = 8 packed columns), B = V MN-major (dh contiguous, keys
+      // are rows of 128 B): 16 keys = 2048 B; dh panels 16384 B apart.
       auto issue_pv = [&](int x, int j, int half) {
         const uint64_t v_desc = make_smem_desc(smem_u32(smem + L::OFF_V + ((j - j0) % VS) * L::TILE_BYTES), 16384, 1024);
 #pragma unroll
-        for (int kk = 0; kk < FA_BK / 32; ++kk) {
-          const int k = half * (FA_BK / 32) + kk;
-          umma_f16_ts(tmem_base + 256 + x * 128, tmem_base + x * 128 + k * 8, v_desc + ((k * 2048) >> 4), idesc_pv,
+        for (int kk = 0; kk < 4; ++kk) {
+          const int k = half * 4 + kk;
+          umma_f16_ts(tmem_base + F::TM_O + x * 128, tmem_base + x * 128 + half * (BUFS == 2 ? STEP : 32) + kk * 8, v_desc + ((k * 2048) >> 4), idesc_pv,
                       (j > lo_t[x] || k > 0) ? 1u : 0u);
         }
         if (half == 1 && j == n_kv_t[x] - 1) umma_commit(&o_full[x]);
+        else if (BUFS == 2) umma_commit(&pv_done[x]);
       };
       bool ok = mbar_wait(q_full, 0, abort_word) && mbar_wait(&k_full[0], 0, abort_word);
       if (ok) {
         tc_fence_after();
-        if (n_kv_t[0] > 0) issue_s(0, j0);
-        if (n_kv_t[1] > 0 && lo_t[1] == j0) issue_s(1, j0);
+#pragma unroll
+        for (int buf = 0; buf < BUFS; ++buf)
+#pragma unroll
+          for (int x = 0; x < NT; ++x)
+            if (n_kv_t[x] > 0 && lo_t[x] == j0) issue_s(x, BUFS * j0 + buf);
         umma_commit(&k_empty[0]);
       }
       for (int j = j0; j < n_kv && ok; ++j) {
         const int st = (j - j0) & 1, sv = (j - j0) % VS;
         const uint32_t pv = ((j - j0) / VS) & 1;
         bool v_ready = false, k_ready = false;
+        // tile by tile, half by half
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
+        for (int i = 0; i < 2 * NT; ++i) {
+          const int x = i / 2, half = i % 2;
+          if (!ok) break;
           if (j >= lo_t[x] && j < n_kv_t[x]) {
-            ok = mbar_wait(&p_full[2 * x], (j - lo_t[x]) & 1, abort_word) && (v_ready || mbar_wait(&v_full[sv], pv, abort_word));
+            ok = mbar_wait(&p_full[2 * x + half], (j - lo_t[x]) & 1, abort_word) && (v_ready || mbar_wait(&v_full[sv], pv, abort_word));
             if (!ok) break;
             v_ready = true;
             tc_fence_after();
-            FWD_TRACE(1, j, x * 4 + 0);
-            issue_pv(x, j, 0);
-            ok = mbar_wait(&p_full[2 * x + 1], (j - lo_t[x]) & 1, abort_word);
-            if (!ok) break;
-            tc_fence_after();
-            issue_pv(x, j, 1);
-            FWD_TRACE(1, j, x * 4 + 1);
+            FWD_TRACE(1, j, x * 4 + half);
+            issue_pv(x, j, half);
           }
-          if (x == 1) umma_commit(&v_empty[sv]);   // both tiles are done with V_j
-          if (j + 1 >= lo_t[x] && j + 1 < n_kv_t[x]) {
+          // the buffer that P just left takes S of the next tile
+          if ((BUFS == 2 || half == 1) && j + 1 >= lo_t[x] && j + 1 < n_kv_t[x]) {
             ok = k_ready || mbar_wait(&k_full[st ^ 1], ((j + 1 - j0) >> 1) & 1, abort_word);
             if (!ok) break;
             k_ready = true;
             tc_fence_after();
-            issue_s(x, j + 1);
+            issue_s(x, BUFS * (j + 1) + (BUFS == 2 ? half : 0));
             FWD_TRACE(1, j, x * 4 + 2);
           }
         }
+        if (ok) umma_commit(&v_empty[sv]);       // both tiles are done with V_j
         if (ok && j + 1 < n_kv) umma_commit(&k_empty[st ^ 1]);   // both tiles are done with K_{j+1}
       }
       if (!ok) *abort_word = ERR_WAIT_FULL;
     }
-  } else if (active) {
+  }
+  } else {
+  if (!F::TWO) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(F::REGS_SOFTMAX));
+  if (active) {
     // ----------------------------------------------------------------- softmax warps: one thread per query row
-    const int x = (warp - 2) >> 2;              // tile A (warps 2-5) or B (warps 6-9)
+    const int x = NT == 1 ? 0 : (warp - F::FIRST) >> 2;        // tile A or B
     const int quarter = warp & 3;               // TMEM lanes [32*quarter, 32*quarter+32) are visible to this warp
     const int r = quarter * 32 + lane;          // row inside the query tile
-    const int q0 = (pair * 2 + x) * FA_BQ;
-    const int n_kv_x = x == 0 ? n_kv_t[0] : n_kv_t[1];
-    const int lo_x = x == 0 ? lo_t[0] : lo_t[1];
+    const int q0 = (pair * NT + x) * FA_BQ;
+    const int n_kv_x = x == 0 ? n_kv_t[0] : n_kv_t[NT - 1];
+    const int lo_x = x == 0 ? lo_t[0] : lo_t[NT - 1];
     const int q_idx = q0 + r;                   // query of this thread
     const int q_key = q_idx + shift;            // its position among the keys
     const int q_low = WINDOW ? q_key - p.window : -1;   // the last key it no longer sees
     const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
-    const uint32_t tm_s = tmem_base + x * 128 + lane_addr;
-    const uint32_t tm_o = tmem_base + 256 + x * 128 + lane_addr;
+    const uint32_t tm_x = tmem_base + x * 128 + lane_addr;
+    const uint32_t tm_o = tmem_base + F::TM_O + x * 128 + lane_addr;
     float m_run = -INFINITY;                    // running reference max in scaled log2 units
     float l_run = 0.f;                          // running row sum relative to m_run
     bool ok = true;
@@ -358,56 +372,50 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       const __nv_bfloat16* grow = p.gate + (long long)(row_base + q_idx) * p.ld_gate + h * p.vdim;
       for (int i = 0; i < p.vdim; i += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(grow + i));
     }
-    for (int j = lo_x; j < n_kv_x; ++j) {
-      const int trole = warp;
-      FWD_TRACE(trole, j, 0);
-      if (!mbar_wait(&s_full[x], (j - lo_x) & 1, abort_word)) { ok = false; break; }
+    for (int t = BUFS * lo_x; t < BUFS * n_kv_x; ++t) {
+      const int trole = warp - F::FIRST + 2, buf = t % BUFS;
+      const uint32_t tm_s = tm_x + buf * STEP;
+      FWD_TRACE(trole, t, 0);
+      if (!mbar_wait(&s_full[2 * x + buf], (t / BUFS - lo_x) & 1, abort_word)) { ok = false; break; }
       tc_fence_after();
-      FWD_TRACE(trole, j, 1);
-      const int k0 = j * FA_BK;
+      FWD_TRACE(trole, t, 1);
+      const int k0 = t * STEP;
       // tile touches the diagonal or the lower edge of the window (warp-uniform)
-      const bool diag = (k0 + FA_BK - 1 > q0 + shift) || (WINDOW && k0 <= q0 + FA_BQ - 1 + shift - p.window);
-      // pass 1: row maximum over the raw scores (the softmax scale is positive, so it is applied afterwards).
-      // The load of chunk c+1 is in flight while chunk c is reduced.
-      float mx = -INFINITY;
-      // Key k0 + e is visible iff e - first <= span as unsigned numbers (one comparison for both edges of the window).
+      const bool diag = (k0 + STEP - 1 > q0 + shift) || (WINDOW && k0 <= q0 + FA_BQ - 1 + shift - p.window);
+      // The row's scores stay in registers from here to P.  Key k0 + e is visible iff e - first <= span as unsigned numbers (one comparison for
+      // both edges of the window).
       const int first = q_low + 1 - k0;
       const uint32_t span = WINDOW ? (uint32_t)(p.window - 1) : 0u;
-      auto hidden = [&](int e) { return WINDOW ? (uint32_t)(e - first) > span : k0 + e > q_key; };
-      auto row_max = [&](const bool masked) __attribute__((always_inline)) {
-        uint32_t sa[32], sb[32];
-        tmem_ld_32x32(tm_s, sa);
-        tmem_ld_wait();
+      uint32_t s[STEP / 32][32];
 #pragma unroll
-        for (int c = 0; c < FA_BK / 32; ++c) {
-          uint32_t (&cur)[32] = (c & 1) ? sb : sa;
-          uint32_t (&nxt)[32] = (c & 1) ? sa : sb;
-          if (c + 1 < FA_BK / 32) tmem_ld_32x32(tm_s + (c + 1) * 32, nxt);
-          if (masked) {
+      for (int c = 0; c < STEP / 32; ++c) tmem_ld_32x32(tm_s + c * 32, s[c]);
+      tmem_ld_wait();
+      if (diag) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (hidden(c * 32 + i)) cur[i] = 0xff800000u;   // -inf
-          }
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) mx = fmax3(mx, __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]));
-          if (c + 1 < FA_BK / 32) tmem_ld_wait();
-        }
-      };
-      if (WINDOW) {                    // two copies: tiles inside the window pay nothing for its edges
-        if (diag) row_max(true);
-        else row_max(false);
-      } else {
-        row_max(diag);
+        for (int e = 0; e < STEP; ++e)
+          if (WINDOW ? (uint32_t)(e - first) > span : k0 + e > q_key) s[e / 32][e % 32] = 0xff800000u;   // -inf
       }
+      // row maximum over the raw scores (the softmax scale is positive, so it is applied afterwards)
+      float mc[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t* v = &s[c * STEP / 128][c * STEP / 4 % 32];
+        mc[c] = fmaxf(__uint_as_float(v[0]), __uint_as_float(v[1]));
+#pragma unroll
+        for (int i = 2; i < STEP / 4; i += 2) mc[c] = fmax3(mc[c], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+      }
+      float mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3]));
       mx *= p.scale_log2;
-      FWD_TRACE(trole, j, 2);
+      FWD_TRACE(trole, t, 2);
       // Lazy rescale: keep the old reference max unless it moved by more than 8 (a factor 256).
       float m_new = m_run;
       if (mx > m_run + 8.f) m_new = mx;
       const bool need = m_new != m_run;
       const float alpha = (m_run == -INFINITY) ? 0.f : fa_exp2(m_run - m_new);
-      // S_X(j) was issued after P_X V_{j-1}, so that MMA has completed and O_X may be rescaled here.
-      if (j > lo_x && __any_sync(0xffffffffu, need)) {
+      if (t > BUFS * lo_x && __any_sync(0xffffffffu, need)) {
+        // O_X is at rest until P_X(t) is published.  With one buffer S_X(t) was issued behind P_X(t - 1) V, which has completed.
+        if (BUFS == 2 && !mbar_wait(&pv_done[x], (t - 1) & 1, abort_word)) { ok = false; break; }
+        tc_fence_after();
         const float f = need ? alpha : 1.f;
 #pragma unroll 1
         for (int c = 0; c < HW / 32; ++c) {
@@ -419,53 +427,32 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
           tmem_st_32x32(tm_o + c * 32, o);
         }
       }
-      FWD_TRACE(trole, j, 3);
-      // pass 2: P = exp2(S * scale - m), row sum, bf16 pack; P chunk c (16 packed columns) lands on S columns
-      // [16c, 16c+16), all of which this thread has already read.
-      // (a row whose window starts in a later tile has seen no key yet: every P is masked to zero below)
+      FWD_TRACE(trole, t, 3);
+      // P = exp2(S * scale - m), row sum, bf16 pack; P (packed columns) lands on S columns, which this thread has read.
+      // (a row whose window starts in a later tile has seen no key yet: all its scores are -inf, every P is zero)
       const float m_ref = (WINDOW && m_new == -INFINITY) ? 0.f : m_new;
       float sum = 0.f, sum1 = 0.f;
-      auto weights = [&](const bool masked) __attribute__((always_inline)) {
-        uint32_t sa[32], sb[32];
-        tmem_ld_32x32(tm_s, sa);
-        tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < FA_BK / 32; ++c) {
-          uint32_t (&s)[32] = (c & 1) ? sb : sa;
-          uint32_t (&nxt)[32] = (c & 1) ? sa : sb;
-          uint32_t pk[16];
-          if (c + 1 < FA_BK / 32) tmem_ld_32x32(tm_s + (c + 1) * 32, nxt);   // in flight while this chunk is processed
+      for (int c = 0; c < STEP / 32; ++c) {
+        uint32_t pk[16];
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float x0, x1;
-            fma2(x0, x1, __uint_as_float(s[i]), __uint_as_float(s[i + 1]), p.scale_log2, -m_ref);
-            float e0 = ((i & 7) < FA_POLY_PER_8) ? fa_exp2_poly(x0) : fa_exp2(x0);
-            float e1 = (((i + 1) & 7) < FA_POLY_PER_8) ? fa_exp2_poly(x1) : fa_exp2(x1);
-            if (masked) {
-              e0 = hidden(c * 32 + i) ? 0.f : e0;
-              e1 = hidden(c * 32 + i + 1) ? 0.f : e1;
-            }
-            add2(sum, sum1, e0, e1);
-            pk[i / 2] = pack_bf16x2(e0, e1);
-          }
-          if (c + 1 < FA_BK / 32) tmem_ld_wait();   // before the store below: wait::ld covers the prefetched chunk
-          tmem_st_32x16(tm_s + c * 16, pk);
-          if (c == 1 || c == 3) {   // publish this half of P
-            tmem_st_wait();
-            tc_fence_before();
-            mbar_arrive(&p_full[2 * x + (c >> 1)]);
-          }
+        for (int i = 0; i < 32; i += 2) {
+          float x0, x1;
+          fma2(x0, x1, __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]), p.scale_log2, -m_ref);
+          const float e0 = fa_exp2(x0), e1 = fa_exp2(x1);
+          add2(sum, sum1, e0, e1);
+          pk[i / 2] = pack_bf16x2(e0, e1);
         }
-      };
-      if (WINDOW) {
-        if (diag) weights(true);
-        else weights(false);
-      } else {
-        weights(diag);
+        tmem_st_32x16(tm_s + c * 16, pk);
+        if (c % 2 == 1) {          // publish 64 keys
+          tmem_st_wait();
+          tc_fence_before();
+          mbar_arrive(&p_full[2 * x + (BUFS == 2 ? buf : c / 2)]);
+        }
       }
       l_run = l_run * (need ? alpha : 1.f) + (sum + sum1);
       m_run = m_new;
-      FWD_TRACE(trole, j, 4);
+      FWD_TRACE(trole, t, 4);
     }
     // ------------------------------------------------------------------- epilogue
     if (ok && n_kv_x > 0) ok = mbar_wait(&o_full[x], 0, abort_word);
@@ -533,6 +520,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
       *abort_word = ERR_WAIT_TMEM_FULL;
     }
   }
+  }
 
   __syncwarp();
   tc_fence_before();
@@ -545,7 +533,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, F::TMEM);
   }
 }
 
@@ -559,8 +547,9 @@ static int launch_flash_fwd(const CUtensorMap& tm, const CUtensorMap& tm_kv, con
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess) return -3;
     configured = true;
   }
-  const int grid = p.batch * p.heads * ((p.n_qblk + 1) / 2);   // one CTA per pair of query tiles
-  launch_dep(kern, grid, FA_THREADS, L::TOTAL, stream, tm, tm_kv, tm_kr != nullptr ? *tm_kr : tm_kv, p);
+  using F = FwdShape<DH, ROPE>;
+  const int grid = p.batch * p.heads * ((p.n_qblk + F::TILES - 1) / F::TILES);
+  launch_dep(kern, grid, F::THREADS, L::TOTAL, stream, tm, tm_kv, tm_kr != nullptr ? *tm_kr : tm_kv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -131,15 +131,23 @@ __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, const __
   }
 }
 
-// The element-wise stage of both kernels is spread over BWD_CG warpgroups: warpgroup g handles
-// columns [g*BWD_COLS, (g+1)*BWD_COLS) of every 64-column step, so 8 warps (2 per scheduler) hide each
-// other's TMEM-load, exp2 and shared-memory latencies instead of one warp per scheduler.
+// How an instance fills an SM.  Heads of 128: one CTA, whose element-wise stage is spread over two warpgroups (warpgroup g handles its share of
+// the columns of every step, so 8 warps hide each other's TMEM-load, exp2 and shared-memory latencies), with two S / dP buffers.  Heads of
+// 64 (and 32): two CTAs with one warpgroup, half of the tensor memory and single buffers each, which hide each other's latencies, first
+// loads and epilogues.
+template <int DH, bool TWO>
+struct BwdShape {
+  static_assert(!TWO || DH == 64, "two CTAs share the tensor memory of heads of 64 columns");
+  static constexpr int CTAS = TWO ? 2 : 1;                      // per SM
+  static constexpr int CG = TWO ? 1 : 2;                        // warpgroups
+  static constexpr int COMPUTE = 128 * CG, THREADS = 64 + COMPUTE;      // + TMA warp + MMA warp
+  static constexpr int TMEM = 512 / CTAS;
+  static constexpr int BUFS = TWO ? 1 : 2;                      // S^T / dP^T buffers of the dK/dV kernel
+  static constexpr int VEC_STEPS = TWO ? 16 : 32;               // dK/dV: steps whose lse / delta are staged in shared memory at a time
+  static constexpr int KEYS = TWO ? 64 : 128;                   // dQ: keys per step
+  static constexpr int KSTAGES = TWO ? 4 : 3, VSTAGES = TWO ? 3 : 2;    // dQ: K and V rings
+};
 constexpr int BWD_RING = 4;   // TMA ring depth of the dK/dV kernel's per-step Q / dO tiles
-constexpr int DKDV_VEC_STEPS = 32;   // steps whose lse / delta are staged in shared memory at a time
-constexpr int BWD_CG = 2;
-constexpr int BWD_COLS = 64 / BWD_CG;                 // 32 columns per thread and step
-constexpr int BWD_COMPUTE_THREADS = 128 * BWD_CG;     // 256
-constexpr int BWD_THREADS = 64 + BWD_COMPUTE_THREADS; // + TMA warp + MMA warp
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -155,7 +163,7 @@ __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
 // P^T and dS^T never touch shared memory: the compute warps write them as packed bf16 over the S^T / dP^T
 // columns they have just read (tcgen05.st) and the dV / dK MMAs take their A operand from tensor memory.
 // The shared memory that frees holds a five-stage Q / dO ring.
-template <int DH>
+template <int DH, bool TWO>
 struct DkDvSmem {
   static constexpr int PANELS = DH / 64;
   static constexpr int KV_TILE = 128 * DH * 2;   // K_j or V_j (128 keys)
@@ -164,19 +172,20 @@ struct DkDvSmem {
   static constexpr int OFF_V = OFF_K + KV_TILE;
   static constexpr int OFF_Q = OFF_V + KV_TILE;                // BWD_RING stages
   static constexpr int OFF_DO = OFF_Q + BWD_RING * Q_TILE;     // BWD_RING stages
-  static constexpr int OFF_VEC = OFF_DO + BWD_RING * Q_TILE;   // lse and delta of DKDV_VEC_STEPS steps (floats)
-  static constexpr int OFF_BAR = OFF_VEC + 2 * DKDV_VEC_STEPS * 64 * 4;
+  static constexpr int OFF_VEC = OFF_DO + BWD_RING * Q_TILE;   // lse and delta of VEC_STEPS steps (floats)
+  static constexpr int OFF_BAR = OFF_VEC + 2 * BwdShape<DH, TWO>::VEC_STEPS * 64 * 4;
   static constexpr int NUM_BARS = 1 + 2 * BWD_RING + 5;
   static constexpr int TOTAL = OFF_BAR + NUM_BARS * 8 + 16 + 1024;
 };
 
-template <int DH, int HW>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+template <int DH, int HW, bool TWO>
+__global__ void __launch_bounds__(BwdShape<DH, TWO>::THREADS, BwdShape<DH, TWO>::CTAS)
 flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 over qkv
                   const __grid_constant__ CUtensorMap tm_q,    // box 64 x 64 over qkv
                   const __grid_constant__ CUtensorMap tm_do,   // box 64 x 64 over dO
                   const FlashBwdParams p) {
-  using L = DkDvSmem<DH>;
+  using L = DkDvSmem<DH, TWO>;
+  using B = BwdShape<DH, TWO>;
   const uint64_t t_cta_start = globaltimer_ns();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -189,8 +198,8 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
   uint64_t* all_done = p_full + 2;                 // every MMA of the CTA has completed
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + L::NUM_BARS);
   volatile uint32_t* abort_word = tmem_holder + 1;
-  float* lse_s = reinterpret_cast<float*>(smem + L::OFF_VEC);   // [DKDV_VEC_STEPS * 64]
-  float* delta_s = lse_s + DKDV_VEC_STEPS * 64;                 // [DKDV_VEC_STEPS * 64]
+  float* lse_s = reinterpret_cast<float*>(smem + L::OFF_VEC);   // [VEC_STEPS * 64]
+  float* delta_s = lse_s + B::VEC_STEPS * 64;                   // [VEC_STEPS * 64]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Longest-first order over the whole grid (small j = most query steps), so the tail of the launch is made of
@@ -212,7 +221,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], BWD_COMPUTE_THREADS);
+      mbar_init(&p_full[i], B::COMPUTE);
     }
     mbar_init(all_done, 1);
     *abort_word = 0;
@@ -222,7 +231,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
     prefetch_tensormap(&tm_do);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_holder, 512);
+    tmem_alloc(tmem_holder, B::TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -230,10 +239,10 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
   tc_fence_after();
   pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tm_st = tmem_base;         // S^T: 2 x 64 columns
-  const uint32_t tm_dpt = tmem_base + 128;  // dP^T: 2 x 64 columns
-  const uint32_t tm_dv = tmem_base + 256;   // DH columns
-  const uint32_t tm_dk = tmem_base + 384;   // DH columns
+  const uint32_t tm_st = tmem_base;                                // S^T: BUFS x 64 columns
+  const uint32_t tm_dpt = tmem_base + B::BUFS * 64;                // dP^T: BUFS x 64 columns
+  const uint32_t tm_dv = tmem_base + B::BUFS * 128;                // DH columns
+  const uint32_t tm_dk = tmem_base + B::BUFS * 128 + B::TMEM / 4;  // DH columns
 
   const int col_q = h * HW, col_k = p.d + h * HW, col_v = 2 * p.d + h * HW;
 
@@ -268,7 +277,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
       constexpr uint32_t idesc_34 = make_idesc_bf16(128, DH, false, true);
       const uint32_t k_addr = smem_u32(smem + L::OFF_K), v_addr = smem_u32(smem + L::OFF_V);
       auto issue12 = [&](int t) {
-        const int st = t & 1, rs = t % BWD_RING;
+        const int st = t % B::BUFS, rs = t % BWD_RING;
         const uint32_t q_addr = smem_u32(smem + L::OFF_Q + rs * L::Q_TILE);
         const uint32_t do_addr = smem_u32(smem + L::OFF_DO + rs * L::Q_TILE);
 #pragma unroll
@@ -290,8 +299,8 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
       bool ok = mbar_wait(kv_full, 0, abort_word) && mbar_wait(&qd_full[0], 0, abort_word);
       if (ok) { tc_fence_after(); issue12(0); }
       for (int t = 0; t < n_steps && ok; ++t) {
-        const int st = t & 1;
-        if (t + 1 < n_steps) {
+        const int st = t % B::BUFS;
+        if (B::BUFS == 2 && t + 1 < n_steps) {
           // Buffer (t+1)&1 is free: its last readers, the compute warps of step t-1, arrived on p_full before the
           // dV / dK MMAs of step t-1 were issued, and those MMAs precede this issue in the tensor pipe.
           ok = mbar_wait(&qd_full[(t + 1) % BWD_RING], ((t + 1) / BWD_RING) & 1, abort_word);
@@ -301,29 +310,36 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
           issue12(t + 1);
           BWD_TRACE(1, t, 1);
         }
-        ok = mbar_wait(&p_full[st], (t >> 1) & 1, abort_word);
+        ok = mbar_wait(&p_full[st], (t / B::BUFS) & 1, abort_word);
         if (!ok) break;
         tc_fence_after();
         BWD_TRACE(1, t, 2);
         const int rs = t % BWD_RING;
         const uint32_t q_addr = smem_u32(smem + L::OFF_Q + rs * L::Q_TILE);
         const uint32_t do_addr = smem_u32(smem + L::OFF_DO + rs * L::Q_TILE);
-        // K = 64 queries.  A: column group g of the compute warps left queries [32g, 32g+32) as 16 packed columns
+        // K = 64 queries.  A: the compute warps left queries [32g, 32g+32) as 16 packed columns
         // at column 32g of the S^T / dP^T buffer.  B operands are MN-major: dh contiguous, 16 queries = 2048 B per
         // step, dh panels 8192 B apart.
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint32_t a_off = st * 64 + (k >> 1) * BWD_COLS + (k & 1) * 8;
+          const uint32_t a_off = st * 64 + (k >> 1) * 32 + (k & 1) * 8;
           umma_f16_ts(tm_dv, tm_st + a_off, make_smem_desc(do_addr + k * 2048, 8192, 1024), idesc_34,
                       (t > 0 || k > 0) ? 1u : 0u);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint32_t a_off = st * 64 + (k >> 1) * BWD_COLS + (k & 1) * 8;
+          const uint32_t a_off = st * 64 + (k >> 1) * 32 + (k & 1) * 8;
           umma_f16_ts(tm_dk, tm_dpt + a_off, make_smem_desc(q_addr + k * 2048, 8192, 1024), idesc_34,
                       (t > 0 || k > 0) ? 1u : 0u);
         }
         umma_commit(&qd_empty[rs]);
+        if (B::BUFS == 1 && t + 1 < n_steps) {
+          // S^T and dP^T take the place of P^T and dS^T, which the MMAs just issued read first
+          ok = mbar_wait(&qd_full[(t + 1) % BWD_RING], ((t + 1) / BWD_RING) & 1, abort_word);
+          if (!ok) break;
+          tc_fence_after();
+          issue12(t + 1);
+        }
         if (t == n_steps - 1) umma_commit(all_done);
         BWD_TRACE(1, t, 3);
       }
@@ -332,7 +348,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
   } else {
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;      // key row inside the tile
-    const int tid = (warp - 2) * 32 + lane; // 0..511 among the compute threads
+    const int tid = (warp - 2) * 32 + lane; // among the compute threads
     const int cg = (warp - 2) >> 2;         // column group of this warpgroup
     const int key_idx = k0 + r;
     const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
@@ -340,71 +356,75 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
     const float* delta_g = p.delta + ((size_t)b * p.heads + h) * p.seq;
     bool ok = true;
     // lse (in log2 units; +inf zeroes the probabilities of padded queries) and delta * scale of the next
-    // DKDV_VEC_STEPS steps are staged in shared memory by all compute threads together, so no step waits on a
+    // VEC_STEPS steps are staged in shared memory by all compute threads together, so no step waits on a
     // global load; the two barriers around a refill are reached by every compute thread, also after a failed wait.
     for (int t = 0; t < n_steps; ++t) {
-      const int st = t & 1;
-      const uint32_t ph = (t >> 1) & 1;
+      const int st = t % B::BUFS;
+      const uint32_t ph = (t / B::BUFS) & 1;
       const int qb = (i0 + t) * 64;
       BWD_TRACE(warp, t, 0);
-      if (t % DKDV_VEC_STEPS == 0) {
-        if (t > 0) named_barrier_sync(1, BWD_COMPUTE_THREADS);   // everyone is done with the previous chunk
+      if (t % B::VEC_STEPS == 0) {
+        if (t > 0) named_barrier_sync(1, B::COMPUTE);   // everyone is done with the previous chunk
         const int q_first = (i0 + t) * 64;
-        constexpr int PER = DKDV_VEC_STEPS * 64 / BWD_COMPUTE_THREADS;
+        constexpr int PER = B::VEC_STEPS * 64 / B::COMPUTE;
         float lv[PER], dv[PER];
 #pragma unroll
         for (int i = 0; i < PER; ++i) {   // all loads in flight before the first store
-          const int qi = q_first + tid + i * BWD_COMPUTE_THREADS;
+          const int qi = q_first + tid + i * B::COMPUTE;
           lv[i] = (qi < p.seq) ? lse_g[qi] : INFINITY;
           dv[i] = (qi < p.seq) ? delta_g[qi] : 0.f;
         }
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
-          lse_s[tid + i * BWD_COMPUTE_THREADS] = lv[i] * 1.4426950408889634f;
-          delta_s[tid + i * BWD_COMPUTE_THREADS] = dv[i] * p.scale;
+          lse_s[tid + i * B::COMPUTE] = lv[i] * 1.4426950408889634f;
+          delta_s[tid + i * B::COMPUTE] = dv[i] * p.scale;
         }
-        named_barrier_sync(1, BWD_COMPUTE_THREADS);
+        named_barrier_sync(1, B::COMPUTE);
       }
       if (!ok) continue;
       BWD_TRACE(warp, t, 1);
       if (!mbar_wait(&s_full[st], ph, abort_word)) { ok = false; continue; }
       tc_fence_after();
       BWD_TRACE(warp, t, 2);
-      uint32_t sreg[BWD_COLS], dreg[BWD_COLS];
-      tmem_ld_32x32(tm_st + lane_addr + st * 64 + cg * BWD_COLS, sreg);
-      tmem_ld_32x32(tm_dpt + lane_addr + st * 64 + cg * BWD_COLS, dreg);
-      tmem_ld_wait();
-      BWD_TRACE(warp, t, 3);
       const bool need_mask = (qb < k0 + 128);   // tile touches the diagonal
-      const float* lse_v = lse_s + (t % DKDV_VEC_STEPS) * 64 + cg * BWD_COLS;   // lse * log2(e); +inf marks a padded query
-      const float* dlt_v = delta_s + (t % DKDV_VEC_STEPS) * 64 + cg * BWD_COLS;  // delta * scale
-      // Eight columns at a time: two 16-byte broadcast reads each of lse and delta, eight independent
-      // exp2 / multiply chains, four packed results each of P^T and dS^T (bf16 packing on the integer pipe).
-      uint32_t pk[BWD_COLS / 2], dk[BWD_COLS / 2];
+      // 32 columns (queries) at a time; with two warpgroups each has its 32
 #pragma unroll
-      for (int c0 = 0; c0 < BWD_COLS; c0 += 8) {
-        float lr[8], dr[8], pe[8], ds[8];
-        *reinterpret_cast<float4*>(lr) = *reinterpret_cast<const float4*>(lse_v + c0);
-        *reinterpret_cast<float4*>(lr + 4) = *reinterpret_cast<const float4*>(lse_v + c0 + 4);
-        *reinterpret_cast<float4*>(dr) = *reinterpret_cast<const float4*>(dlt_v + c0);
-        *reinterpret_cast<float4*>(dr + 4) = *reinterpret_cast<const float4*>(dlt_v + c0 + 4);
+      for (int g = cg; g < 2; g += B::CG) {
+        uint32_t sreg[32], dreg[32];
+        tmem_ld_32x32(tm_st + lane_addr + st * 64 + g * 32, sreg);
+        tmem_ld_32x32(tm_dpt + lane_addr + st * 64 + g * 32, dreg);
+        tmem_ld_wait();
+        BWD_TRACE(warp, t, 3);
+        const float* lse_v = lse_s + (t % B::VEC_STEPS) * 64 + g * 32;   // lse * log2(e); +inf marks a padded query
+        const float* dlt_v = delta_s + (t % B::VEC_STEPS) * 64 + g * 32;  // delta * scale
+        // Eight columns at a time: two 16-byte broadcast reads each of lse and delta, eight independent
+        // exp2 / multiply chains, four packed results each of P^T and dS^T (bf16 packing on the integer pipe).
+        uint32_t pk[16], dk[16];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) pe[e] = fast_exp2(__uint_as_float(sreg[c0 + e]) * p.scale_log2 - lr[e]);
-        if (need_mask) {
+        for (int c0 = 0; c0 < 32; c0 += 8) {
+          float lr[8], dr[8], pe[8], ds[8];
+          *reinterpret_cast<float4*>(lr) = *reinterpret_cast<const float4*>(lse_v + c0);
+          *reinterpret_cast<float4*>(lr + 4) = *reinterpret_cast<const float4*>(lse_v + c0 + 4);
+          *reinterpret_cast<float4*>(dr) = *reinterpret_cast<const float4*>(dlt_v + c0);
+          *reinterpret_cast<float4*>(dr + 4) = *reinterpret_cast<const float4*>(dlt_v + c0 + 4);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) pe[e] = (qb + cg * BWD_COLS + c0 + e < key_idx) ? 0.f : pe[e];
+          for (int e = 0; e < 8; ++e) pe[e] = fast_exp2(__uint_as_float(sreg[c0 + e]) * p.scale_log2 - lr[e]);
+          if (need_mask) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) pe[e] = (qb + g * 32 + c0 + e < key_idx) ? 0.f : pe[e];
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) ds[e] = pe[e] * (__uint_as_float(dreg[c0 + e]) * p.scale - dr[e]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            pk[c0 / 2 + e] = pack_bf16x2_alu(pe[2 * e], pe[2 * e + 1]);
+            dk[c0 / 2 + e] = pack_bf16x2_alu(ds[2 * e], ds[2 * e + 1]);
+          }
         }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) ds[e] = pe[e] * (__uint_as_float(dreg[c0 + e]) * p.scale - dr[e]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          pk[c0 / 2 + e] = pack_bf16x2_alu(pe[2 * e], pe[2 * e + 1]);
-          dk[c0 / 2 + e] = pack_bf16x2_alu(ds[2 * e], ds[2 * e + 1]);
-        }
+        BWD_TRACE(warp, t, 4);
+        tmem_st_32x16(tm_st + lane_addr + st * 64 + g * 32, pk);
+        tmem_st_32x16(tm_dpt + lane_addr + st * 64 + g * 32, dk);
       }
-      BWD_TRACE(warp, t, 4);
-      tmem_st_32x16(tm_st + lane_addr + st * 64 + cg * BWD_COLS, pk);
-      tmem_st_32x16(tm_dpt + lane_addr + st * 64 + cg * BWD_COLS, dk);
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&p_full[st]);
@@ -417,7 +437,7 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
       __nv_bfloat16* dk_row = p.dqkv + (size_t)(row_base + key_idx) * 3 * p.d + col_k;
       __nv_bfloat16* dv_row = p.dqkv + (size_t)(row_base + key_idx) * 3 * p.d + col_v;
 #pragma unroll 1
-      for (int c = cg; c < HW / 32; c += BWD_CG) {   // each warpgroup stores its own 32-column slices
+      for (int c = cg; c < HW / 32; c += B::CG) {   // each warpgroup stores its own 32-column slices
         uint32_t a[32], g[32];
         tmem_ld_32x32(tm_dk + lane_addr + c * 32, a);
         tmem_ld_32x32(tm_dv + lane_addr + c * 32, g);
@@ -455,41 +475,43 @@ flash_dkdv_kernel(const __grid_constant__ CUtensorMap tm_kv,   // box 64 x 128 o
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, B::TMEM);
   }
   BWD_CTA_LOG_END(0, t_cta_start, n_steps);
 }
 
 // ----------------------------------------------------------------------------------- dQ
-// CTA = 128 queries of one (b, h); walks 128-key steps j up to the diagonal:
-//   S = Q K_j^T and dP = dO V_j^T  (128 x 128 fp32 each, single buffered in tensor memory)
+// CTA = 128 queries of one (b, h); walks steps j of 128 keys (heads of 128) or 64 up to the diagonal:
+//   S = Q K_j^T and dP = dO V_j^T  (fp32, single buffered in tensor memory)
 //   dS = P * (dP - delta) * scale   written by the compute warps as packed bf16 into tensor memory
 //   dQ += dS K_j                    A operand straight from tensor memory, B = K_j MN-major
-// dS never touches shared memory, which therefore holds Q, dO, three K stages and two V stages (a K tile
+// dS never touches shared memory, which therefore holds Q, dO and rings of K and V (a K tile
 // stays live until its dQ MMA, a V tile only until its dP MMA).  Tensor pipe order per step:
 // [S, dP of step t+1] [dQ of step t], so the element-wise work on step t+1 overlaps the dQ MMAs of step t.
-constexpr int DQ_KSTAGES = 3;
-constexpr int DQ_VSTAGES = 2;
-
-template <int DH>
+template <int DH, bool TWO>
 struct DqSmem {
   static constexpr int PANELS = DH / 64;
-  static constexpr int TILE = 128 * DH * 2;   // Q_i, dO_i, K_j or V_j (128 rows)
+  static constexpr int TILE = 128 * DH * 2;   // Q_i or dO_i (128 rows)
+  static constexpr int KV_TILE = BwdShape<DH, TWO>::KEYS * DH * 2, KV_PANEL = BwdShape<DH, TWO>::KEYS * 128;      // K_j or V_j
+  static constexpr int DQ_KSTAGES = BwdShape<DH, TWO>::KSTAGES, DQ_VSTAGES = BwdShape<DH, TWO>::VSTAGES;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_DO = OFF_Q + TILE;
   static constexpr int OFF_K = OFF_DO + TILE;                 // DQ_KSTAGES stages
-  static constexpr int OFF_V = OFF_K + DQ_KSTAGES * TILE;     // DQ_VSTAGES stages
-  static constexpr int OFF_BAR = OFF_V + DQ_VSTAGES * TILE;
+  static constexpr int OFF_V = OFF_K + DQ_KSTAGES * KV_TILE;     // DQ_VSTAGES stages
+  static constexpr int OFF_BAR = OFF_V + DQ_VSTAGES * KV_TILE;
   static constexpr int NUM_BARS = 1 + 2 * DQ_KSTAGES + 2 * DQ_VSTAGES + 2 + 2 + 1;
   static constexpr int TOTAL = OFF_BAR + NUM_BARS * 8 + 16 + 1024;
 };
 
-template <int DH, int HW>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+template <int DH, int HW, bool TWO>
+__global__ void __launch_bounds__(BwdShape<DH, TWO>::THREADS, BwdShape<DH, TWO>::CTAS)
 flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 over qkv
+                const __grid_constant__ CUtensorMap tm_kv,    // box 64 x KEYS over qkv
                 const __grid_constant__ CUtensorMap tm_do,    // box 64 x 128 over dO
                 const FlashBwdParams p) {
-  using L = DqSmem<DH>;
+  using L = DqSmem<DH, TWO>;
+  using B = BwdShape<DH, TWO>;
+  constexpr int DQ_KSTAGES = B::KSTAGES, DQ_VSTAGES = B::VSTAGES, KEYS = B::KEYS;
   const uint64_t t_cta_start = globaltimer_ns();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -515,7 +537,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
   const int b = bh / p.heads, h = bh % p.heads;
   const int row_base = b * p.seq;
   const int q0 = iblk * 128;
-  const int n_steps = iblk + 1;   // 128-key steps up to and including the diagonal tile
+  const int n_steps = (min(q0 + 128, p.seq) + KEYS - 1) / KEYS;   // up to and including the diagonal
 
   if (threadIdx.x == 0) {
     mbar_init(qd_full, 1);
@@ -528,17 +550,18 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
       mbar_init(&v_empty[i], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(s_empty, BWD_COMPUTE_THREADS);
-    mbar_init(&p_full[0], BWD_COMPUTE_THREADS);
-    mbar_init(&p_full[1], BWD_COMPUTE_THREADS);
+    mbar_init(s_empty, B::COMPUTE);
+    mbar_init(&p_full[0], B::COMPUTE);
+    mbar_init(&p_full[1], B::COMPUTE);
     mbar_init(dq_done, 1);
     *abort_word = 0;
     fence_barrier_init();
     prefetch_tensormap(&tm_qkv);
+    prefetch_tensormap(&tm_kv);
     prefetch_tensormap(&tm_do);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_holder, 512);
+    tmem_alloc(tmem_holder, B::TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -546,10 +569,10 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
   tc_fence_after();
   pdl_sync();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tm_s = tmem_base;           // 128 columns
-  const uint32_t tm_dp = tmem_base + 128;    // 128 columns
-  const uint32_t tm_ds = tmem_base + 256;    // 2 x 64 columns of packed bf16 pairs
-  const uint32_t tm_dq = tmem_base + 384;    // DH columns
+  const uint32_t tm_s = tmem_base;               // KEYS columns
+  const uint32_t tm_dp = tmem_base + KEYS;       // KEYS columns
+  const uint32_t tm_ds = tmem_base + 2 * KEYS;   // 2 x KEYS / 2 columns of packed bf16 pairs
+  const uint32_t tm_dq = tmem_base + 3 * KEYS;   // DH columns
 
   const int col_q = h * HW, col_k = p.d + h * HW, col_v = 2 * p.d + h * HW;
 
@@ -565,19 +588,19 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
       }
       for (int t = 0; t < n_steps; ++t) {
         const int ks = t % DQ_KSTAGES, vs = t % DQ_VSTAGES;
-        const int krow = row_base + t * 128;
+        const int krow = row_base + t * KEYS;
         if (!mbar_wait(&k_empty[ks], ((t / DQ_KSTAGES) & 1) ^ 1, abort_word)) { *abort_word = ERR_WAIT_EMPTY; break; }
         BWD_TRACE(0, t, 0);
-        mbar_expect_tx(&k_full[ks], L::TILE);
+        mbar_expect_tx(&k_full[ks], L::KV_TILE);
 #pragma unroll
         for (int pn = 0; pn < L::PANELS; ++pn)
-          tma_load_2d(smem + L::OFF_K + ks * L::TILE + pn * 16384, &tm_qkv, &k_full[ks], col_k + pn * 64, krow);
+          tma_load_2d(smem + L::OFF_K + ks * L::KV_TILE + pn * L::KV_PANEL, &tm_kv, &k_full[ks], col_k + pn * 64, krow);
         if (!mbar_wait(&v_empty[vs], ((t / DQ_VSTAGES) & 1) ^ 1, abort_word)) { *abort_word = ERR_WAIT_EMPTY; break; }
         BWD_TRACE(0, t, 1);
-        mbar_expect_tx(&v_full[vs], L::TILE);
+        mbar_expect_tx(&v_full[vs], L::KV_TILE);
 #pragma unroll
         for (int pn = 0; pn < L::PANELS; ++pn)
-          tma_load_2d(smem + L::OFF_V + vs * L::TILE + pn * 16384, &tm_qkv, &v_full[vs], col_v + pn * 64, krow);
+          tma_load_2d(smem + L::OFF_V + vs * L::KV_TILE + pn * L::KV_PANEL, &tm_kv, &v_full[vs], col_v + pn * 64, krow);
       }
     } else if (lane == 1 && p.trace != nullptr && (int)blockIdx.x == p.trace_cta) {
       // tuning aid: arrival time of every K and V tile
@@ -593,22 +616,22 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
     if (elect_one()) {
       const int lane = 0;   // the tracing macro stamps from the issuing thread
       (void)lane;
-      constexpr uint32_t idesc_12 = make_idesc_bf16(128, 128, false, false);
+      constexpr uint32_t idesc_12 = make_idesc_bf16(128, KEYS, false, false);
       constexpr uint32_t idesc_3 = make_idesc_bf16(128, DH, false, true);
       const uint64_t q_desc = make_smem_desc(smem_u32(smem + L::OFF_Q), 16, 1024);
       const uint64_t do_desc = make_smem_desc(smem_u32(smem + L::OFF_DO), 16, 1024);
       auto issue12 = [&](int t) {
-        const uint64_t k_desc = make_smem_desc(smem_u32(smem + L::OFF_K + (t % DQ_KSTAGES) * L::TILE), 16, 1024);
-        const uint64_t v_desc = make_smem_desc(smem_u32(smem + L::OFF_V + (t % DQ_VSTAGES) * L::TILE), 16, 1024);
+        const uint64_t k_desc = make_smem_desc(smem_u32(smem + L::OFF_K + (t % DQ_KSTAGES) * L::KV_TILE), 16, 1024);
+        const uint64_t v_desc = make_smem_desc(smem_u32(smem + L::OFF_V + (t % DQ_VSTAGES) * L::KV_TILE), 16, 1024);
 #pragma unroll
         for (int k = 0; k < HW / 16; ++k) {
-          const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4;
-          umma_f16_ss(tm_s, q_desc + off, k_desc + off, idesc_12, k > 0 ? 1u : 0u);
+          const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4, offk = ((k / 4) * L::KV_PANEL + (k % 4) * 32) >> 4;
+          umma_f16_ss(tm_s, q_desc + off, k_desc + offk, idesc_12, k > 0 ? 1u : 0u);
         }
 #pragma unroll
         for (int k = 0; k < HW / 16; ++k) {
-          const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4;
-          umma_f16_ss(tm_dp, do_desc + off, v_desc + off, idesc_12, k > 0 ? 1u : 0u);
+          const uint32_t off = ((k / 4) * 16384 + (k % 4) * 32) >> 4, offk = ((k / 4) * L::KV_PANEL + (k % 4) * 32) >> 4;
+          umma_f16_ss(tm_dp, do_desc + off, v_desc + offk, idesc_12, k > 0 ? 1u : 0u);
         }
         umma_commit(s_full);
         umma_commit(&v_empty[t % DQ_VSTAGES]);
@@ -631,12 +654,12 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
         if (!ok) break;
         tc_fence_after();
         BWD_TRACE(1, t, 2);
-        // K = 128 keys; A = dS_t from tensor memory (16 keys = 8 packed columns); B = K_t MN-major: 16 keys are
-        // 2048 B apart inside a 64-column panel, the dh panels 16384 B apart.
-        const uint64_t kmn_desc = make_smem_desc(smem_u32(smem + L::OFF_K + (t % DQ_KSTAGES) * L::TILE), 16384, 1024);
-        const uint32_t a_tmem = tm_ds + (t & 1) * 64;
+        // K = KEYS keys; A = dS_t from tensor memory (16 keys = 8 packed columns); B = K_t MN-major: 16 keys are
+        // 2048 B apart inside a 64-column panel, the dh panels KV_PANEL apart.
+        const uint64_t kmn_desc = make_smem_desc(smem_u32(smem + L::OFF_K + (t % DQ_KSTAGES) * L::KV_TILE), L::KV_PANEL, 1024);
+        const uint32_t a_tmem = tm_ds + (t & 1) * (KEYS / 2);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
+        for (int k = 0; k < KEYS / 16; ++k)
           umma_f16_ts(tm_dq, a_tmem + k * 8, kmn_desc + ((k * 2048) >> 4), idesc_3, (t > 0 || k > 0) ? 1u : 0u);
         umma_commit(&k_empty[t % DQ_KSTAGES]);
         if (t == n_steps - 1) umma_commit(dq_done);
@@ -648,7 +671,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const int q_idx = q0 + r;
-    const int cg = (warp - 2) >> 2;          // this thread's 64 of the step's 128 keys
+    const int cg = (warp - 2) >> 2;          // this thread's 64 of the step's keys
     const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
     const bool valid = q_idx < p.seq;
     const size_t vec = ((size_t)b * p.heads + h) * p.seq + q_idx;
@@ -671,9 +694,9 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
       tc_fence_before();
       mbar_arrive(s_empty);      // S and dP may be overwritten by the MMAs of step t+1
       BWD_TRACE(trole, t, 2);
-      const int kb = t * 128 + cg * 64;
+      const int kb = t * KEYS + cg * 64;
       uint32_t packed[32];
-      if (t == n_steps - 1) {   // diagonal tile: causal mask
+      if (t * KEYS + KEYS > q0) {   // a tile on the diagonal: causal mask
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
@@ -703,7 +726,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
       }
       BWD_TRACE(trole, t, 3);
       // Buffer t&1 was last read by the dQ MMAs of step t-2, which precede the S MMAs of step t in the tensor pipe.
-      tmem_st_32x32(tm_ds + lane_addr + (t & 1) * 64 + cg * 32, packed);
+      tmem_st_32x32(tm_ds + lane_addr + (t & 1) * (KEYS / 2) + cg * 32, packed);
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&p_full[t & 1]);
@@ -714,7 +737,7 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
       tc_fence_after();
       __nv_bfloat16* dq_row = p.dqkv + (size_t)(row_base + q_idx) * 3 * p.d + col_q;
 #pragma unroll 1
-      for (int c = cg; c < HW / 32; c += BWD_CG) {
+      for (int c = cg; c < HW / 32; c += B::CG) {
         uint32_t a[32];
         tmem_ld_32x32(tm_dq + lane_addr + c * 32, a);
         tmem_ld_wait();
@@ -745,12 +768,12 @@ flash_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box 64 x 128 ov
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, B::TMEM);
   }
   BWD_CTA_LOG_END(1, t_cta_start, n_steps);
 }
 
-template <int DH, int HW = DH>
+template <int DH, int HW, bool TWO>
 static int launch_flash_bwd(const void* qkv, const void* dout, const FlashBwdParams& p, cudaStream_t stream) {
   const uint64_t rows = (uint64_t)p.batch * p.seq;
   CUtensorMap tm_qkv128, tm_qkv64, tm_do128, tm_do64;
@@ -758,12 +781,12 @@ static int launch_flash_bwd(const void* qkv, const void* dout, const FlashBwdPar
   if (make_tmap_bf16_2d(&tm_qkv64, qkv, rows, 3ull * p.d, 3ull * p.d, 64, 64)) return -20;
   if (make_tmap_bf16_2d(&tm_do128, dout, rows, (uint64_t)p.d, (uint64_t)p.d, 64, 128)) return -20;
   if (make_tmap_bf16_2d(&tm_do64, dout, rows, (uint64_t)p.d, (uint64_t)p.d, 64, 64)) return -20;
-  auto k1 = flash_dkdv_kernel<DH, HW>;
-  auto k2 = flash_dq_kernel<DH, HW>;
+  auto k1 = flash_dkdv_kernel<DH, HW, TWO>;
+  auto k2 = flash_dq_kernel<DH, HW, TWO>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DkDvSmem<DH>::TOTAL) != cudaSuccess) return -3;
-    if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<DH>::TOTAL) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DkDvSmem<DH, TWO>::TOTAL) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<DH, TWO>::TOTAL) != cudaSuccess) return -3;
     configured = true;
   }
   const int n_kblk = (p.seq + 127) / 128;
@@ -772,8 +795,9 @@ static int launch_flash_bwd(const void* qkv, const void* dout, const FlashBwdPar
   if (p.trace_cta == BWD_CTA_LOG) { }
   else if (p.trace_cta >= 0) p1.trace = nullptr;
   else { p2.trace = nullptr; p1.trace_cta = -p.trace_cta - 1; }
-  launch_dep(k1, p.batch * p.heads * n_kblk, BWD_THREADS, DkDvSmem<DH>::TOTAL, stream, tm_qkv128, tm_qkv64, tm_do64, p1);
-  launch_dep(k2, p.batch * p.heads * n_kblk, BWD_THREADS, DqSmem<DH>::TOTAL, stream, tm_qkv128, tm_do128, p2);
+  launch_dep(k1, p.batch * p.heads * n_kblk, BwdShape<DH, TWO>::THREADS, DkDvSmem<DH, TWO>::TOTAL, stream, tm_qkv128, tm_qkv64, tm_do64, p1);
+  launch_dep(k2, p.batch * p.heads * n_kblk, BwdShape<DH, TWO>::THREADS, DqSmem<DH, TWO>::TOTAL, stream, tm_qkv128,
+             BwdShape<DH, TWO>::KEYS == 64 ? tm_qkv64 : tm_qkv128, tm_do128, p2);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -789,6 +813,15 @@ static int g_bwd_trace_cta = 0;
 extern "C" void b200_flash_bwd_set_trace(long long* buf, int cta) {
   g_bwd_trace = buf;
   g_bwd_trace_cta = cta;
+}
+
+// Heads of 64 and 32: two CTAs per SM where there is more work than the longest CTA, which then has half of an SM, can hide.  Work of a CTA in
+// steps of 128 plus three for its ends.  us, one -> two CTAs per SM (heads of 64; heads x tokens): below the line 12 x 2048 61 -> 90, 36 x 777
+// 41 -> 49, 36 x 1024 49 -> 60, 24 x 2048 100 -> 104, 60 x 400 33 -> 34; above it 60 x 777 63 -> 56, 100 x 400 48 -> 41, 24 x 4096 310 -> 289,
+// 192 x 1024 254 -> 210, 600 x 777 596 -> 467.  One or two tiles of keys: below 60 x 256 19 -> 23, above 148 x 256 31 -> 28, 192 x 64 21 -> 17.
+static bool bwd_two_per_sm(long long heads, long long tiles) {
+  const long long work = heads * (tiles * (tiles + 1) / 2 + 3 * tiles), longest = tiles + 3;
+  return 10 * work > 148 * longest * (tiles <= 2 ? 12 : 16);
 }
 
 // qkv (rows, 3d), o / dout (rows, d) bf16; lse (batch, heads, seq) from the forward; delta: scratch of the
@@ -824,8 +857,10 @@ static int flash_bwd_impl(const void* qkv, const void* o, const void* dout, cons
   p.status = status;
   p.rope_cs = rope_cs; p.rope_ctx = rope_ctx;
   p.trace = g_bwd_trace; p.trace_cta = g_bwd_trace_cta;
-  if (dh == 32) return launch_flash_bwd<64, 32>(qkv, dout, p, stream);
-  return dh == 64 ? launch_flash_bwd<64>(qkv, dout, p, stream) : launch_flash_bwd<128>(qkv, dout, p, stream);
+  if (dh == 128) return launch_flash_bwd<128, 128, false>(qkv, dout, p, stream);
+  const bool two = bwd_two_per_sm((long long)batch * heads, (seq + 127) / 128);
+  if (dh == 32) return two ? launch_flash_bwd<64, 32, true>(qkv, dout, p, stream) : launch_flash_bwd<64, 32, false>(qkv, dout, p, stream);
+  return two ? launch_flash_bwd<64, 64, true>(qkv, dout, p, stream) : launch_flash_bwd<64, 64, false>(qkv, dout, p, stream);
 }
 
 extern "C" int b200_flash_bwd(const void* qkv, const void* o, const void* dout, const float* lse, float* delta,

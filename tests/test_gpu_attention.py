@@ -106,3 +106,26 @@ def test_narrow_heads(b, s, h, dh):
     plain = native.rope_(dqkv.contiguous(), cache, None, h, True, s)
     a, c = (t.view(b * s, 3, h, dh)[:, :, clean].float() for t in (turned, plain))
     assert (a - c).abs().max().item() < 3e-2 * max(1.0, c.abs().max().item())
+
+
+@pytest.mark.parametrize("b,s,h,dh", [(50, 1, 6, 64), (60, 64, 4, 32), (38, 65, 8, 64), (50, 128, 6, 32), (37, 129, 8, 64), (20, 191, 12, 32),
+                                      (25, 257, 8, 64), (12, 449, 10, 32), (10, 777, 12, 64)])
+def test_heads_of_64_and_32_on_shared_sms(b, s, h, dh):
+    """Enough sequences that two backward CTAs share an SM (and fewer, on one each): lengths at the edges of the 64- and 128-key tiles, every
+    sequence as if it ran alone, with large scores among small ones."""
+    from llm_systems_from_scratch_b200.ops import attention, native, torch_impl
+    qkv = _rand_qkv(b, s, h, dh, seed=s)
+    qkv.view(b * s, 3, h, dh)[::17, 0] *= 8                       # rows whose maximum moves late
+    do = torch.randn(b * s, h * dh, device="cuda").bfloat16()
+    o, lse = attention.attention_fwd(qkv, b, s, h)
+    dqkv = attention.attention_bwd(do, qkv, o, lse, b, s, h)
+    ro, rl = torch_impl.attention_fwd(qkv.float(), b, s, h)
+    ref = torch_impl.attention_bwd(do.float(), qkv.float(), ro, rl, b, s, h)
+    # P and O are rounded to bf16 (2^-9 each); the scores' sums are fp32
+    assert (o.float() - ro).norm() < 6e-3 * ro.norm() and (lse - rl).abs().max().item() < 2e-2
+    # P and dS are rounded to bf16 (2^-9 each, about 2.4e-3 of the norm together with the result's own rounding)
+    assert (dqkv.float() - ref).norm() < 1e-2 * ref.norm()
+    n = s * (b // 2)                                              # the same values whatever shares the SM
+    alone = attention.attention_bwd(do[n:n + s].contiguous(), qkv[n:n + s].contiguous(), o[n:n + s].contiguous(), lse[b // 2:b // 2 + 1].contiguous(), 1, s, h)
+    assert torch.equal(alone, dqkv[n:n + s])
+    native.check_status()

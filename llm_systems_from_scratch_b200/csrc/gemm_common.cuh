@@ -170,6 +170,29 @@ __device__ __forceinline__ void epilogue_rope(const float* table, int ctx, int d
   }
 }
 
+// The same in two steps: four vectors of cosines and four of sines of 32 columns, and the rotation.
+__device__ __forceinline__ void load_rope_columns(const GemmParams& p, int row, int col0, float4* v) {
+  const float* cs = p.rope_cs + (size_t)(row % p.rope_seq) * (p.rope_dh / 2) + col0 % p.rope_dh / 2;
+  const float* sn = cs + (size_t)p.rope_ctx * (p.rope_dh / 2);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    v[q] = *reinterpret_cast<const float4*>(cs + q * 4);
+    v[4 + q] = *reinterpret_cast<const float4*>(sn + q * 4);
+  }
+}
+__device__ __forceinline__ void apply_rope_columns(const float4* v, uint32_t (&acc)[32]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float cc[4] = {v[q].x, v[q].y, v[q].z, v[q].w}, ss[4] = {v[4 + q].x, v[4 + q].y, v[4 + q].z, v[4 + q].w};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float x0 = __uint_as_float(acc[q * 8 + 2 * t]), x1 = __uint_as_float(acc[q * 8 + 2 * t + 1]);
+      acc[q * 8 + 2 * t] = __float_as_uint(cc[t] * x0 - ss[t] * x1);
+      acc[q * 8 + 2 * t + 1] = __float_as_uint(ss[t] * x0 + cc[t] * x1);
+    }
+  }
+}
+
 // v Phi(v) for 16 values v = alpha * acc, Phi the normal distribution function: Phi(v) = 1/2 + v P(v^2) on [-4, 4], P of degree 8 fitted by
 // weighted least squares (error 4e-6), Phi(+-4) beyond.  For results that are rounded to bf16.  (With one epilogue warp per scheduler
 // only the instructions of other elements hide a latency: no branches, and all elements take each step together.)

@@ -140,7 +140,8 @@ __device__ __forceinline__ int list_pairs(const int* __restrict__ tile_group, in
 }
 
 // GROUPED: the 128-row tiles of A belong to the groups of rows of B in p.tile_group (negative: skipped); see list_pairs.
-template <bool A_MN, bool B_MN, bool GROUPED = false>
+// ROPE: the rotated QKV projection with TMA stores (p.rope_cs set), and no other epilogue.
+template <bool A_MN, bool B_MN, bool GROUPED = false, bool ROPE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmH,
@@ -391,6 +392,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int m_blk, n_blk, kb_lo, kb_hi, part;
       tile_coords(unit_tile(unit, kb_lo, kb_hi, part), p, num_m_tiles, m_blk, n_blk);
       const int acc = local & 1;
+      bool stored;
+      const int row0 = tile_row(m_blk, stored) + quarter * 32;
+      const int row = stored ? row0 + lane : p.M;
+      const int n0 = n_blk * P_BN;
+      // ROPE: cosines and sines of 64 columns, requested before the accumulator is waited for; where heads have 64 columns or 32 they serve the
+      // whole row.  With short contractions the epilogue is the longer part of a tile, and most of it were these loads (rotated QKV
+      // projection of 16384 rows, us: width 512, heads of 32 42.7 -> 31.6; width 768, heads of 64 73.0 -> 50.5; width 2048, heads of 128 284 -> 270).  An instance of its own: the
+      // gated epilogues miss the registers otherwise.
+      float4 turn[ROPE ? 16 : 1];
+      int turn_at = -1;       // column of a head that they start with
+      auto load_turn = [&](int col) {
+        if constexpr (ROPE) {
+          if (turn_at == col % p.rope_dh) return;
+          turn_at = col % p.rope_dh;
+          load_rope_columns(p, row, col, turn);
+          load_rope_columns(p, row, col + 32, turn + 8);
+        }
+      };
+      if (ROPE && n0 < 2 * p.rope_d) load_turn(n0);
       if (!mbar_wait(&tmem_full[acc], acc_phase[acc], abort_word)) {
         if (lane == 0) report(p, abort_word, ERR_WAIT_TMEM_FULL);
         ok = false;
@@ -398,10 +418,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       acc_phase[acc] ^= 1;
       tc_fence_after();
-      bool stored;
-      const int row0 = tile_row(m_blk, stored) + quarter * 32;
-      const int row = stored ? row0 + lane : p.M;
-      const int n0 = n_blk * P_BN;
       const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc * P_BN;
       // registers -> swizzled slab in shared memory -> TMA store (or TMA add).  Row `lane` of a slab is one 128-byte
       // line; its 16-byte pieces are permuted by (row & 7) as the 128-byte swizzle of the tensor maps expects, which
@@ -440,7 +456,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
         continue;
       }
-      if (p.swiglu_f > 0 && p.C == nullptr) {
+      if (!ROPE && p.swiglu_f > 0 && p.C == nullptr) {
         // the product alone: nothing is rounded before it
         const int col = n_blk * P_HALF;
 #pragma unroll 1
@@ -462,7 +478,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           }
           emit(&tmH, col + c * 64, o, false);
         }
-      } else if (p.swiglu_f > 0 && p.tma_store) {
+      } else if (!ROPE && p.swiglu_f > 0 && p.tma_store) {
         // accumulator columns [0,128) are gate_j, [128,256) the matching up_j; three outputs per 64 columns
         const int col = n_blk * P_HALF;
 #pragma unroll 1
@@ -501,7 +517,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           }
           emit(&tmH, col + c * 64, og, false);
         }
-      } else if (p.swiglu_f > 0) {
+      } else if (!ROPE && p.swiglu_f > 0) {
         // accumulator columns [0,128) are gate_j, [128,256) the matching up_j
         const int col = n_blk * P_HALF;
 #pragma unroll 1
@@ -532,7 +548,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             }
           }
         }
-      } else if (p.tma_store && p.epi == EPI_SWIGLU_BWD) {
+      } else if (!ROPE && p.tma_store && p.epi == EPI_SWIGLU_BWD) {
         // acc = dh (this row, 256 columns); R holds gate | up; d(gate) goes out through tmC, d(up) through tmH.
         // The gate / up pieces of the next 32 columns are fetched while the current 32 are computed, so that the
         // row-strided loads are off the critical path; two 32-column halves fill one 64-column slab per output.
@@ -601,8 +617,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         out_slab = 0;     // both slabs are in flight: the next emit() must wait for them (it waits for all but one)
         if (lane == 0) tma_store_wait_read<0>();
         __syncwarp();
-      } else if (p.tma_store) {
-        const bool out_f32 = p.epi == EPI_F32 || p.epi == EPI_F32_ACC;
+      } else if (ROPE || p.tma_store) {
+        const bool out_f32 = !ROPE && (p.epi == EPI_F32 || p.epi == EPI_F32_ACC);
         const int cols_per_chunk = out_f32 ? 32 : 64;
         const int nchunks = P_BN / cols_per_chunk;
 #pragma unroll 1
@@ -623,11 +639,14 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               epilogue_finish(p, col, p.N - col, r0);
               epilogue_finish(p, col + 32, p.N - col - 32, r1);
             }
-            if (p.rope_cs != nullptr && col < 2 * p.rope_d) {      // N = 3 * rope_d, heads are multiples of 32 columns
-              epilogue_rope(p, row, col, r0);
-              epilogue_rope(p, row, col + 32, r1);
+            if constexpr (ROPE) {
+              if (col < 2 * p.rope_d) {      // N = 3 * rope_d, heads are multiples of 32 columns
+                load_turn(col);
+                apply_rope_columns(turn, r0);
+                apply_rope_columns(turn + 8, r1);
+              }
             }
-            if (p.epi == EPI_BF16_RES && row < p.M) {
+            if (!ROPE && p.epi == EPI_BF16_RES && row < p.M) {
               const __nv_bfloat16* rp = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)row * p.ldr + col;
               if (col + 64 <= p.N && (p.ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(p.R) & 15) == 0) {
 #pragma unroll
@@ -735,10 +754,10 @@ pair_tail_sum_kernel(const float4* __restrict__ ws, OUT* __restrict__ C, const G
   }
 }
 
-template <bool A_MN, bool B_MN, bool GROUPED = false>
+template <bool A_MN, bool B_MN, bool GROUPED = false, bool ROPE = false>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmH,
                        GemmParams p, int sms, cudaStream_t stream) {
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, GROUPED>;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, GROUPED, ROPE>;
   constexpr int SMEM = GROUPED ? P_SMEM_GROUPED : P_SMEM;
   static bool configured = false;
   if (!configured) {
@@ -874,6 +893,7 @@ static int gemm_pair_impl(const void* A, const void* B, void* C, const void* R, 
   if (C == nullptr && !p.tma_store) return -13;
   const int sms = pair_sms();
   if (tile_group != nullptr) return p.tma_store ? launch_pair<false, false, true>(tmA, tmB, tmC, tmH, p, sms, stream) : -13;
+  if (rope_cs != nullptr && p.tma_store && !a_mn && !b_mn) return launch_pair<false, false, false, true>(tmA, tmB, tmC, tmH, p, sms, stream);
   if (splits > 1 && p.tma_store) {
     const int tiles = ((M + 255) / 256) * ((N + P_BN - 1) / P_BN), rest = tiles % (sms / 2);
     if (rest > 0 && make_tmap_out_2d(&tmH, true, ws, (uint64_t)rest * splits * 256, P_BN, P_BN, 32, 32) == 0) {

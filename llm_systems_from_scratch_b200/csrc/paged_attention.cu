@@ -5,125 +5,158 @@
 // Cache layout per layer: (num_pages, page_size, H*dh) bf16 for K and for V.  A request's tokens live in
 // the pages listed in its row of `block_tables`.
 //
-// Decode attention is bandwidth bound (every cached K and V byte is read once per step), so the kernel is
-// organised around reading whole token rows: one CTA serves one request (all its heads) over one split of the
-// context, 16 lanes cover the 256 bytes of one head (dh = 128; 8 lanes for dh = 64), scores are reduced with
-// shuffles, the softmax is kept online in registers and eight tokens' rows are in flight per thread.  The context
-// of a request is split over gridDim.y CTAs (flash-decoding); partial (max, sum, output) triples go to a scratch
-// buffer and a second kernel merges them.
+// Decode attention is bandwidth bound (every cached K and V byte is read once per step).  A warp serves one request over one split of its
+// context, for the 256 columns that it reads of a token row with 16 bytes per lane (two heads of 128, four of 64); it keeps its own ring of
+// eight-token chunks in shared memory, filled by cp.async, each lane reading what it copied itself, so that nothing but the data is waited for.
+// Scores are reduced with shuffles, the softmax is kept online in registers.  The context of a request is split over several warps
+// (flash-decoding); partial (max, sum, output) triples go to a scratch buffer and a second kernel merges them.
+//
+// (Before, a CTA of up to 512 threads served all heads over a split, eight tokens' rows in registers and nothing in flight while they were
+// worked on.  2048 columns, us before -> now, the same bits: one request of 901 tokens 24.7 -> 13.6, 20 of 128 to 2400 72.0 -> 40.8, 128 of them
+// 232.1 -> 220.5 (6.23 TB/s).  The splits of a request as one cluster that merges through its shared memory took 10 % longer.)
 #include "ptx.cuh"
 
 namespace b200 {
 
-constexpr int PD_UNROLL = 8;     // tokens whose K / V rows are in flight together, per CTA
+constexpr int PD_CHUNK = 8;      // tokens that are scored together
+constexpr int PD_STAGES = 2;     // chunks of a warp's ring in shared memory: thirteen warps on an SM.  us with two, three, four: 20 requests 40.8, 47.5, 46.5;
+                                 // 128 requests 220.5, 219.8, 221.1; 128 of 64 tokens 21.0, 24.8, 30.4.
+constexpr int PD_STAGE = 2 * PD_CHUNK * 32 * 16;
 
-// 16-byte load of cache data that is read exactly once per step: do not keep it in L1.
-__device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
+// 16 bytes global -> shared past L1; not `valid`: zeros, nothing is read.
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// One CTA = one request x one split of its context; its threads cover ALL heads: thread i owns the 8 head-columns
-// [8 i, 8 i + 8) of the token row, so the CTA reads every cached token as one contiguous row of H * DH elements (and
-// the 16 tokens of a page as one contiguous 16-row block), which is the access pattern DRAM serves at full speed.
-// A head's score is reduced over its DH / 8 neighbouring lanes with shuffles; each thread keeps the online-softmax
-// state (max, sum) of its head and its 8 output columns for the whole split, so nothing is combined inside the CTA.
-// The K and V rows of PD_UNROLL tokens are requested before the first score is computed.
 template <int DH>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(32)
 paged_decode_kernel(const __nv_bfloat16* __restrict__ q,        // (R, 3d) packed qkv or (R, d): row stride q_ld
                     const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
                     const int* __restrict__ block_tables, const int* __restrict__ context_lens,
                     float* __restrict__ part_o,                  // (R, H, splits, DH)
                     float* __restrict__ part_ml,                 // (R, H, splits, 2)
+                    __nv_bfloat16* __restrict__ out,             // (R, H * DH), written here; null: by the merge
                     int q_ld, int heads, int page_size, int max_pages, int splits, float scale_log2, int num_pages,
                     uint32_t* __restrict__ status) {
-  pdl_sync();
-  constexpr int LPT = DH / 8;            // lanes per head (16-byte loads)
-  const int r = blockIdx.x, split = blockIdx.y;
-  const int d = heads * DH;
-  const int col = threadIdx.x * 8;       // first of this thread's 8 columns of the token row
-  const bool active = col < d;           // the block is rounded up to whole warps
+  extern __shared__ uint4 pd_ring[];      // [stage][K, V][token of the chunk][lane]: a lane reads what it copied itself
+  constexpr int LPT = DH / 8;             // lanes per head (16-byte pieces)
+  const int lane = threadIdx.x;
+  const int d = heads * DH, groups = (d + 255) / 256;
+  const int unit = blockIdx.x;
+  const int g = unit % groups, split = unit / groups % splits, r = unit / (groups * splits);
+  const int col = (g * 32 + lane) * 8;    // first of this lane's 8 columns of the token row
+  const bool active = col < d;
   const int h = active ? col / DH : 0;
-  const int li = (threadIdx.x % LPT);
+  const int li = lane % LPT;
+  pdl_sync();
   // The tables come from the host scheduler; a length beyond the table or a page id beyond the cache is reported
   // through the status word and skipped, never dereferenced.
+  // Length, page ids and query are requested together.
   int ctx = context_lens[r];
-  if (ctx < 0 || ctx > max_pages * page_size) {
-    if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (1u << 8));
-    ctx = ctx < 0 ? 0 : max_pages * page_size;
-  }
-  // splits start on multiples of PD_UNROLL tokens so that a chunk of PD_UNROLL tokens never straddles a page whose
-  // size is a multiple of PD_UNROLL: one table lookup (and one integer division) per chunk instead of one per token
-  const int per = ((ctx + splits - 1) / splits + PD_UNROLL - 1) / PD_UNROLL * PD_UNROLL;
-  const int t0 = split * per;
-  const int t1 = min(ctx, t0 + per);
-
+  const int* table = block_tables + (size_t)r * max_pages;
+  int page0 = 0, ids = lane < max_pages ? table[lane] : 0;      // ids of 32 pages from page0 on, one per lane: a request does not wait for them
   float qv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (active) {
     const uint4 u = *reinterpret_cast<const uint4*>(q + (size_t)r * q_ld + col);
     const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), e = unpack_bf16x2(u.w);
     qv[0] = a.x; qv[1] = a.y; qv[2] = b.x; qv[3] = b.y; qv[4] = c.x; qv[5] = c.y; qv[6] = e.x; qv[7] = e.y;
   }
-  float m = -INFINITY, l = 0.f;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const int* table = block_tables + (size_t)r * max_pages;
-  for (int tb = t0; tb < t1; tb += PD_UNROLL) {
-    uint4 ku[PD_UNROLL], vu[PD_UNROLL];
-    bool valid[PD_UNROLL];
-    const int pg = tb / page_size, off = tb - pg * page_size;
-    if (off + PD_UNROLL <= page_size) {
-      // the whole chunk lies in one page: consecutive rows of the cache
-      const int page = table[pg];
-      const bool page_ok = (unsigned)page < (unsigned)num_pages;
-      if (!page_ok && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (2u << 8));
-      const size_t row0 = ((size_t)(page_ok ? page : 0) * page_size + off) * d + col;
-#pragma unroll
-      for (int u = 0; u < PD_UNROLL; ++u) {
-        valid[u] = page_ok && tb + u < t1;
-        ku[u] = make_uint4(0, 0, 0, 0);
-        vu[u] = make_uint4(0, 0, 0, 0);
-        if (valid[u] && active) {
-          ku[u] = ld_stream(k_cache + row0 + (size_t)u * d);
-          vu[u] = ld_stream(v_cache + row0 + (size_t)u * d);
+  if (ctx < 0 || ctx > max_pages * page_size) {
+    if (lane == 0 && status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (1u << 8));
+    ctx = ctx < 0 ? 0 : max_pages * page_size;
+  }
+  // splits start on multiples of PD_CHUNK tokens, so that a chunk never straddles a page whose size is a multiple of that
+  const int per = ((ctx + splits - 1) / splits + PD_CHUNK - 1) / PD_CHUNK * PD_CHUNK;
+  const int t0 = split * per;
+  const int t1 = min(ctx, t0 + per);
+  const bool whole = page_size % PD_CHUNK == 0;
+  int page = t0 / page_size, off = t0 - page * page_size;      // of the next chunk to request
+  uint32_t valid_bits = 0;                 // one byte per requested chunk, the youngest in the lowest
+  const uint32_t ring = smem_u32(pd_ring + lane);
+  auto request = [&](int tb, int stage) {
+    uint32_t mask = 0;
+    if (tb < t1) {
+      const uint32_t dst = ring + stage * PD_STAGE;
+      if (whole) {
+        if (page - page0 >= 32) {
+          page0 = page;
+          ids = page + lane < max_pages ? table[page + lane] : 0;
         }
-      }
-    } else {
+        const int id = __shfl_sync(0xffffffffu, ids, page - page0);
+        const bool ok = (unsigned)id < (unsigned)num_pages;
+        if (!ok && lane == 0 && status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (2u << 8));
+        const size_t at = ((size_t)(ok ? id : 0) * page_size + off) * d + col;
 #pragma unroll
-      for (int u = 0; u < PD_UNROLL; ++u) {
-        const int t = tb + u;
-        valid[u] = t < t1;
-        ku[u] = make_uint4(0, 0, 0, 0);
-        vu[u] = make_uint4(0, 0, 0, 0);
-        if (valid[u]) {
-          const int page = table[t / page_size];
-          if ((unsigned)page >= (unsigned)num_pages) {
-            if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (2u << 8));
-            valid[u] = false;
-          } else if (active) {
-            const size_t row = ((size_t)page * page_size + (t % page_size)) * d + col;
-            ku[u] = ld_stream(k_cache + row);
-            vu[u] = ld_stream(v_cache + row);
+        for (int u = 0; u < PD_CHUNK; ++u) {
+          const bool valid = ok && tb + u < t1;
+          if (valid) mask |= 1u << u;
+          if (active) {
+            cp_async_16(dst + u * 512, k_cache + (valid ? at + (size_t)u * d : 0), valid);
+            cp_async_16(dst + (PD_CHUNK + u) * 512, v_cache + (valid ? at + (size_t)u * d : 0), valid);
+          }
+        }
+        off += PD_CHUNK;
+        if (off == page_size) {
+          off = 0;
+          ++page;
+        }
+      } else {
+#pragma unroll 1
+        for (int u = 0; u < PD_CHUNK; ++u) {
+          const int t = tb + u;
+          bool valid = t < t1;
+          size_t at = 0;
+          if (valid) {
+            const int id = table[t / page_size];
+            if ((unsigned)id >= (unsigned)num_pages) {
+              if (lane == 0 && status != nullptr) atomicCAS(status, 0u, ERR_BAD_ARG | (2u << 8));
+              valid = false;
+            } else {
+              at = ((size_t)id * page_size + (t % page_size)) * d + col;
+              mask |= 1u << u;
+            }
+          }
+          if (active) {
+            cp_async_16(dst + u * 512, k_cache + (valid ? at : 0), valid);
+            cp_async_16(dst + (PD_CHUNK + u) * 512, v_cache + (valid ? at : 0), valid);
           }
         }
       }
     }
+    valid_bits = valid_bits << 8 | mask;
+    cp_async_commit();
+  };
+
+#pragma unroll
+  for (int s = 0; s < PD_STAGES - 1; ++s) request(t0 + s * PD_CHUNK, s);
+  float m = -INFINITY, l = 0.f;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  int stage = 0;
+#pragma unroll 1
+  for (int tb = t0; tb < t1; tb += PD_CHUNK) {
+    request(tb + (PD_STAGES - 1) * PD_CHUNK, stage == 0 ? PD_STAGES - 1 : stage - 1);
+    cp_async_wait<PD_STAGES - 1>();
+    const uint32_t valid = valid_bits >> (8 * (PD_STAGES - 1));
+    const uint4* kr = pd_ring + stage * (2 * PD_CHUNK * 32) + lane;
+    const uint4* vr = kr + PD_CHUNK * 32;
     // scores of the whole chunk first (independent of one another), then ONE running-max update for the chunk:
     // the serial chain of the online softmax is per chunk, not per token
-    float sc[PD_UNROLL];
+    float sc[PD_CHUNK];
     float mc = m;
 #pragma unroll
-    for (int u = 0; u < PD_UNROLL; ++u) {
-      const float2 k0 = unpack_bf16x2(ku[u].x), k1 = unpack_bf16x2(ku[u].y), k2 = unpack_bf16x2(ku[u].z),
-                   k3 = unpack_bf16x2(ku[u].w);
+    for (int u = 0; u < PD_CHUNK; ++u) {
+      const uint4 ku = kr[u * 32];
+      const float2 k0 = unpack_bf16x2(ku.x), k1 = unpack_bf16x2(ku.y), k2 = unpack_bf16x2(ku.z), k3 = unpack_bf16x2(ku.w);
       float s = qv[0] * k0.x + qv[1] * k0.y + qv[2] * k1.x + qv[3] * k1.y + qv[4] * k2.x + qv[5] * k2.y +
                 qv[6] * k3.x + qv[7] * k3.y;
 #pragma unroll
       for (int o = LPT / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      sc[u] = valid[u] ? s * scale_log2 : -INFINITY;
+      sc[u] = (valid >> u & 1) ? s * scale_log2 : -INFINITY;
       mc = fmaxf(mc, sc[u]);
     }
     if (mc > -INFINITY) {
@@ -132,24 +165,31 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q,        // (R, 3d) packe
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] *= corr;
 #pragma unroll
-      for (int u = 0; u < PD_UNROLL; ++u) {
+      for (int u = 0; u < PD_CHUNK; ++u) {
         const float p = exp2f(sc[u] - mc);    // 0 for tokens beyond the split or on a bad page
         l += p;
-        const float2 v0 = unpack_bf16x2(vu[u].x), v1 = unpack_bf16x2(vu[u].y), v2 = unpack_bf16x2(vu[u].z),
-                     v3 = unpack_bf16x2(vu[u].w);
+        const uint4 vu = vr[u * 32];
+        const float2 v0 = unpack_bf16x2(vu.x), v1 = unpack_bf16x2(vu.y), v2 = unpack_bf16x2(vu.z), v3 = unpack_bf16x2(vu.w);
         acc[0] += p * v0.x; acc[1] += p * v0.y; acc[2] += p * v1.x; acc[3] += p * v1.y;
         acc[4] += p * v2.x; acc[5] += p * v2.y; acc[6] += p * v3.x; acc[7] += p * v3.y;
       }
       m = mc;
     }
+    if (++stage == PD_STAGES) stage = 0;
   }
-  if (active) {
-    const size_t idx = ((size_t)r * heads + h) * splits + split;
-    float4* o = reinterpret_cast<float4*>(part_o + idx * DH + li * 8);
-    o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-    if (li == 0) { part_ml[idx * 2] = m; part_ml[idx * 2 + 1] = l; }
+  if (!active) return;
+  if (out != nullptr) {                       // one split: as the merge of one part
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = l > 0.f ? pack_bf16x2(acc[2 * e] / l, acc[2 * e + 1] / l) : 0u;
+    *reinterpret_cast<uint4*>(out + (size_t)r * d + col) = make_uint4(o[0], o[1], o[2], o[3]);
+    return;
   }
+  const size_t idx = ((size_t)r * heads + h) * splits + split;
+  float4* o = reinterpret_cast<float4*>(part_o + idx * DH + li * 8);
+  o[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  o[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  if (li == 0) { part_ml[idx * 2] = m; part_ml[idx * 2 + 1] = l; }
 }
 
 template <int DH>
@@ -255,23 +295,21 @@ extern "C" int b200_paged_decode(const void* q, const void* k_cache, const void*
     return -10;
   if (rows <= 0) return 0;
   if (splits < 1) splits = 1;
-  const int threads = (heads * (dh / 8) + 31) / 32 * 32;      // one thread per 8 columns of the token row, whole warps
-  if (threads > 512) return -12;     // heads * dh <= 4096
-  const dim3 grid(rows, splits);
+  if (heads * dh > 4096) return -12;
+  const long long units = (long long)rows * splits * ((heads * dh + 255) / 256);
+  if (units > 0x7fffffffll) return -12;
   const float sl2 = scale * 1.4426950408889634f;
-  if (dh == 128) {
-    launch_dep(paged_decode_kernel<128>, grid, threads, 0, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache,
-               (const __nv_bfloat16*)v_cache, block_tables, context_lens, part_o, part_ml, q_ld, heads, page_size,
-               max_pages, splits, sl2, num_pages, status);
-    launch_dep(paged_decode_merge_kernel<128>, rows * heads, 128, 0, st, part_o, part_ml, (__nv_bfloat16*)out, heads,
-               splits);
-  } else {
-    launch_dep(paged_decode_kernel<64>, grid, threads, 0, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache,
-               (const __nv_bfloat16*)v_cache, block_tables, context_lens, part_o, part_ml, q_ld, heads, page_size,
-               max_pages, splits, sl2, num_pages, status);
-    launch_dep(paged_decode_merge_kernel<64>, rows * heads, 64, 0, st, part_o, part_ml, (__nv_bfloat16*)out, heads,
-               splits);
-  }
+  __nv_bfloat16* direct = splits == 1 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? (__nv_bfloat16*)out : nullptr;
+  auto launch = [&](auto attend, auto merge) {
+    launch_dep(attend, dim3((unsigned)units), 32, PD_STAGES * PD_STAGE, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache,
+               (const __nv_bfloat16*)v_cache, block_tables, context_lens, part_o, part_ml, direct, q_ld, heads, page_size, max_pages, splits,
+               sl2, num_pages, status);
+    if (direct == nullptr) launch_dep(merge, rows * heads, dh, 0, st, part_o, part_ml, (__nv_bfloat16*)out, heads, splits);
+  };
+  if (dh == 128)
+    launch(paged_decode_kernel<128>, paged_decode_merge_kernel<128>);
+  else
+    launch(paged_decode_kernel<64>, paged_decode_merge_kernel<64>);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

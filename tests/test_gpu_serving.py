@@ -254,6 +254,29 @@ def test_long_steps_leave_rotation_and_append_to_a_launch_of_their_own(rows, wid
     assert bool(apart) != fused
 
 
+@pytest.mark.parametrize("page", [1, 5, 8, 12, 16])
+@pytest.mark.parametrize("heads,dh", [(1, 64), (5, 64), (3, 128), (32, 128)])
+@pytest.mark.parametrize("splits", [1, 2, 7])
+def test_paged_decode_forms(page, heads, dh, splits):
+    """Pages that chunks of eight tokens straddle and ones that they do not, rows of columns that are no multiple of a warp's 256, contexts of
+    more pages than a warp holds ids for, of none, one, a chunk and its edges; a query with a row pitch of its own."""
+    from llm_systems_from_scratch_b200.ops import native, serving_ops, torch_impl
+    d, lens = heads * dh, [0, 1, 7, 8, 9, 64, 100, 33 * page + 1, 65 * page]
+    per, r = 65 * page if page > 1 else 100, len(lens)
+    g = torch.Generator(device="cuda").manual_seed(page)
+    n_pages = -(-per // page) + 40
+    kc, vc = (torch.randn(n_pages, page, d, device="cuda", generator=g).bfloat16() for _ in "kv")
+    tables = torch.stack([torch.randperm(n_pages, device="cuda", generator=g)[:-(-per // page)] for _ in range(r)]).int()
+    lens = torch.tensor([min(n, tables.shape[1] * page) for n in lens], dtype=torch.int32, device="cuda")
+    q = torch.randn(r, 3 * d, device="cuda", generator=g).bfloat16()
+    out = serving_ops.paged_decode_attention(q, kc, vc, tables, lens, heads, splits)
+    assert not out[0].any()
+    ref = torch_impl.paged_decode_attention(q[1:, :d].double(), kc.double(), vc.double(), tables[1:], lens[1:], heads)
+    assert (out[1:].double() - ref).norm() <= 2.0 ** -8 * ref.norm()          # one rounding to bf16 is at most 2^-9
+    assert torch.equal(serving_ops.paged_decode_attention(q[:, :d].contiguous(), kc, vc, tables, lens, heads, splits), out)
+    native.check_status()
+
+
 @pytest.mark.parametrize("heads,dh,ff", [(4, 64, 704), (2, 128, 688), (16, 128, 5504)])
 def test_all_layers_from_one_call(heads, dh, ff, monkeypatch):
     """Prompts (short, and long enough for CTA pairs), a portion that continues beside single tokens, steps of single tokens and a captured

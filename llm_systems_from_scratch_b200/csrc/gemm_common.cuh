@@ -171,9 +171,9 @@ __device__ __forceinline__ void epilogue_rope(const float* table, int ctx, int d
 }
 
 // The same in two steps: four vectors of cosines and four of sines of 32 columns, and the rotation.
-__device__ __forceinline__ void load_rope_columns(const GemmParams& p, int row, int col0, float4* v) {
-  const float* cs = p.rope_cs + (size_t)(row % p.rope_seq) * (p.rope_dh / 2) + col0 % p.rope_dh / 2;
-  const float* sn = cs + (size_t)p.rope_ctx * (p.rope_dh / 2);
+__device__ __forceinline__ void load_rope_columns(const float* table, int ctx, int dh, int pos, int col0, float4* v) {
+  const float* cs = table + (size_t)pos * (dh / 2) + col0 % dh / 2;
+  const float* sn = cs + (size_t)ctx * (dh / 2);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     v[q] = *reinterpret_cast<const float4*>(cs + q * 4);
@@ -260,16 +260,37 @@ __device__ __forceinline__ void epilogue_rope(const GemmParams& p, int row, int 
   epilogue_rope(p.rope_cs, p.rope_ctx, p.rope_dh, row % p.rope_seq, col0, acc);
 }
 
-// The same for QkvAppend: the sums are rounded to bf16 first and rotated as rope_kv_append_kernel does, so that a step's values do not
-// depend on whether it takes this path.
-__device__ __forceinline__ void epilogue_append_rope(const QkvAppend& a, int row, int col0, uint32_t (&acc)[32]) {
+// 32 columns of a row of the projection that QkvAppend belongs to; `turn` as load_rope_columns has it.  The sums are rounded to bf16 first and
+// rotated as rope_kv_append_kernel does, so that a step's values do not depend on whether it takes this path.
+__device__ __forceinline__ void append_store(const GemmParams& p, int row, long long slot, int col0, const float4* turn, uint32_t (&acc)[32]) {
+  const QkvAppend& a = p.append;
+  if (row >= p.M) return;
+  if (col0 < 2 * a.d) {                                  // chunks are whole and inside a head (checked on the host)
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float2 v = unpack_bf16x2(pack_bf16x2(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1])));
-    acc[2 * j] = __float_as_uint(v.x);
-    acc[2 * j + 1] = __float_as_uint(v.y);
+    for (int j = 0; j < 16; ++j) {
+      const float2 v = unpack_bf16x2(pack_bf16x2(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1])));
+      acc[2 * j] = __float_as_uint(v.x);
+      acc[2 * j + 1] = __float_as_uint(v.y);
+    }
+    apply_rope_columns(turn, acc);
   }
-  epilogue_rope(a.cs, a.ctx, a.dh, a.positions[row], col0, acc);
+  uint4 o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t w[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) w[t] = pack_bf16x2(__uint_as_float(acc[j * 8 + 2 * t]), __uint_as_float(acc[j * 8 + 2 * t + 1]));
+    o[j] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  uint4* c = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + col0);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) c[j] = o[j];
+  if (col0 >= a.d && slot >= 0) {
+    const bool is_k = col0 < 2 * a.d;
+    uint4* to = reinterpret_cast<uint4*>((is_k ? a.k_cache : a.v_cache) + slot * a.d + (col0 - (is_k ? 1 : 2) * a.d));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) to[j] = o[j];
+  }
 }
 
 __device__ __forceinline__ float gate_of(float g) { return __fdividef(1.f, 1.f + __expf(-g)); }
@@ -282,8 +303,6 @@ __device__ __forceinline__ void epilogue_store(const GemmParams& p, int row, int
   if (ncols <= 0) return;
   if (p.finished) epilogue_finish(p, col0, ncols, acc);
   if (p.rope_cs != nullptr && col0 < 2 * p.rope_d && ncols == 32) epilogue_rope(p, row, col0, acc);
-  if (p.append.cs != nullptr && col0 < 2 * p.append.d)        // chunks are whole and inside a head (checked on the host)
-    epilogue_append_rope(p.append, row, col0, acc);
   if (p.epi == EPI_SWIGLU_BWD) {
     // as the stand-alone kernel (fast division apart): dh is rounded to bf16 first, gate and up are read as bf16
     const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(p.R) + (long long)row * p.ldr + col0;
@@ -372,19 +391,6 @@ __device__ __forceinline__ void epilogue_store(const GemmParams& p, int row, int
         for (int t = 0; t < 4; ++t)
           o[t] = pack_bf16x2(__uint_as_float(acc[j * 8 + 2 * t]), __uint_as_float(acc[j * 8 + 2 * t + 1]));
         *reinterpret_cast<uint4*>(c + j * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-      }
-      if (p.append.cs != nullptr && col0 >= p.append.d) {
-        const long long slot = append_slot(p.append, row, p.status);
-        const bool is_k = col0 < 2 * p.append.d;
-        __nv_bfloat16* dst = (is_k ? p.append.k_cache : p.append.v_cache) + slot * p.append.d + (col0 - (is_k ? 1 : 2) * p.append.d);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t o[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t)
-            o[t] = pack_bf16x2(__uint_as_float(acc[j * 8 + 2 * t]), __uint_as_float(acc[j * 8 + 2 * t + 1]));
-          if (slot >= 0) *reinterpret_cast<uint4*>(dst + j * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-        }
       }
     } else {
 #pragma unroll

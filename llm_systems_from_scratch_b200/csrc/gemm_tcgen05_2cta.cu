@@ -406,8 +406,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if constexpr (ROPE) {
           if (turn_at == col % p.rope_dh) return;
           turn_at = col % p.rope_dh;
-          load_rope_columns(p, row, col, turn);
-          load_rope_columns(p, row, col + 32, turn + 8);
+          load_rope_columns(p.rope_cs, p.rope_ctx, p.rope_dh, row % p.rope_seq, col, turn);
+          load_rope_columns(p.rope_cs, p.rope_ctx, p.rope_dh, row % p.rope_seq, col + 32, turn + 8);
         }
       };
       if (ROPE && n0 < 2 * p.rope_d) load_turn(n0);

@@ -119,7 +119,8 @@ struct GemmParams {
   //              (a mixture of experts whose tokens are sorted by expert); a negative group skips the tile
   //   by columns (`batch` > 1): problem g reads A columns from g * a_step, B rows from g * group_rows and writes C (and
   //              reads R) columns from g * c_step (one small matrix per attention head)
-  int row_step;               // rows of a row tile, at most BM (single-CTA kernel; below BM only with K-major A and no `tile_group`)
+  int row_step;               // rows of a row tile that are copied, at most BM (single-CTA kernel; below BM only with K-major A).  Row tiles are
+                              // this many rows apart, with `tile_group` BM
   const int* tile_group;
   int group_rows;
   int batch, a_step, c_step;

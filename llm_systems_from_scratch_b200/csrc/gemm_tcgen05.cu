@@ -21,11 +21,14 @@ namespace b200 {
 // decoder, us, let in -> not: 1500 rows 7373 -> 7350 (noise), 3000 rows 11335 -> 11127, 8192 rows 24170 -> 24040.
 constexpr int PDL_TRIGGER_M = 2048;
 
-template <int BN, int STAGES>
+// A_ROWS: rows of an A tile that a stage has room for.  With fewer than BM the MMA, which reads BM rows, reads on into the stages behind (and
+// from the last ones into B's), for rows of the accumulator that nobody looks at; B follows A for that.
+template <int BN, int STAGES, int A_ROWS>
 struct GemmSmem {
-  static constexpr int A_BYTES = BM * BK * 2;
+  static constexpr int A_BYTES = A_ROWS * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int DATA_BYTES = STAGES * (A_BYTES + B_BYTES);
+  static_assert(STAGES * B_BYTES >= BM * BK * 2 - A_BYTES, "the MMA's rows must lie in the ring");
   // barriers: full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2]; then tmem holder + abort word
   static constexpr int BAR_BYTES = (2 * STAGES + 4) * 8 + 16;
   static constexpr int TOTAL = DATA_BYTES + BAR_BYTES + 1024;  // + alignment slack
@@ -37,11 +40,13 @@ enum GemmGroup : int { GROUP_NONE = 0, GROUP_ROWS = 1, GROUP_COLS = 2 };
 // SWIGLU (grouped kernels): B holds group_rows = 2 N rows per group, gate rows first; a BN-wide tile is BN / 2 gate rows
 // and the matching BN / 2 up rows, and the epilogue stores silu(gate) * up (or relu(gate) * up).
 // APPEND: the QKV projection of a serving step (see QkvAppend), and nothing else.
-template <int BN, bool A_MN, bool B_MN, int STAGES, int GROUP = GROUP_NONE, bool SWIGLU = false, bool APPEND = false>
+template <int BN, bool A_MN, bool B_MN, int STAGES, int GROUP = GROUP_NONE, bool SWIGLU = false, bool APPEND = false,
+          int A_ROWS = BM>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const GemmParams p) {
-  using S = GemmSmem<BN, STAGES>;
+  static_assert(A_ROWS == BM || (!A_MN && !B_MN), "rows beyond a tile are K-major");
+  using S = GemmSmem<BN, STAGES, A_ROWS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
@@ -129,7 +134,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (GROUP == GROUP_ROWS) group = p.tile_group[m_blk];
         if (GROUP == GROUP_COLS) group = tile / tiles_one;
         if (GROUP == GROUP_ROWS && group < 0) continue;
-        const int m0 = m_blk * p.row_step, n0 = (GROUP != GROUP_NONE ? group * p.group_rows : 0) + n_blk * BN_OUT;
+        const int m0 = m_blk * (GROUP == GROUP_ROWS ? BM : p.row_step), n0 = (GROUP != GROUP_NONE ? group * p.group_rows : 0) + n_blk * BN_OUT;
         if (unit != (int)blockIdx.x) early = 0;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           const bool posted = kb - kb_lo < early;
@@ -232,7 +237,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       const int acc = local & 1;
       ++local;
       const int row_in_tile = quarter * 32 + lane;
-      const int row = row_in_tile < p.row_step ? m_blk * p.row_step + row_in_tile : p.M;
+      const int row = row_in_tile < p.row_step ? m_blk * (GROUP == GROUP_ROWS ? BM : p.row_step) + row_in_tile : p.M;
       const int n0 = n_blk * BN_OUT;
       // APPEND: position, slot and angles are requested before the accumulator is waited for, the next 32 columns' angles before these are turned.
       // What bounded this epilogue was one chain of three loads per 32 columns.  us a launch, 2048 columns, read behind the accumulator -> ahead: 200
@@ -471,17 +476,25 @@ static int row_step_of(int M) {
   return mt > 2 ? BM : ((M + mt - 1) / mt + 7) / 8 * 8;
 }
 
-template <int BN, bool A_MN, bool B_MN, int GROUP = GROUP_NONE, bool SWIGLU = false, bool APPEND = false>
+// Experts' tiles of a decode step hold at most the step's rows (`most` of b200_gemm_bf16_grouped): only those are copied, and with up to this
+// many a stage has no room for more, eight stages of 128 weight rows instead of six.  us a launch, eight experts, 64 rows in the step, 2 x 2752 x 2048
+// (gated) and 2048 x 2752: 51 -> 45, 24 -> 22 (floor 28 and 14); the step of the layered decoder 3130 -> 3010.
+constexpr int GROUP_A_ROWS = 64;
+
+template <int BN, bool A_MN, bool B_MN, int GROUP = GROUP_NONE, bool SWIGLU = false, bool APPEND = false, int A_ROWS = BM>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, int max_ctas, cudaStream_t stream) {
-  constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? 6 : 8);
-  using S = GemmSmem<BN, STAGES>;
-  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, STAGES, GROUP, SWIGLU, APPEND>;
+  constexpr int FULL = (BN == 256) ? 4 : (BN == 128 ? 6 : 8);
+  constexpr int STAGES = A_ROWS == BM ? FULL : 196608 / (BK * 2 * (A_ROWS + BN));
+  using S = GemmSmem<BN, STAGES, A_ROWS>;
+  static_assert(S::TOTAL <= 232448, "shared memory of one CTA");
+  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, STAGES, GROUP, SWIGLU, APPEND, A_ROWS>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return -3;
     configured = true;
   }
-  p.num_m_tiles = (p.M + p.row_step - 1) / p.row_step;
+  const int tile_rows = GROUP == GROUP_ROWS ? BM : p.row_step;
+  p.num_m_tiles = (p.M + tile_rows - 1) / tile_rows;
   constexpr int BN_OUT = SWIGLU ? BN / 2 : BN;
   p.num_n_tiles = (p.N + BN_OUT - 1) / BN_OUT;
   p.group_m = 16;
@@ -698,13 +711,14 @@ extern "C" int b200_gemm_bf16_splitk_finish(const void* A, const void* B, void* 
 //   tile_group == null: `batch` problems side by side: problem g multiplies A[:, g * a_step : g * a_step + K] with
 //     B[g * group_rows : g * group_rows + N, :] into C[:, g * c_step : g * c_step + N].  a_step must be a multiple of 8.
 //     With `swiglu` B has the 2 N rows of one gated feed-forward per problem, as above (any M).
+// most: with `tile_group`, rows of a tile that hold something (rounded up to 8; the others are neither read nor written), 0: all.
 // swiglu: 0 off, 1 silu(gate) * up, 2 relu(gate) * up.  head_gate: with epi 5, R (M, batch) holds one gate per problem.
 // finish: null, or what to do with the accumulators first (not with swiglu).
 // Columns of A past a problem's K (up to the next multiple of 64) are multiplied with zeros, so they must be finite.
 extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, const void* R, int M, int N, int K,
                                       long long lda, long long ldb, long long ldc, long long ldr, const int* tile_group,
                                       int n_groups, int group_rows, int batch, int a_step, int c_step, int swiglu,
-                                      int epi, int head_gate, const GemmFinish* finish, uint32_t* status, cudaStream_t stream) {
+                                      int epi, int head_gate, int most, const GemmFinish* finish, uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return -10;
@@ -716,6 +730,7 @@ extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, con
   if (head_gate && c_step <= 0) return -11;
   if (rows && ((M % BM) || n_groups <= 0 || group_rows != (swiglu ? 2 * N : N))) return -12;
   if (!rows && (batch <= 0 || (a_step & 7) || group_rows < (swiglu ? 2 * N : N))) return -12;
+  if (most < 0 || most > BM || (most && !rows)) return -12;
   if (swiglu < 0 || swiglu > 2 || (swiglu && (epi != EPI_BF16 || finish != nullptr))) return -12;
   if (finish != nullptr && finish->bias != nullptr && (rows || batch > 1)) return -12;
   if (finish != nullptr && finish->act == ACT_GELU && epi != EPI_BF16) return -12;
@@ -733,7 +748,7 @@ extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, con
   CUtensorMap tmA, tmB;
   const uint64_t a_cols = rows ? (uint64_t)K : (uint64_t)(batch - 1) * a_step + K;
   const uint64_t b_rows = rows ? (uint64_t)n_groups * group_rows : (uint64_t)batch * group_rows;
-  const int row_step = rows ? BM : row_step_of(M);
+  const int row_step = !rows ? row_step_of(M) : most ? (most + 7) / 8 * 8 : BM;
   int rc = make_tmap_bf16_2d(&tmA, A, (uint64_t)M, a_cols, (uint64_t)lda, 64, row_step);
   if (rc) return -20 + rc;
   rc = make_tmap_bf16_2d(&tmB, B, b_rows, (uint64_t)K, (uint64_t)ldb, 64, swiglu ? bn / 2 : bn);
@@ -759,6 +774,16 @@ extern "C" int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, con
     if (bn == 256) return launch_gemm<256, false, false, GROUP_COLS, true>(tmA, tmB, p, 0, stream);
     if (bn == 128) return launch_gemm<128, false, false, GROUP_COLS, true>(tmA, tmB, p, 0, stream);
     return launch_gemm<64, false, false, GROUP_COLS, true>(tmA, tmB, p, 0, stream);
+  }
+  if (rows && row_step <= GROUP_A_ROWS) {
+    if (swiglu) {
+      if (bn == 256) return launch_gemm<256, false, false, GROUP_ROWS, true, false, GROUP_A_ROWS>(tmA, tmB, p, 0, stream);
+      if (bn == 128) return launch_gemm<128, false, false, GROUP_ROWS, true, false, GROUP_A_ROWS>(tmA, tmB, p, 0, stream);
+      return launch_gemm<64, false, false, GROUP_ROWS, true, false, GROUP_A_ROWS>(tmA, tmB, p, 0, stream);
+    }
+    if (bn == 256) return launch_gemm<256, false, false, GROUP_ROWS, false, false, GROUP_A_ROWS>(tmA, tmB, p, 0, stream);
+    if (bn == 128) return launch_gemm<128, false, false, GROUP_ROWS, false, false, GROUP_A_ROWS>(tmA, tmB, p, 0, stream);
+    return launch_gemm<64, false, false, GROUP_ROWS, false, false, GROUP_A_ROWS>(tmA, tmB, p, 0, stream);
   }
   if (rows && swiglu) {
     if (bn == 256) return launch_gemm<256, false, false, GROUP_ROWS, true>(tmA, tmB, p, 0, stream);

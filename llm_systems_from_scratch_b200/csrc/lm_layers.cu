@@ -32,7 +32,8 @@ int b200_gemm_bf16_pair_swiglu(const void* A, const void* B, void* C, void* H, i
                                int rank, uint32_t* status, cudaStream_t stream);
 int b200_gemm_bf16_grouped(const void* A, const void* B, void* C, const void* R, int M, int N, int K, long long lda, long long ldb,
                            long long ldc, long long ldr, const int* tile_group, int n_groups, int group_rows, int batch, int a_step, int c_step,
-                           int swiglu, int epi, int head_gate, const GemmFinish* finish, uint32_t* status, cudaStream_t stream);
+                           int swiglu, int epi, int head_gate, int most, const GemmFinish* finish, uint32_t* status,
+                           cudaStream_t stream);
 }
 
 // Passed by pointer through the C interface: the field order is part of it.
@@ -111,7 +112,7 @@ extern "C" int b200_lm_layers(const LmStep* step, cudaStream_t st) {
       LM(paired);
     } else if (s.glu != LM_GLU_ROUNDED) {
       LM(b200_gemm_bf16_grouped(s.h, w.wgu, s.act, nullptr, s.rows, s.ff, s.d, s.d, s.d, s.ff, 0, nullptr, 0, 2 * s.ff, 1, 0, 0, 1, EPI_B_STABLE, 0,
-                                nullptr, s.status, st));
+                                0, nullptr, s.status, st));
     } else {
       LM(lm_product(s, s.pgu, s.h, w.wgu, s.gu, nullptr, 2 * s.ff, s.d, st));
       LM(b200_silu_mul_fwd(s.gu, s.act, s.rows, s.ff, st));

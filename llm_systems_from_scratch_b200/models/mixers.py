@@ -535,6 +535,8 @@ class TableExperts:
         self.table = _expect("table", get("table"), vocab, top).to(device=device, dtype=torch.int32).contiguous()
         if int(self.table.min()) < 0 or int(self.table.max()) >= experts:
             raise ValueError("the expert table names an expert that does not exist")
+        # how often a token's row may name one expert: what its tile can hold per token
+        self.repeats = int((self.table[:, :, None] == self.table[:, None, :]).sum(2).max())
         gu = torch.cat([_expect(f"e{e}.{k}", get(f"e{e}.{k}"), ff, width) for e in range(experts) for k in ("gate", "up")])
         self.w_gu = mo.padded_weight(gu, dtype, device)                            # (experts * 2 ff, width), gate first
         self.w_down = mo.padded_weight(torch.cat([_expect(f"e{e}.down", get(f"e{e}.down"), width, ff)
@@ -544,9 +546,10 @@ class TableExperts:
         """Rows of the expert-sorted buffers for a step of ``tokens`` rows."""
         return mo.plan_tiles(tokens, self.experts, self.top) * mo.TILE
 
-    def __call__(self, xg, tile_group):
-        hidden = mo.gemm_rows(xg, self.w_gu, tile_group, self.ff, swiglu=True)
-        return mo.gemm_rows(hidden, self.w_down, tile_group, self.width, swiglu=False)
+    def __call__(self, xg, tile_group, tokens: int):
+        most = tokens * self.repeats
+        hidden = mo.gemm_rows(xg, self.w_gu, tile_group, self.ff, swiglu=True, most=most)
+        return mo.gemm_rows(hidden, self.w_down, tile_group, self.width, swiglu=False, most=most)
 
 
 class RoutedExperts:
@@ -604,8 +607,9 @@ class RoutedExperts:
             z = mo.linear(h, self.w_router, out_dtype=torch.float32)               # what is routed by is 32-bit
             choice, rank, weight = mo.moe_route(z[:, :cols], self.correction, slots, self.experts, self.top, count, fold, self.bias)
         xg, pos, groups = mo.moe_dispatch(h, choice, rank, count, fold)
-        y = mo.gemm_rows(mo.gemm_rows(xg, self.w_up, groups, self.ff, self.gated, None if self.gated else "gelu"), self.w_down, groups, self.width,
-                         False)
+        most = rows * self.top                    # a row of scores that are no numbers may choose one expert more than once
+        y = mo.gemm_rows(mo.gemm_rows(xg, self.w_up, groups, self.ff, self.gated, None if self.gated else "gelu", most), self.w_down, groups,
+                         self.width, False, most=most)
         if self.gate is not None:
             return mo.ExpertOutputs(y, pos, self.gain, weight, h if self.identity else None), self.gate(h)[:, self.gate.at["out"]]
         if fold or not self.shared:

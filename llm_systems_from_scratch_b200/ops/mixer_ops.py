@@ -38,7 +38,7 @@ def _lib():
             "b200_glu_any": [P, P, L, I, L, L, I, I, P],
             "b200_gate_sigmoid": [P, P, L, I, I, L, L, I, P],
             "b200_gemm_f32": [P, P, P, I, I, I, L, L, L, I, P, I, I, I, I, P, P],
-            "b200_gemm_bf16_grouped": [P, P, P, P, I, I, I, L, L, L, L, P, I, I, I, I, I, I, I, I, P, P, P],
+            "b200_gemm_bf16_grouped": [P, P, P, P, I, I, I, L, L, L, L, P, I, I, I, I, I, I, I, I, I, P, P, P],
             "b200_gemm_bf16_pair_grouped": [P, P, P, I, I, I, L, L, L, P, I, I, P, P, P],
             "b200_moe_route": [P, L, P, P, P, P, P, P, P, I, I, I, I, I, P],
             "b200_moe_route_rows": [P, L, P, L, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
@@ -131,10 +131,11 @@ def linear(a, w, out=None, accumulate=False, out_dtype=None, bias=None, alpha: f
     return out
 
 
-def gemm_rows(a, w, tile_group, n: int, swiglu: bool, act: str | None = None):
+def gemm_rows(a, w, tile_group, n: int, swiglu: bool, act: str | None = None, most: int = TILE):
     """Every 128-row tile t of a (P, K) times the rows of w that belong to group tile_group[t] (negative: skipped, the
     rows of the result stay undefined).  ``swiglu``: a group has 2 n rows, gate rows first, and the result is
-    silu(gate) * up; otherwise n rows and ``act`` of the product."""
+    silu(gate) * up; otherwise n rows and ``act`` of the product.  ``most``: no tile holds more rows than this; what is behind them in a tile
+    stays undefined."""
     rows = 2 * n if swiglu else n
     if not a.is_cuda:
         return mixer_torch.gemm_rows(a, w, tile_group, rows, n, swiglu, act)
@@ -153,7 +154,8 @@ def gemm_rows(a, w, tile_group, n: int, swiglu: bool, act: str | None = None):
                 _check(rc, "gemm_pair_grouped")
                 return out
         _check(lib.b200_gemm_bf16_grouped(_ptr(a), _ptr(w), _ptr(out), None, p, n, k, a.stride(0), w.stride(0), out.stride(0),
-                                          0, _ptr(tile_group), w.shape[0] // rows, rows, 1, 0, 0, int(swiglu), 0, 0, _ref(finish),
+                                          0, _ptr(tile_group), w.shape[0] // rows, rows, 1, 0, 0, int(swiglu), 0, 0,
+                                          most if most < TILE else 0, _ref(finish),
                                           _ptr(native.status_word(a.device)), _stream()), "gemm_grouped")
         return out
     out = rows_buffer(p, rows, a.dtype, a.device)
@@ -178,7 +180,7 @@ def glu(a, w, n: int, act: str):
         return out
     if a.dtype == torch.bfloat16:
         _check(lib.b200_gemm_bf16_grouped(_ptr(a), _ptr(w), _ptr(out), None, m, n, k, a.stride(0), w.stride(0), out.stride(0), 0, None,
-                                          0, 2 * n, 1, 0, 0, 2 if act == "relu" else 1, native.EPI_B_STABLE, 0, None,
+                                          0, 2 * n, 1, 0, 0, 2 if act == "relu" else 1, native.EPI_B_STABLE, 0, 0, None,
                                           _ptr(native.status_word(a.device)), _stream()), "gemm_glu")
         return out
     gu = linear(a, w)
@@ -205,7 +207,7 @@ def gemm_heads(a, w, heads: int, k: int, n: int, out=None, gate=None, a_step: in
         epi = (5 if gate is not None else 0) | native.EPI_B_STABLE
         _check(lib.b200_gemm_bf16_grouped(_ptr(a), _ptr(w), _ptr(out), _ptr(gate), a.shape[0], n, k, a.stride(0), w.stride(0),
                                           out.stride(0), 0 if gate is None else gate.stride(0), None, 0, w.shape[0] // heads,
-                                          heads, a_step, c_step, 0, epi, int(by_head), None, _ptr(native.status_word(a.device)),
+                                          heads, a_step, c_step, 0, epi, int(by_head), 0, None, _ptr(native.status_word(a.device)),
                                           _stream()), "gemm_heads")
         return out
     _check(lib.b200_gemm_f32(_ptr(a), _ptr(w), _ptr(out), a.shape[0], n, k, a.stride(0), w.stride(0), out.stride(0), 0, None,

@@ -178,7 +178,7 @@ class ParallelLayers(LayeredBackend):
             embed, pending = (None, None), None
             layer.mixer(h, x, batch, self.cache.entries[run])
             if ex is not None:
-                pending = (ex(xg, groups), pos, 1.0 / ex.top)
+                pending = (ex(xg, groups, batch.n_rows), pos, 1.0 / ex.top)
             if trace is not None:
                 if pending is not None:
                     mo.residual_norm(x, pending=pending)

@@ -477,3 +477,30 @@ def test_more_row_tiles_than_a_pair_lists(monkeypatch):
             at.setattr(mo, "PAIR_GROUP_ROWS", (1 << 30, 1 << 30))
             assert torch.equal(got, mo.gemm_rows(x, w, tile_group, 64, False))
     native.check_status()
+
+
+@pytest.mark.parametrize("most", [1, 9, 33, 64, 65, 127])
+@pytest.mark.parametrize("groups", [[0], [2, 0, 1], [3, 3, -1, 1, -1], list(range(8))])
+@pytest.mark.parametrize("n,k,act", [(24, 64, "silu"), (1344, 512, "silu"), (8, 72, None), (768, 1344, "gelu")])
+def test_grouped_products_of_few_rows(most, groups, n, k, act, monkeypatch):
+    """Tiles of which only the first rows hold something: those are whole tiles' bits, the rest of the buffer is left alone."""
+    from llm_systems_from_scratch_b200.ops import mixer_ops as mo, native
+    tile_group = torch.tensor(groups, dtype=torch.int32, device="cuda")
+    g = torch.Generator("cuda").manual_seed(n)
+    gated = act == "silu"
+    x = torch.full((len(groups) * 128, k), float("nan"), device="cuda", dtype=torch.bfloat16)
+    live = (torch.arange(len(groups), device="cuda")[:, None] * 128 + torch.arange(most, device="cuda"))[tile_group >= 0].flatten()
+    x[live] = torch.randn(len(live), k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(8 * n * (2 if gated else 1), k, generator=g, device="cuda") / k ** 0.5).bfloat16()
+    made = []
+
+    def rows_buffer(rows, cols, dtype, device):
+        made.append(torch.full((rows, cols), 7.0, dtype=dtype, device=device))
+        return made[-1]
+    monkeypatch.setattr(mo, "rows_buffer", rows_buffer)
+    got, want = (mo.gemm_rows(x, w, tile_group, n, gated, None if gated else act, **kw) for kw in ({"most": most}, {}))
+    assert torch.equal(got[live], want[live])
+    read = (most + 7) // 8 * 8                                    # rows are copied eight at a time
+    rest = (torch.arange(len(x), device="cuda") % 128 >= read) | (tile_group.repeat_interleave(128) < 0)
+    assert bool((got[rest] == 7.0).all())
+    native.check_status()

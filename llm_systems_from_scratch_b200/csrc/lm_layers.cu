@@ -1,6 +1,6 @@
 // All layers of one serving step of the TransformerLM from one call: the same launches, in the same order and with the same arguments, that
 // the ops make one by one.  A launch through Python takes the host about 13 us, which is what bounds short prompts (200 tokens, 24 layers of
-// 2048: 2845 us op by op, 2300 from here, which the device needs).
+// 2048: 2845 us op by op, 2300 from here, when the device needed that).
 // Which kernel a product takes is decided by the caller (`LmProduct`), once per step.
 #include "gemm_common.cuh"
 
